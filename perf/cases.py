@@ -182,8 +182,8 @@ def tolerance(case: dict):
     if case["act"] == "f32":
         return {"rel": 1e-5, "max": 1e-4, "differ": 0.0005}
     if case["kind"].startswith("logesun"):
-        # a router's near tie sends a token to another expert of almost the same weight
-        return {"rel": 0.02 if case["act"] == "f16" else 0.03, "max": 0.9, "differ": 0.005}
+        # a router's near tie may send a token to another expert of almost the same weight
+        return {"rel": 0.005, "max": 0.1, "differ": 0.005} if case["act"] == "f16" else {"rel": 0.03, "max": 0.5, "differ": 0.01}
     return {"rel": 0.003, "max": 0.02, "differ": 0.002} if case["act"] == "f16" else {"rel": 0.02, "max": 0.15, "differ": 0.005}
 
 
@@ -303,6 +303,9 @@ def _layered_counts(case: dict, cfg: dict):
 def _layered_weights(cfg: dict, seed: int) -> dict:
     r, width = _Random(seed), cfg["width"]
     w = {"embed": r(cfg["vocab"], width)}
+    routed = any((layer["mlp"] or {}).get("kind") == "moe" for layer in cfg["layers"])
+    if routed:
+        w["embed"][:, 0] = 12.0     # what every token has in common: the routers' offset
     gain = dict(std=0.1, mean=1.0)
     for n, layer in enumerate(cfg["layers"]):
         p, m, f = f"l{n}", layer["mixer"], layer["mlp"]
@@ -339,10 +342,15 @@ def _layered_weights(cfg: dict, seed: int) -> dict:
             w.update({u + ".gate": r.matrix(ff, width), u + ".up": r.matrix(ff, width), u + ".down": r.matrix(width, ff)})
         w[p + ".norm2b"] = r(width, std=0.05, mean=0.5 if f["kind"] == "dense" else 0.25)
         if f["kind"] == "moe":
-            w[p + ".mlp.router"] = r.matrix(f["router"]["experts"], width)
+            # Scores that fall off within the chosen ones: the last of them, which rounding may exchange for the next, hardly
+            # counts.  With scores near one another a single such exchange outweighs all rounding errors of a pass.
+            w[p + ".mlp.router"] = r.matrix(f["router"]["experts"], width) * 6.0
+            w[p + ".mlp.router"][:, 0] = -1.7
     w["final.norm"] = r(width, **gain)
     head = torch.empty_like(w["embed"])
     head[_successors(seed)] = w["embed"] * width ** -0.5
+    if routed:
+        head[:, 0] = 0.0
     w["head"] = head.to(torch.bfloat16).float()
     return w
 
