@@ -347,15 +347,23 @@ attn_combine_kernel(AttnStreamArgs a) {
   const long long ih = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (ih >= (long long)a.n_items * a.n_heads) return;
   const float* rec0 = a.scratch + (size_t)ih * a.n_splits * ATTN_SCRATCH_STRIDE;
-  float m = -INFINITY;
-  for (int s = 0; s < a.n_splits; ++s) m = fmaxf(m, rec0[s * ATTN_SCRATCH_STRIDE + 64]);
+  // lane s holds the maximum and sum of splits s and s + 32 (at most 64 splits), so both are one round of loads
+  const int s1 = lane + 32;
+  const float m0 = lane < a.n_splits ? rec0[lane * ATTN_SCRATCH_STRIDE + 64] : -INFINITY;
+  const float m1 = s1 < a.n_splits ? rec0[s1 * ATTN_SCRATCH_STRIDE + 64] : -INFINITY;
+  const float l0 = lane < a.n_splits ? rec0[lane * ATTN_SCRATCH_STRIDE + 65] : 0.f;
+  const float l1 = s1 < a.n_splits ? rec0[s1 * ATTN_SCRATCH_STRIDE + 65] : 0.f;
+  float m = fmaxf(m0, m1);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   const float m_safe = (m == -INFINITY) ? 0.f : m;
-  float l = 0.f, o0 = 0.f, o1 = 0.f;
+  const float f0 = exp2f(m0 - m_safe), f1 = exp2f(m1 - m_safe);
+  const float l = warp_sum(l0 * f0 + l1 * f1);
+  float o0 = 0.f, o1 = 0.f;
+#pragma unroll 8
   for (int s = 0; s < a.n_splits; ++s) {
-    const float* rec = rec0 + s * ATTN_SCRATCH_STRIDE;
-    const float sc = exp2f(rec[64] - m_safe);
-    l += rec[65] * sc;
-    const float2 v = *reinterpret_cast<const float2*>(rec + 2 * lane);
+    const float sc = __shfl_sync(0xffffffffu, s < 32 ? f0 : f1, s & 31);
+    const float2 v = *reinterpret_cast<const float2*>(rec0 + s * ATTN_SCRATCH_STRIDE + 2 * lane);
     o0 += v.x * sc;
     o1 += v.y * sc;
   }
@@ -368,7 +376,7 @@ attn_combine_kernel(AttnStreamArgs a) {
 
 int arcb_launch_attn_stream(const AttnStreamArgs& a, cudaStream_t stream) {
   if (a.n_items <= 0) return 0;
-  if (a.n_splits < 1 || (a.n_splits > 1 && !a.scratch)) return -1;
+  if (a.n_splits < 1 || a.n_splits > 64 || (a.n_splits > 1 && !a.scratch)) return -1;
   const long long n_work = (long long)a.n_items * a.n_heads * a.n_splits;
   const long long blocks = (n_work + WARPS_PER_CTA - 1) / WARPS_PER_CTA;
   if (blocks > 0x7fffffffLL) return -1;

@@ -11,6 +11,15 @@ namespace {
 
 constexpr int ROWS_PER_CTA = 4;
 
+// One CTA per row instead of one warp: launches of at most this many rows leave most of the machine idle
+// otherwise, and a row's time is then one warp's chain of loads and shuffles (1280 columns: 40 floats a lane).
+// B200, us per launch inside the captured step, warp / CTA per row: norm of 6 rows of 1280 columns 4.8 / 1.8, of 128 rows
+// of 1024 3.8 / 1.8; head of 16 rows of 1024 21.5 / 4.0, step begin 9.1 / 2.9.  2048 such CTAs are one wave; above that the
+// warp form reads at the HBM rate.
+constexpr int CTA_ROW_MAX = 2048;
+constexpr int CTA_THREADS = 128;
+constexpr int CTA_MAX_D = CTA_THREADS * 4 * 4;   // columns a CTA holds in registers
+
 // sum of squares of a row held in global memory, warp-cooperative
 __device__ __forceinline__ float row_sumsq(const float* __restrict__ x, int d, int lane) {
   float ss = 0.f;
@@ -73,6 +82,24 @@ __device__ __forceinline__ void row_norm_store(const float* __restrict__ x, cons
   }
 }
 
+// Embedding row into registers (a CTA's share of it), and into the residual stream.
+template <int NV>
+__device__ __forceinline__ void cta_embed(float4 (&v)[NV], float* x, const float* tok_row, const float* ex_row, int d) {
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = (threadIdx.x + k * CTA_THREADS) * 4;
+    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < d) {
+      v[k] = __ldg(reinterpret_cast<const float4*>(tok_row + i));
+      if (ex_row) {
+        const float4 e = __ldg(reinterpret_cast<const float4*>(ex_row + i));
+        v[k].x += e.x; v[k].y += e.y; v[k].z += e.z; v[k].w += e.w;
+      }
+      *reinterpret_cast<float4*>(x + i) = v[k];
+    }
+  }
+}
+
 __device__ __forceinline__ void row_embed(float* __restrict__ x, const float* __restrict__ tok_row,
                                           const float* __restrict__ ex_row, int d, int lane) {
   for (int i = lane * 4; i < d; i += 128) {
@@ -84,6 +111,55 @@ __device__ __forceinline__ void row_embed(float* __restrict__ x, const float* __
     *reinterpret_cast<float4*>(x + i) = v;
   }
   __syncwarp();
+}
+
+// Sum over the CTA's four warps, in a fixed order; every thread gets it.
+__device__ __forceinline__ float cta_sum4(float v, float* sm) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return (sm[0] + sm[1]) + (sm[2] + sm[3]);
+}
+
+// The row's columns tid * 4 + k * 512 in v (zeros beyond d): norm, gain, 16-bit operand.
+template <int NV>
+__device__ __forceinline__ void cta_norm_store(const float4 (&v)[NV], const float* w, uint16_t* out, int d, float eps,
+                                               int act_f16, float* sm) {
+  float4 g[NV];
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = (threadIdx.x + k * CTA_THREADS) * 4;
+    g[k] = i < d ? __ldg(reinterpret_cast<const float4*>(w + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+  }
+  const float inv = rsqrtf(cta_sum4(ss, sm) / (float)d + eps);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = (threadIdx.x + k * CTA_THREADS) * 4;
+    if (i < d) {
+      uint2 pk;
+      pk.x = pack2_act((v[k].x * inv) * g[k].x, (v[k].y * inv) * g[k].y, act_f16);
+      pk.y = pack2_act((v[k].z * inv) * g[k].z, (v[k].w * inv) * g[k].w, act_f16);
+      *reinterpret_cast<uint2*>(out + i) = pk;
+    }
+  }
+}
+
+template <int NV>
+__global__ void __launch_bounds__(CTA_THREADS)
+rmsnorm_cta_kernel(const float* x, const float* w, uint16_t* out, int d, float eps, int act_f16) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float sm[4];
+  const float* row = x + (size_t)blockIdx.x * d;
+  float4 v[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = (threadIdx.x + k * CTA_THREADS) * 4;
+    v[k] = i < d ? __ldcg(reinterpret_cast<const float4*>(row + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  cta_norm_store<NV>(v, w, out + (size_t)blockIdx.x * d, d, eps, act_f16, sm);
 }
 
 __global__ void __launch_bounds__(ROWS_PER_CTA * 32)
@@ -116,8 +192,46 @@ embed_norm_kernel(EmbedArgs a) {
   row_norm_store(x, a.ln_w, a.xn16 + (size_t)row * a.d, a.d, a.eps, a.act_f16, lane);
 }
 
-// GridStateUpdater.update (src/inference.py:127-168) for one sequence, then the
-// embedding of the fed token and the first RMSNorm of the step.
+// GridStateUpdater.update (src/inference.py:127-168) for sequence b after token tok.
+__device__ __forceinline__ void grid_step(const DecodeState& st, int b, int tok) {
+  int x = st.gx[b], y = st.gy[b], in_out = st.gin[b];
+  const bool is_start = tok == TOK_START, is_sep = tok == TOK_IOSEP, is_end = tok == TOK_END,
+             is_nl = tok == TOK_NEWLINE, is_color = tok < 10;
+  int z = in_out ? 3 : 1;
+  if (is_start) z = 0;
+  if (is_sep) z = 2;
+  if (is_end) z = 4;
+  const int xc = min(max(x, 0), 30), yc = min(max(y, 0), 29);
+  st.pos[3 * b + 0] = (is_start || is_sep || is_end || is_nl) ? 0 : xc;
+  st.pos[3 * b + 1] = (is_start || is_sep || is_end) ? 0 : yc;
+  st.pos[3 * b + 2] = z;
+  if (is_start || is_sep) { x = 0; y = 0; }
+  if (is_start) in_out = 0;
+  if (is_sep) in_out = 1;
+  if (is_nl) { x = 0; y = min(y + 1, 29); }
+  if (is_color) x = min(x + 1, 30);
+  st.gx[b] = min(max(x, 0), 30);
+  st.gy[b] = min(max(y, 0), 29);
+  st.gin[b] = in_out;
+  const int len = st.cur_len[b];
+  if (len >= st.t_max) {
+    // cache row is full: drop the key and attend to what is there
+    arcb_set_error(st.err, ARCB_DEV_BAD_INDEX);
+    st.slot[b] = -1;
+    st.kv_len[b] = st.t_max;
+  } else {
+    st.slot[b] = len;
+    st.kv_len[b] = len + 1;
+  }
+}
+
+__device__ __forceinline__ const float* example_row(const EmbedArgs& a, int b) {
+  if (!a.example_ids) return nullptr;
+  const int ex = min(max(a.example_ids[b], 0), a.num_examples - 1);
+  return a.example_embed + (size_t)ex * a.d;
+}
+
+// Grid state, then the embedding of the fed token and the first RMSNorm of the step; one warp or one CTA per sequence.
 __global__ void __launch_bounds__(ROWS_PER_CTA * 32)
 decode_begin_kernel(DecodeState st, EmbedArgs a) {
   pdl_launch_dependents();
@@ -126,78 +240,30 @@ decode_begin_kernel(DecodeState st, EmbedArgs a) {
   if (b >= st.n_seqs) return;
   const int lane = threadIdx.x & 31;
   const int tok = st.cur_tok[b];
-  if (lane == 0) {
-    int x = st.gx[b], y = st.gy[b], in_out = st.gin[b];
-    const bool is_start = tok == TOK_START, is_sep = tok == TOK_IOSEP, is_end = tok == TOK_END,
-               is_nl = tok == TOK_NEWLINE, is_color = tok < 10;
-    int z = in_out ? 3 : 1;
-    if (is_start) z = 0;
-    if (is_sep) z = 2;
-    if (is_end) z = 4;
-    const int xc = min(max(x, 0), 30), yc = min(max(y, 0), 29);
-    st.pos[3 * b + 0] = (is_start || is_sep || is_end || is_nl) ? 0 : xc;
-    st.pos[3 * b + 1] = (is_start || is_sep || is_end) ? 0 : yc;
-    st.pos[3 * b + 2] = z;
-    if (is_start || is_sep) { x = 0; y = 0; }
-    if (is_start) in_out = 0;
-    if (is_sep) in_out = 1;
-    if (is_nl) { x = 0; y = min(y + 1, 29); }
-    if (is_color) x = min(x + 1, 30);
-    st.gx[b] = min(max(x, 0), 30);
-    st.gy[b] = min(max(y, 0), 29);
-    st.gin[b] = in_out;
-    const int len = st.cur_len[b];
-    if (len >= st.t_max) {
-      // cache row is full: drop the key and attend to what is there
-      arcb_set_error(st.err, ARCB_DEV_BAD_INDEX);
-      st.slot[b] = -1;
-      st.kv_len[b] = st.t_max;
-    } else {
-      st.slot[b] = len;
-      st.kv_len[b] = len + 1;
-    }
-  }
+  if (lane == 0) grid_step(st, b, tok);
   const int tk = min(max(tok, 0), a.vocab - 1);
-  const float* ex_row = nullptr;
-  if (a.example_ids) {
-    int ex = a.example_ids[b];
-    ex = min(max(ex, 0), a.num_examples - 1);
-    ex_row = a.example_embed + (size_t)ex * a.d;
-  }
   float* x = a.x + (size_t)b * a.d;
-  row_embed(x, a.token_embed + (size_t)tk * a.d, ex_row, a.d, lane);
+  row_embed(x, a.token_embed + (size_t)tk * a.d, example_row(a, b), a.d, lane);
   row_norm_store(x, a.ln_w, a.xn16 + (size_t)b * a.d, a.d, a.eps, a.act_f16, lane);
 }
 
-__global__ void __launch_bounds__(ROWS_PER_CTA * 32)
-head_kernel(HeadArgs a, DecodeState st) {
+template <int NV>
+__global__ void __launch_bounds__(CTA_THREADS)
+decode_begin_cta_kernel(DecodeState st, EmbedArgs a) {
   pdl_launch_dependents();
   pdl_wait();
-  const int i = blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5);
-  if (i >= a.rows) return;
-  const int lane = threadIdx.x & 31;
-  const int row = a.row_index ? a.row_index[i] : i;
-  const float* x = a.x + (size_t)row * a.d;
-  const float ss = row_sumsq(x, a.d, lane);
-  const float inv = rsqrtf(ss / (float)a.d + a.eps);
-  float acc[ARCB_VOCAB];
-#pragma unroll
-  for (int v = 0; v < ARCB_VOCAB; ++v) acc[v] = 0.f;
-  for (int c = lane * 4; c < a.d; c += 128) {
-    const float4 xv = *reinterpret_cast<const float4*>(x + c);
-    const float4 g = __ldg(reinterpret_cast<const float4*>(a.lnf_w + c));
-    const float n0 = (xv.x * inv) * g.x, n1 = (xv.y * inv) * g.y, n2 = (xv.z * inv) * g.z,
-                n3 = (xv.w * inv) * g.w;
-#pragma unroll
-    for (int v = 0; v < ARCB_VOCAB; ++v) {
-      const float4 w = __ldg(reinterpret_cast<const float4*>(a.lm_head + (size_t)v * a.d + c));
-      acc[v] += n0 * w.x + n1 * w.y + n2 * w.z + n3 * w.w;
-    }
-  }
-#pragma unroll
-  for (int v = 0; v < ARCB_VOCAB; ++v) acc[v] = warp_sum(acc[v]);
-  if (lane != 0) return;
+  __shared__ float sm[4];
+  const int b = blockIdx.x;
+  const int tok = st.cur_tok[b];
+  const int tk = min(max(tok, 0), a.vocab - 1);
+  float4 v[NV];
+  cta_embed<NV>(v, a.x + (size_t)b * a.d, a.token_embed + (size_t)tk * a.d, example_row(a, b), a.d);
+  if (threadIdx.x == CTA_THREADS - 1) grid_step(st, b, tok);   // a thread with the fewest columns
+  cta_norm_store<NV>(v, a.ln_w, a.xn16 + (size_t)b * a.d, a.d, a.eps, a.act_f16, sm);
+}
 
+// Argmax, and in the generating modes the bookkeeping of row i; one thread.
+__device__ __forceinline__ void head_finish(const HeadArgs& a, const DecodeState& st, int i, const float (&acc)[ARCB_VOCAB]) {
   int best = 0;
   float bv = acc[0];
 #pragma unroll
@@ -314,6 +380,85 @@ head_kernel(HeadArgs a, DecodeState st) {
   st.cur_tok[b] = tok;
 }
 
+__global__ void __launch_bounds__(ROWS_PER_CTA * 32)
+head_kernel(HeadArgs a, DecodeState st) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int i = blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5);
+  if (i >= a.rows) return;
+  const int lane = threadIdx.x & 31;
+  const int row = a.row_index ? a.row_index[i] : i;
+  const float* x = a.x + (size_t)row * a.d;
+  const float ss = row_sumsq(x, a.d, lane);
+  const float inv = rsqrtf(ss / (float)a.d + a.eps);
+  float acc[ARCB_VOCAB];
+#pragma unroll
+  for (int v = 0; v < ARCB_VOCAB; ++v) acc[v] = 0.f;
+  for (int c = lane * 4; c < a.d; c += 128) {
+    const float4 xv = *reinterpret_cast<const float4*>(x + c);
+    const float4 g = __ldg(reinterpret_cast<const float4*>(a.lnf_w + c));
+    const float n0 = (xv.x * inv) * g.x, n1 = (xv.y * inv) * g.y, n2 = (xv.z * inv) * g.z,
+                n3 = (xv.w * inv) * g.w;
+#pragma unroll
+    for (int v = 0; v < ARCB_VOCAB; ++v) {
+      const float4 w = __ldg(reinterpret_cast<const float4*>(a.lm_head + (size_t)v * a.d + c));
+      acc[v] += n0 * w.x + n1 * w.y + n2 * w.z + n3 * w.w;
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < ARCB_VOCAB; ++v) acc[v] = warp_sum(acc[v]);
+  if (lane == 0) head_finish(a, st, i, acc);
+}
+
+// One CTA of eight warps per row: NV float4 of the row a thread, the 14 sums met in shared memory.
+constexpr int HEAD_THREADS = 256;
+template <int NV>
+__global__ void __launch_bounds__(HEAD_THREADS)
+head_cta_kernel(HeadArgs a, DecodeState st) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float sm[HEAD_THREADS / 32][16];
+  const int i = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* x = a.x + (size_t)(a.row_index ? a.row_index[i] : i) * a.d;
+  // the norm's factor is the same for all columns: it multiplies the finished sums
+  float part[15];
+#pragma unroll
+  for (int v = 0; v < 15; ++v) part[v] = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int c = (tid + k * HEAD_THREADS) * 4;
+    if (c < a.d) {
+      const float4 xv = __ldcg(reinterpret_cast<const float4*>(x + c));
+      const float4 g = __ldg(reinterpret_cast<const float4*>(a.lnf_w + c));
+      part[14] += (xv.x * xv.x + xv.y * xv.y) + (xv.z * xv.z + xv.w * xv.w);
+      const float4 n = make_float4(xv.x * g.x, xv.y * g.y, xv.z * g.z, xv.w * g.w);
+#pragma unroll
+      for (int v = 0; v < ARCB_VOCAB; ++v) {
+        const float4 w = __ldg(reinterpret_cast<const float4*>(a.lm_head + (size_t)v * a.d + c));
+        part[v] += (n.x * w.x + n.y * w.y) + (n.z * w.z + n.w * w.w);
+      }
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < 15; ++v) {
+    const float s = warp_sum(part[v]);
+    if (lane == 0) sm[warp][v] = s;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  float s = 0.f;
+  if (lane < 15) {
+#pragma unroll
+    for (int w = 0; w < HEAD_THREADS / 32; ++w) s += sm[w][lane];
+  }
+  const float inv = rsqrtf(__shfl_sync(0xffffffffu, s, 14) / (float)a.d + a.eps);
+  s *= inv;
+  float acc[ARCB_VOCAB];
+#pragma unroll
+  for (int v = 0; v < ARCB_VOCAB; ++v) acc[v] = __shfl_sync(0xffffffffu, s, v);
+  if (lane == 0) head_finish(a, st, i, acc);
+}
+
 // dst row = (r / blk) * blk_stride + blk_off + r % blk.  Every value is first rounded to bf16 (the
 // model's precision); container: 0 = fp32, 1 = bf16, 2 = IEEE half holding the bf16-rounded value
 // (exact for |w| >= 2^-14, within 2^-25 absolute below; saturates at +-65504).
@@ -338,12 +483,19 @@ __global__ void pack_rows_kernel(const float* __restrict__ src, void* __restrict
 
 }  // namespace
 
+static bool cta_per_row(int rows, int d) { return rows <= CTA_ROW_MAX && d <= CTA_MAX_D; }
+
 int arcb_launch_rmsnorm(const float* x, const float* w, void* out16, int rows, int d, float eps,
                         int act_f16, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (d % 4) return -1;
-  const cudaError_t e = arcb_launch(rmsnorm_kernel, dim3((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), dim3(ROWS_PER_CTA * 32), 0,
-                                    stream, x, w, reinterpret_cast<uint16_t*>(out16), rows, d, eps, act_f16);
+  uint16_t* out = reinterpret_cast<uint16_t*>(out16);
+  auto cta = [&](auto kernel) { return arcb_launch(kernel, dim3(rows), dim3(CTA_THREADS), 0, stream, x, w, out, d, eps, act_f16); };
+  const cudaError_t e = !cta_per_row(rows, d) ? arcb_launch(rmsnorm_kernel, dim3((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
+                                                            dim3(ROWS_PER_CTA * 32), 0, stream, x, w, out, rows, d, eps, act_f16)
+                        : d <= CTA_THREADS * 4 ? cta(rmsnorm_cta_kernel<1>)
+                        : d <= CTA_THREADS * 8 ? cta(rmsnorm_cta_kernel<2>)
+                                               : cta(rmsnorm_cta_kernel<4>);
   arcb_count_launch(1);
   return (int)e;
 }
@@ -357,16 +509,23 @@ int arcb_launch_embed_norm(const EmbedArgs& a, cudaStream_t stream) {
 }
 
 int arcb_launch_decode_begin(const DecodeState& st, const EmbedArgs& a, cudaStream_t stream) {
-  const cudaError_t e = arcb_launch(decode_begin_kernel, dim3((st.n_seqs + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
-                                    dim3(ROWS_PER_CTA * 32), 0, stream, st, a);
+  auto cta = [&](auto kernel) { return arcb_launch(kernel, dim3(st.n_seqs), dim3(CTA_THREADS), 0, stream, st, a); };
+  const cudaError_t e = !cta_per_row(st.n_seqs, a.d) ? arcb_launch(decode_begin_kernel, dim3((st.n_seqs + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
+                                                                   dim3(ROWS_PER_CTA * 32), 0, stream, st, a)
+                        : a.d <= CTA_THREADS * 4 ? cta(decode_begin_cta_kernel<1>)
+                        : a.d <= CTA_THREADS * 8 ? cta(decode_begin_cta_kernel<2>)
+                                                 : cta(decode_begin_cta_kernel<4>);
   arcb_count_launch(1);
   return (int)e;
 }
 
 int arcb_launch_head(const HeadArgs& a, const DecodeState& st, cudaStream_t stream) {
   if (a.rows <= 0) return 0;
-  const cudaError_t e = arcb_launch(head_kernel, dim3((a.rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), dim3(ROWS_PER_CTA * 32),
-                                    0, stream, a, st);
+  auto cta = [&](auto kernel) { return arcb_launch(kernel, dim3(a.rows), dim3(HEAD_THREADS), 0, stream, a, st); };
+  const cudaError_t e = !cta_per_row(a.rows, a.d) ? arcb_launch(head_kernel, dim3((a.rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
+                                                                dim3(ROWS_PER_CTA * 32), 0, stream, a, st)
+                        : a.d <= HEAD_THREADS * 4 ? cta(head_cta_kernel<1>)
+                                                  : cta(head_cta_kernel<2>);
   arcb_count_launch(1);
   return (int)e;
 }

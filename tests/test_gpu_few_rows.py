@@ -1,0 +1,103 @@
+"""Kernels of steps with few rows, through the C ABI and small models, at the edges of their tiles and of the rules that
+choose them."""
+import math
+
+import pytest
+import torch
+
+from gpu_util import have_b200, stream, to_act
+from mdlarc_scale_b200 import _lib, registry
+from mdlarc_scale_b200.layered import Segment
+from oracle import vodavik as vo
+from vodavik_util import attention, config, mlstm, oracle_logits, rel_error, tokens
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_b200(), reason="needs a B200")]
+
+
+@pytest.fixture(scope="module")
+def lib():
+    return _lib.load()
+
+
+@pytest.mark.parametrize("d", [128, 640, 1280, 2048, 2176])
+@pytest.mark.parametrize("rows", [1, 2048, 2049])
+def test_row_kernels_on_both_sides_of_their_rules(lib, rows, d):
+    """Norm and head with a CTA per row (up to 2048 rows of 2048 columns) and with a warp per row beyond."""
+    g = torch.Generator(device="cuda").manual_seed(rows + d)
+    x = torch.randn(rows, d, device="cuda", generator=g) * 3
+    w = torch.randn(d, device="cuda", generator=g)
+    out = torch.empty(rows, d, device="cuda", dtype=torch.float16)
+    _lib.check(lib.arcb_op_rmsnorm(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, d, 1e-5, _lib.ACT_F16, stream()))
+    n = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    # half: 2^-11 of rounding (2^-25 where it is subnormal); fp32: a sum of d squares and four products
+    assert ((out.double() - n).abs() <= n.abs() * (2 ** -11 + 1e-6 * math.sqrt(d)) + 2 ** -24).all()
+    head = torch.randn(14, d, device="cuda", generator=g) * d ** -0.5
+    logits = torch.empty(rows, 14, device="cuda")
+    am = torch.empty(rows, dtype=torch.int32, device="cuda")
+    _lib.check(lib.arcb_op_head(x.data_ptr(), None, w.data_ptr(), head.data_ptr(), logits.data_ptr(), am.data_ptr(), rows, d, 1e-5, stream()))
+    ref = n @ head.double().T
+    bound = (n.abs() @ head.double().abs().T) * 2 ** -24 * (d / 32 + 16)    # longest chain of additions
+    assert ((logits.double() - ref).abs() <= bound).all()
+    assert torch.equal(am.long(), logits.argmax(-1))
+
+
+@pytest.mark.parametrize("splits", [31, 32, 33, 64])
+def test_split_merge(lib, splits):
+    """Two lanes' worth of splits, some of them without keys."""
+    B, H, T = 2, 3, 700
+    g = torch.Generator(device="cuda").manual_seed(splits)
+    q = to_act(torch.randn(B, H, 64, device="cuda", generator=g), _lib.ACT_F16)
+    k, v = (torch.randn(B, H, T, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    lens = torch.tensor([700, 35], dtype=torch.int32, device="cuda")
+    out = torch.empty_like(q)
+    scratch = torch.empty(lib.arcb_attn_scratch_bytes(B, H, splits), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.arcb_op_decode_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), None, lens.data_ptr(), None, B, H, T,
+                                            splits, scratch.data_ptr(), _lib.ACT_F16, stream()))
+    for i, n in enumerate(lens.tolist()):
+        p = torch.softmax(torch.einsum("hd,htd->ht", q[i].double(), k[i, :, :n].double()) / 8, -1)
+        ref = torch.einsum("ht,htd->hd", p, v[i, :, :n].double())
+        assert ((out[i].double() - ref).abs() <= ref.abs() * 2 ** -11 + 1e-5).all()
+
+
+@pytest.mark.parametrize("fmt", [_lib.ACT_F16, _lib.ACT_BF16])
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64, 65])
+@pytest.mark.parametrize("N,K", [(128, 64), (384, 256), (1280, 704), (1024, 3392)])
+def test_few_row_products(lib, M, N, K, fmt):
+    """Row tiles of 8, 16, 32 and 64 and one row beyond; K of fewer blocks than warps, and of more than are in flight."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = to_act(torch.randn(M, K, device="cuda", generator=g), fmt)
+    w = to_act((torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).to(torch.bfloat16).float(), fmt)
+    bias = torch.randn(N, device="cuda", generator=g)
+    ref = a.double() @ w.double().T
+    bound = (a.double().abs() @ w.double().abs().T) * 2 ** -24 * (K / 16 + 16)
+    y = torch.full((M + 1, N), 7.0, device="cuda")
+    _lib.check(lib.arcb_op_gemm(a.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, K, fmt, _lib.GEMM_AUTO, stream()))
+    assert ((y[:M].double() - ref).abs() <= bound).all() and (y[M] == 7).all()
+    x0 = torch.randn(M + 1, N, device="cuda", generator=g)
+    got = []
+    for _ in range(2):
+        x = x0.clone()
+        _lib.check(lib.arcb_op_gemm_residual(a.data_ptr(), w.data_ptr(), bias.data_ptr(), x.data_ptr(), M, N, K, fmt, _lib.GEMM_AUTO, stream()))
+        got.append(x)
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0][M], x0[M])
+    ref = ref + x0[:M].double() + bias.double()
+    assert ((got[0][:M].double() - ref).abs() <= bound + (ref.abs() + x0[:M].double().abs() + bias.double().abs()) * 2 ** -22).all()
+
+
+# widths whose norms hold a row in one to eight registers a thread, and one beyond; a vocabulary off and on quads of columns
+@pytest.mark.parametrize("width,vocab", [(500, 333), (1000, 332), (2050, 96), (4100, 64)])
+def test_layered_steps_of_few_rows(width, vocab):
+    cfg = config(width, vocab, [attention(4, 2, 64, 64, ff=200), mlstm(2, 64, 64)])
+    w = vo.random_weights(cfg, width)
+    toks = tokens(cfg, 70, 3)
+    want = oracle_logits(cfg, w, toks)
+    for fmt, tol in (("f32", 3e-5), ("f16", 1e-2), ("bf16", 6e-2)):
+        eng = registry.build_engine(cfg, w, "cuda:0", fmt)
+        for first in (1, 9, 40, 66):
+            s = eng.new_session(3, 70, 1, 70, stop_on_end=False)
+            slot = s.acquire()
+            rows = [s.step([Segment(slot, toks[:first], list(range(first)))])[0]]
+            rows += [s.step([Segment(slot, [t], [0])])[0] for t in toks[first:]]
+            s.poll()
+            s.close()
+            assert rel_error(torch.cat(rows), want) < tol
