@@ -8,10 +8,9 @@
 //
 // With n_splits > 1 every split writes (m, l, acc[64]) to scratch and a second kernel merges
 // the splits; with n_splits == 1 the normalised output is written directly.
-#include <cstdlib>
-
 #include "attn_stream.cuh"
 #include "launch.cuh"
+#include "ptx_sm100.cuh"
 
 namespace {
 
@@ -191,12 +190,18 @@ attn_stream_kernel(AttnStreamArgs a) {
 constexpr int COOP_WARPS = 4;
 constexpr int COOP_ROWS = 32;
 
-template <int WARPS, int ROWS, int MIN_CTAS>
+// CLUSTER: the splits of one (item, head) are the CTAs of a cluster.  They leave their partials in the first one's shared
+// memory, which merges them in the splits' order: no scratch and no merge launch.  B200, attention with its merge, us a layer:
+// 6 sequences x 20 heads over 5.2 k rows 35.7 (five splits and a merge launch) -> 27.9 (four), one sequence x 4 heads over
+// 190 rows 8.6 (32 one-warp splits) -> 3.3 (one).
+template <int WARPS, int ROWS, int MIN_CTAS, bool CLUSTER>
 __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS)
 attn_stream_coop_kernel(AttnStreamArgs a) {
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ float s_part[WARPS][ATTN_SCRATCH_STRIDE];
+  __shared__ float s_split[CLUSTER ? ATTN_CLUSTER_MAX : 1][ATTN_SCRATCH_STRIDE];
+  if constexpr (CLUSTER) sm100::cluster_arrive();      // every CTA has started before any writes to another's memory
+  pdl_wait();
   const int lane = threadIdx.x & 31, wj = threadIdx.x >> 5;
   const long long w = blockIdx.x;                       // grid = n_items * n_heads * n_splits exactly
   const int split = (int)(w % a.n_splits);
@@ -309,7 +314,8 @@ attn_stream_coop_kernel(AttnStreamArgs a) {
     }
   }
   __syncthreads();
-  if (wj != 0) return;
+  if constexpr (CLUSTER) sm100::cluster_wait();
+  if (!CLUSTER && wj != 0) return;
   // warp 0: merge the warps' partials in a fixed order; lane d holds dims 2d, 2d + 1
   float mt = -INFINITY;
 #pragma unroll
@@ -324,7 +330,31 @@ attn_stream_coop_kernel(AttnStreamArgs a) {
     o0 += v.x * sc;
     o1 += v.y * sc;
   }
-  if (a.n_splits == 1) {
+  if constexpr (CLUSTER) {
+    if (wj == 0) {
+      const uint32_t rec = sm100::smem_u32(s_split[split]);
+      sm100::st_shared_cluster_f32(rec + 8 * lane, 0, o0);
+      sm100::st_shared_cluster_f32(rec + 8 * lane + 4, 0, o1);
+      if (lane == 0) {
+        sm100::st_shared_cluster_f32(rec + 4 * 64, 0, mt);
+        sm100::st_shared_cluster_f32(rec + 4 * 65, 0, lt);
+      }
+    }
+    sm100::cluster_sync_all();
+    if (split != 0 || wj != 0) return;
+    mt = -INFINITY;
+    for (int s = 0; s < a.n_splits; ++s) mt = fmaxf(mt, s_split[s][64]);
+    const float safe = (mt == -INFINITY) ? 0.f : mt;
+    lt = o0 = o1 = 0.f;
+    for (int s = 0; s < a.n_splits; ++s) {
+      const float sc = exp2f(s_split[s][64] - safe);
+      const float2 v = *reinterpret_cast<const float2*>(&s_split[s][2 * lane]);
+      lt += s_split[s][65] * sc;
+      o0 += v.x * sc;
+      o1 += v.y * sc;
+    }
+  }
+  if (CLUSTER || a.n_splits == 1) {
     const float inv = (lt > 0.f) ? 1.f / lt : 0.f;
     uint32_t* op = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(a.out16) + (size_t)ih * ARCB_HEAD_DIM) + lane;
     *op = pack2_act(o0 * inv, o1 * inv, a.act_f16);
@@ -376,19 +406,25 @@ attn_combine_kernel(AttnStreamArgs a) {
 
 int arcb_launch_attn_stream(const AttnStreamArgs& a, cudaStream_t stream) {
   if (a.n_items <= 0) return 0;
-  if (a.n_splits < 1 || a.n_splits > 64 || (a.n_splits > 1 && !a.scratch)) return -1;
+  if (a.n_splits < 1 || a.n_splits > 64) return -1;
   const long long n_work = (long long)a.n_items * a.n_heads * a.n_splits;
   const long long blocks = (n_work + WARPS_PER_CTA - 1) / WARPS_PER_CTA;
   if (blocks > 0x7fffffffLL) return -1;
-  // enough (item, head, split) work items for two CTAs per SM, and a cache whose per-split share can fill
-  // one CTA iteration (4 x 32 rows): one CTA per item (see the kernel's comment); launches over a few
-  // dozen rows per split keep one warp per item (13.4 against 14.9 ms for 15 decode steps of 16 sequences)
-  static const int coop_min = [] { const char* e = getenv("ARCB_ATTN_COOP_MIN"); return e ? atoi(e) : 296; }();  // A/B switch; < 0 disables
+  // Where the cache has a CTA iteration (4 x 32 rows) per split: two to eight splits are the CTAs of a cluster; one split,
+  // or enough work items for two CTAs per SM, a CTA per item (see the kernel's comment).  Many splits of a few dozen rows
+  // keep a warp per item (13.4 against 14.9 ms for 15 decode steps of 16 sequences).
+  const bool coop = n_work <= 0x7fffffffLL && (long long)a.t_max >= (long long)COOP_WARPS * COOP_ROWS * a.n_splits;
   cudaError_t e;
-  if (coop_min >= 0 && n_work >= coop_min && n_work <= 0x7fffffffLL &&
-      (long long)a.t_max >= (long long)COOP_WARPS * COOP_ROWS * a.n_splits) {
-    e = arcb_launch(attn_stream_coop_kernel<COOP_WARPS, COOP_ROWS, 4>, dim3((unsigned)n_work), dim3(COOP_WARPS * 32), 0, stream, a);
-  } else
+  if (coop && a.n_splits > 1 && a.n_splits <= ATTN_CLUSTER_MAX) {
+    e = arcb_launch_cluster(attn_stream_coop_kernel<COOP_WARPS, COOP_ROWS, 4, true>, a.n_splits, dim3((unsigned)n_work),
+                            dim3(COOP_WARPS * 32), 0, stream, a);
+    arcb_count_launch(1);
+    return (int)e;
+  }
+  if (a.n_splits > 1 && !a.scratch) return -1;
+  if (coop && (n_work >= 296 || a.n_splits == 1))
+    e = arcb_launch(attn_stream_coop_kernel<COOP_WARPS, COOP_ROWS, 4, false>, dim3((unsigned)n_work), dim3(COOP_WARPS * 32), 0, stream, a);
+  else
     e = arcb_launch(attn_stream_kernel, dim3((unsigned)blocks), dim3(WARPS_PER_CTA * 32), 0, stream, a);
   arcb_count_launch(1);
   if (e == cudaSuccess && a.n_splits > 1) {

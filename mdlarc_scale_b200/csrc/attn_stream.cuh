@@ -2,6 +2,7 @@
 #pragma once
 #include "common.cuh"
 
+constexpr int ATTN_CLUSTER_MAX = 8;      // splits that are merged inside the launch
 constexpr int ATTN_SCRATCH_STRIDE = 68;  // floats per (item, head, split): 64 acc, m, l, pad
 
 struct AttnStreamArgs {

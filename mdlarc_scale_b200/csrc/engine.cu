@@ -194,25 +194,23 @@ static bool engine_complete(const arcb_engine* e) {
 // ---------------------------------------------------------------------------
 // session
 // ---------------------------------------------------------------------------
-// Split count of decode attention.  t_max = 0: the upper bound used to size the scratch (one warp per
-// work item); with the session's cache capacity known, fewer splits when the launch qualifies for the
-// kernel that puts four warps on every work item (attn_stream.cu), which also spares small batches
-// the merge launch.
-static int choose_splits(const arcb_engine* e, int n_seqs, int requested, int t_max = 0) {
+// Split count of decode attention for a cache of t_max rows: up to eight splits of at least two CTA iterations (256 rows),
+// which one launch merges in clusters.  An SM holds four of its CTAs, so a launch takes as long as its waves of 592 times
+// the rows of a split: the count with the shortest such time is taken, within the first wave if that is 10 % less than with
+// fewer splits, beyond it only if it is 30 % less (2048 items: 39 us unsplit, 48 in two splits).
+// `requested` > 0 is the caller's choice (and the only one that may need scratch).
+static int choose_splits(const arcb_engine* e, int n_seqs, int requested, int t_max) {
   if (requested > 0) return requested > 64 ? 64 : requested;
-  // aim for ~16 resident warps on each of the 148 SMs
   const long long work = (long long)n_seqs * e->cfg.n_heads;
-  long long s = (148LL * 16 + work - 1) / work;
-  if (s < 1) s = 1;
-  if (s > 32) s = 32;
-  static const bool coop_splits = [] { const char* v = getenv("ARCB_COOP_SPLITS"); return !(v && v[0] == '0'); }();  // A/B switch
-  if (t_max > 0 && coop_splits) {
-    long long s4 = (148LL * 4 + work - 1) / work;
-    if (s4 < 1) s4 = 1;
-    if (s4 < s && work * s4 >= 296 && (long long)t_max >= 128 * s4) return (int)s4;
+  int best = 1;
+  double best_time = 0.;
+  for (int s = 1; s <= ATTN_CLUSTER_MAX && (s == 1 || 256LL * s <= t_max); ++s) {
+    const double time = (double)((work * s + 591) / 592) / s;
+    if (s == 1 || time < (work * s <= 592 ? 0.9 : 0.7) * best_time) { best = s; best_time = time; }
   }
-  return (int)s;
+  return best;
 }
+static int scratch_splits(int requested) { return requested > 64 ? 64 : requested > 1 ? requested : 1; }
 
 struct WsLayout {
   size_t x, xn, q, attn, h, k16, v16, scratch, gemm_scratch, ints, total;
@@ -247,7 +245,7 @@ extern "C" int64_t arcb_session_workspace_bytes(const arcb_engine* e, int32_t n_
                                                 int32_t max_prefill_tokens, int32_t attn_splits) {
   if (!e || n_seqs <= 0 || max_prefill_tokens < 0) return -1;
   if (e->lm) return lm_workspace_bytes(e, n_seqs, max_prefill_tokens, attn_splits);
-  return (int64_t)ws_layout(e, n_seqs, max_prefill_tokens, choose_splits(e, n_seqs, attn_splits)).total;
+  return (int64_t)ws_layout(e, n_seqs, max_prefill_tokens, scratch_splits(attn_splits)).total;
 }
 
 extern "C" int64_t arcb_kv_cache_bytes(const arcb_engine* e, int32_t n_seqs, int32_t t_max) {
@@ -282,7 +280,7 @@ extern "C" int arcb_session_create(arcb_engine* e, const arcb_session_desc* dsc,
     return ARCB_OK;
   }
   const int splits = choose_splits(e, dsc->n_seqs, dsc->attn_splits, dsc->t_max);
-  const WsLayout w = ws_layout(e, dsc->n_seqs, dsc->max_prefill_tokens, choose_splits(e, dsc->n_seqs, dsc->attn_splits));
+  const WsLayout w = ws_layout(e, dsc->n_seqs, dsc->max_prefill_tokens, scratch_splits(dsc->attn_splits));
   if ((size_t)dsc->workspace_bytes < w.total) return arcb_fail(ARCB_E_ARG, "workspace too small");
   arcb_session* s = new arcb_session();
   s->eng = e;
@@ -296,7 +294,7 @@ extern "C" int arcb_session_create(arcb_engine* e, const arcb_session_desc* dsc,
   s->h16 = reinterpret_cast<uint16_t*>(base + w.h);
   s->k16 = reinterpret_cast<uint16_t*>(base + w.k16);
   s->v16 = reinterpret_cast<uint16_t*>(base + w.v16);
-  s->attn_scratch = splits > 1 ? reinterpret_cast<float*>(base + w.scratch) : nullptr;
+  s->attn_scratch = dsc->attn_splits > 1 ? reinterpret_cast<float*>(base + w.scratch) : nullptr;
   s->gemm_scratch = reinterpret_cast<float*>(base + w.gemm_scratch);
   int* ints = reinterpret_cast<int*>(base + w.ints);
   const int B = dsc->n_seqs;

@@ -21,21 +21,36 @@ void arcb_pdl_set(bool on);
 void arcb_pdl_suppress(bool on);
 bool arcb_pdl_suppressed();
 
+// `cluster` > 1: CTAs x, x + 1, ... of the grid form clusters of that many (the kernel carries no cluster size of its own).
 template <typename... KArgs, typename... Args>
-inline cudaError_t arcb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                               Args&&... args) {
+inline cudaError_t arcb_launch_cluster(void (*kernel)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                       Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  const bool pdl = arcb_pdl_enabled() && !arcb_pdl_suppressed();
-  cfg.attrs = pdl ? attr : nullptr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  unsigned n = 0;
+  if (arcb_pdl_enabled() && !arcb_pdl_suppressed()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = n ? attr : nullptr;
+  cfg.numAttrs = n;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
   if (e != cudaSuccess) cudaGetLastError();   // reported through the return value; do not leave it for the next API call
   return e;
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t arcb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                               Args&&... args) {
+  return arcb_launch_cluster(kernel, 1, grid, block, smem, stream, std::forward<Args>(args)...);
 }

@@ -275,6 +275,32 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// fp32 at this CTA's shared address `addr`, of CTA `rank` of the cluster
+__device__ __forceinline__ float ld_shared_cluster_f32(uint32_t addr, uint32_t rank) {
+  float v;
+  asm volatile(
+      "{\n"
+      ".reg .b32 a;\n"
+      "mapa.shared::cluster.u32 a, %1, %2;\n"
+      "ld.shared::cluster.f32 %0, [a];\n"
+      "}\n"
+      : "=f"(v)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared_cluster_f32(uint32_t addr, uint32_t rank, float v) {
+  asm volatile(
+      "{\n"
+      ".reg .b32 a;\n"
+      "mapa.shared::cluster.u32 a, %0, %1;\n"
+      "st.shared::cluster.f32 [a], %2;\n"
+      "}\n" ::"r"(addr), "r"(rank), "f"(v)
+      : "memory");
+}
+// the two halves of cluster_sync_all
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

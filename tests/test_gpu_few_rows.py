@@ -59,6 +59,38 @@ def test_split_merge(lib, splits):
         assert ((out[i].double() - ref).abs() <= ref.abs() * 2 ** -11 + 1e-5).all()
 
 
+@pytest.mark.parametrize("T", [256, 1100])
+@pytest.mark.parametrize("splits", [1, 2, 5, 8])
+def test_splits_merged_in_a_cluster(lib, splits, T):
+    """Splits of a launch whose cache has 128 rows for each of them; fewer rows fall back to the merge launch.  Rows at the
+    edges of a split's 16-row granules, empty splits, skipped and empty items, permuted cache rows."""
+    lens_l = [n for n in (1, 15, 16, 17, 127, 129, 255, 256, 640, 1023, 1100, 0, 300) if n <= T]
+    B, H = len(lens_l), 3
+    g = torch.Generator(device="cuda").manual_seed(splits + T)
+    q = to_act(torch.randn(B, H, 64, device="cuda", generator=g), _lib.ACT_F16)
+    k, v = (torch.randn(B, H, T, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    lens = torch.tensor(lens_l, dtype=torch.int32, device="cuda")
+    seqs = torch.randperm(B, device="cuda", generator=g).to(torch.int32)
+    skip = torch.zeros(B, dtype=torch.uint8, device="cuda")
+    skip[2] = 1
+    scratch = torch.full((max(4, lib.arcb_attn_scratch_bytes(B, H, splits)),), 255, dtype=torch.uint8, device="cuda")
+    outs = []
+    for _ in range(2):
+        out = torch.full_like(q, float("nan"))
+        _lib.check(lib.arcb_op_decode_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), seqs.data_ptr(), lens.data_ptr(),
+                                                skip.data_ptr(), B, H, T, splits, scratch.data_ptr(), _lib.ACT_F16, stream()))
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    for i, n in enumerate(lens_l):
+        if n == 0 or i == 2:
+            assert (outs[0][i] == 0).all()
+            continue
+        s = int(seqs[i])
+        p = torch.softmax(torch.einsum("hd,htd->ht", q[i].double(), k[s, :, :n].double()) / 8, -1)
+        ref = torch.einsum("ht,htd->hd", p, v[s, :, :n].double())
+        assert ((outs[0][i].double() - ref).abs() <= ref.abs() * 2 ** -11 + 1e-5).all()
+
+
 @pytest.mark.parametrize("fmt", [_lib.ACT_F16, _lib.ACT_BF16])
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64, 65])
 @pytest.mark.parametrize("N,K", [(128, 64), (384, 256), (1280, 704), (1024, 3392)])
