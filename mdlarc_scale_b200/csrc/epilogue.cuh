@@ -171,15 +171,21 @@ __device__ __forceinline__ float2 rope_cs(const GemmEpilogue& e, const RopeRow& 
 
 // out[2p] = v[2p] cos - v[2p+1] sin ; out[2p+1] = v[2p+1] cos + v[2p] sin
 // (src/transformer.py:51-58, 184-185)
+// `cs0`, `cs1`: qkv_cs of the quad, which may be fetched long before the sums are there.
+__device__ __forceinline__ void qkv_cs(const GemmEpilogue& e, const RopeRow& r, int n, float2& cs0, float2& cs1) {
+  cs0 = cs1 = make_float2(1.f, 0.f);
+  if (n >= 2 * e.d_model) return;  // values do not turn
+  const int p = (n % e.d_model & 63) >> 1;
+  cs0 = rope_cs(e, r, p);
+  cs1 = rope_cs(e, r, p + 1);
+}
 __device__ __forceinline__ void epi_qkv_quad(const GemmEpilogue& e, const RopeRow& r, int m, int n,
-                                             float4 v) {
+                                             float4 v, float2 cs0, float2 cs1) {
   const int d = e.d_model;
   const int sec = n / d;           // 0 q, 1 k, 2 v
   const int c = n - sec * d;       // column inside the section
   const int h = c >> 6, dim = c & 63;
   if (sec < 2) {
-    const int p = dim >> 1;
-    const float2 cs0 = rope_cs(e, r, p), cs1 = rope_cs(e, r, p + 1);
     float4 o;
     o.x = v.x * cs0.x - v.y * cs0.y;
     o.y = v.y * cs0.x + v.x * cs0.y;
@@ -209,6 +215,11 @@ __device__ __forceinline__ void epi_qkv_quad(const GemmEpilogue& e, const RopeRo
       *reinterpret_cast<uint2*>(base16 + (size_t)r.row16 * d + c) = pk;
     }
   }
+}
+__device__ __forceinline__ void epi_qkv_quad(const GemmEpilogue& e, const RopeRow& r, int m, int n, float4 v) {
+  float2 cs0, cs1;
+  qkv_cs(e, r, n, cs0, cs1);
+  epi_qkv_quad(e, r, m, n, v, cs0, cs1);
 }
 
 // Rotate the 16 rotary pairs [P0, P0 + 16) held in v[0..32) (P0 is 0 or 16: first or second half of
@@ -279,15 +290,20 @@ __device__ __forceinline__ void epi_qkv_chunk32(const GemmEpilogue& e, const Rop
   }
 }
 
+// What a quad adds its sums to: the residual, and the bias of `n` (zero where there is none).
+__device__ __forceinline__ float4 resid_old(const GemmEpilogue& e, int m, int n) {
+  return e.overwrite ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(e.x + (size_t)m * e.N + n);
+}
+__device__ __forceinline__ float4 bias_quad(const GemmEpilogue& e, int n) {
+  return e.bias ? __ldg(reinterpret_cast<const float4*>(e.bias + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void epi_resid_quad(const GemmEpilogue& e, int m, int n, float4 v, float4 old, float4 b) {
+  if (e.bias) { v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
+  old.x += v.x; old.y += v.y; old.z += v.z; old.w += v.w;
+  *reinterpret_cast<float4*>(e.x + (size_t)m * e.N + n) = old;
+}
 __device__ __forceinline__ void epi_resid_quad(const GemmEpilogue& e, int m, int n, float4 v) {
-  float4* px = reinterpret_cast<float4*>(e.x + (size_t)m * e.N + n);
-  float4 r = e.overwrite ? make_float4(0.f, 0.f, 0.f, 0.f) : *px;
-  if (e.bias) {
-    const float4 b = __ldg(reinterpret_cast<const float4*>(e.bias + n));
-    v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-  }
-  r.x += v.x; r.y += v.y; r.z += v.z; r.w += v.w;
-  *px = r;
+  epi_resid_quad(e, m, n, v, resid_old(e, m, n), bias_quad(e, n));
 }
 
 __device__ __forceinline__ void epi_store_quad(const GemmEpilogue& e, int m, int n, float4 v) {
@@ -306,10 +322,8 @@ __device__ __forceinline__ float silu_f(float g) { return __fdividef(g, 1.f + __
 
 // Packed column n (n % 128 < 64) holds gate outputs, n + 64 the matching up outputs.
 __device__ __forceinline__ void epi_swiglu_quad(const GemmEpilogue& e, int m, int n, float4 g,
-                                                float4 u) {
+                                                float4 u, float4 bg, float4 bu) {
   if (e.bias) {
-    const float4 bg = __ldg(reinterpret_cast<const float4*>(e.bias + n));
-    const float4 bu = __ldg(reinterpret_cast<const float4*>(e.bias + n + 64));
     g.x += bg.x; g.y += bg.y; g.z += bg.z; g.w += bg.w;
     u.x += bu.x; u.y += bu.y; u.z += bu.z; u.w += bu.w;
   }
@@ -318,6 +332,10 @@ __device__ __forceinline__ void epi_swiglu_quad(const GemmEpilogue& e, int m, in
   pk.x = pack2_act_chk(silu_f(g.x) * u.x, silu_f(g.y) * u.y, e.act_f16, e.err);
   pk.y = pack2_act_chk(silu_f(g.z) * u.z, silu_f(g.w) * u.w, e.act_f16, e.err);
   *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(e.out16) + (size_t)m * (e.N >> 1) + j) = pk;
+}
+
+__device__ __forceinline__ void epi_swiglu_quad(const GemmEpilogue& e, int m, int n, float4 g, float4 u) {
+  epi_swiglu_quad(e, m, n, g, u, bias_quad(e, n), bias_quad(e, n + 64));
 }
 
 // first A row of a row tile

@@ -8,12 +8,17 @@
 //     activation row straight into registers, in the order that mma.m16n8k16 wants its fragments once K is permuted
 //     the same way in both operands (weights are the 16-row operand, activations the 8-column one);
 //   * the first blocks' weights are requested before the wait for the previous kernel (programmatic dependent launch):
-//     they depend on nothing;
+//     they depend on nothing; what the epilogue needs besides the sums (old residual, biases, rotations) is requested
+//     with the first activations, not behind the last sum;
 //   * the eight warps' sums meet in shared memory, always in the same order, and leave through the epilogues' quads.
+// B200, us a launch inside the captured step, tcgen05 tiles / here: 16 rows, QKV of width 1024 10.3 / 4.6, gate/up 10.6 / 5.4,
+// out and down 10.7 / 3.9; 1 row of width 256 6.1 to 6.8 / 1.9 to 2.4; 1 row, mixer projection of width 1280 14.2 / 6.5, its
+// 32 000-column head 26 / 18 (82 MB: 4.6 TB/s); 48 rows of width 1280, outputs 10.9 / 9.0, gated units 12.7 / 10.5.
 #include "common.cuh"
 #include "gemm.cuh"
 #include "gemm_rows.cuh"
 #include "launch.cuh"
+#include "ptx_sm100.cuh"
 
 namespace {
 
@@ -24,9 +29,15 @@ template <int NT, int MT>
 struct GrCfg {
   static constexpr int PITCH = 16 * NT + 4;          // floats: 8 x 4 consecutive accumulators fall on 32 banks
   static constexpr int ROWS = 8 * MT;
-  static constexpr int SMEM = GR_WARPS * ROWS * PITCH * 4;
-  static constexpr int WD = NT == 1 ? 6 : NT == 2 ? 4 : 2;   // weight blocks in flight a warp
-  static constexpr int XD = MT <= 2 ? WD : MT == 4 ? 2 : 1;  // activation blocks in flight; divides WD
+  // Blocks of K in flight a warp: weights in registers, activations in registers up to 16 rows and in shared memory beyond
+  // (asynchronous copies; a lane reads back only its own bytes, so there is no barrier).  Two CTAs fit an SM in every form,
+  // which makes products of up to 2 x 148 column tiles one wave.
+  static constexpr bool RING = MT >= 4;
+  static constexpr int WD = NT == 1 ? (MT <= 2 ? 6 : 3) : MT <= 4 ? 3 : 2;
+  static constexpr int XD = RING ? (MT == 4 ? 4 : 3) : WD;
+  static constexpr int RING_BYTES = RING ? GR_WARPS * XD * MT * 512 : 0;
+  static constexpr int SUM_BYTES = GR_WARPS * ROWS * PITCH * 4;     // the sums take the ring's place
+  static constexpr int SMEM = RING_BYTES > SUM_BYTES ? RING_BYTES : SUM_BYTES;
 };
 
 template <bool F16>
@@ -55,13 +66,99 @@ __device__ __forceinline__ int gr_col(int blk, int nt) {
   return (blk * NT + nt) * 16;
 }
 
+// What a quad's epilogue needs besides its sums, fetched while the products are still on their way.
+struct GrAhead {
+  float4 a, b;
+  RopeRow rr;
+  template <int MODE>
+  __device__ __forceinline__ void load(const GemmEpilogue& ep, int m, int n) {
+    if constexpr (MODE == EPI_RESID) {
+      a = resid_old(ep, m, n);
+      b = bias_quad(ep, n);
+    } else if constexpr (MODE == EPI_SWIGLU) {
+      a = bias_quad(ep, n);
+      b = bias_quad(ep, n + 64);
+    } else if constexpr (MODE == EPI_QKV_ROPE) {
+      rr = rope_row_ctx(ep, m);
+      float2 c0, c1;
+      qkv_cs(ep, rr, n, c0, c1);
+      a = make_float4(c0.x, c0.y, c1.x, c1.y);
+    }
+  }
+};
+
+// Quad q of a CTA's 16 columns of a fused mixer projection (ProjArgs), row m (-1: none).  A head's 64 or 128 columns lie
+// in 4 or 8 CTAs of one cluster, which exchange their rows' sums of squares through shared memory.
+template <int ROWS>
+__device__ __forceinline__ void heads_quad(const GemmEpilogue& ep, int m, int row, int n0, int q, float4 v) {
+  const ProjArgs& p = ep.pj;
+  __shared__ float part[ROWS];
+  const int n = n0 + q * 4;
+  const bool gates = p.off_gate >= 0 && n0 >= p.off_gate;
+  const bool is_q = !gates && n0 < p.H * p.dimp;
+  const bool is_g = !gates && p.off_g >= 0 && n0 >= p.off_g;
+  const bool is_v = !gates && !is_g && p.off_v >= 0 && n0 >= p.off_v;
+  const bool is_k = !gates && !is_q && !is_g && !is_v && p.off_k >= 0;
+  const int sec0 = is_q ? p.off_q : is_k ? p.off_k : is_v ? p.off_v : p.off_g;
+  const int width = (is_q || is_k) ? p.dimp : p.vdimp;
+  const float* gain = is_q ? p.q_norm : is_k ? p.k_norm : nullptr;
+  // biases of whole heads exist in attention layers; the recurrence's bias vector only serves its gates
+  const float* bias = p.recurrent && !gates ? nullptr : p.bias;
+  if (bias) {
+    const float4 b = __ldg(reinterpret_cast<const float4*>(bias + n));
+    v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+  }
+  float post = 1.f;
+  if (p.q_norm || p.k_norm) {                    // the same for the whole cluster
+    float ss = (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+    if (q == 0 && row < ROWS) part[row] = ss;
+    sm100::cluster_sync_all();
+    if (gain && m >= 0) {
+      const uint32_t first = sm100::cluster_ctarank() - (((n0 - sec0) & (width - 1)) >> 4);
+      float sum = 0.f;
+      for (int c = 0; c < width >> 4; ++c) sum += sm100::ld_shared_cluster_f32(sm100::smem_u32(part + row), first + c);
+      post = 1.f / sqrtf(sum / (float)p.dim + p.eps);
+    }
+    sm100::cluster_sync_all();                   // nobody leaves while its sums are read
+  }
+  if (m < 0) return;
+  if (gates) {
+    const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n + i - p.off_gate < 2 * p.H) p.gates[(size_t)m * 2 * p.H + n + i - p.off_gate] = x[i];
+    return;
+  }
+  if (!is_q && !is_g && !is_v && !is_k) return;  // padding columns behind the last section
+  if (is_g && n0 >= p.off_g + p.H * p.vdimp) return;
+  if (is_v && p.off_g < 0 && n0 >= p.off_v + p.G * p.vdimp) return;
+  const int in_head = (n - sec0) & (width - 1);
+  if (is_g) {
+    v = make_float4(sigmoid_f(v.x), sigmoid_f(v.y), sigmoid_f(v.z), sigmoid_f(v.w));
+  } else {
+    if (is_q) post *= query_gain(p, p.pos ? max(p.pos[m], 0) : 0);
+    v.x *= post; v.y *= post; v.z *= post; v.w *= post;
+    if (gain) {
+      const float4 g = __ldg(reinterpret_cast<const float4*>(gain + in_head));
+      v.x *= g.x; v.y *= g.y; v.z *= g.z; v.w *= g.w;
+    }
+  }
+  uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + (size_t)m * p.N + n;
+  if (!p.recurrent && (is_k || is_v)) {
+    const long long cr = proj_cache_row(p, m);
+    if (cr < 0) return;
+    dst = reinterpret_cast<uint16_t*>(is_k ? p.kcache : p.vcache) + (size_t)(cr + (long long)((n - sec0) / width) * p.t_max) * width + in_head;
+  }
+  *reinterpret_cast<uint2*>(dst) = make_uint2(pack2_act_chk(v.x, v.y, ep.act_f16, ep.err), pack2_act_chk(v.z, v.w, ep.act_f16, ep.err));
+}
+
 template <int NT, int MT, int MODE, bool F16>
-__global__ void __launch_bounds__(GR_THREADS)
-gemm_rows_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
+__device__ __forceinline__ void rows_product(const uint16_t* A, const uint16_t* W, const GemmEpilogue& ep, int K, float* red) {
   using Cfg = GrCfg<NT, MT>;
   constexpr int WD = Cfg::WD, XD = Cfg::XD, PITCH = Cfg::PITCH;
   pdl_launch_dependents();
-  extern __shared__ float red[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = gr_col<NT, MODE>(blockIdx.x, 0), m0 = blockIdx.y * Cfg::ROWS;
   const int blocks = (K / 32 - warp + GR_WARPS - 1) / GR_WARPS;      // this warp's blocks of K
@@ -85,16 +182,31 @@ gemm_rows_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
 
   const size_t lda = ep.grp.lda ? ep.grp.lda : K;
   const uint16_t* xp = A + (size_t)(m0 + g) * lda + (ep.grp.n_group ? n0 / ep.grp.n_group * ep.grp.a_group : 0) + warp * 32 + t * 8;
-  uint4 x[XD][MT];
+  uint4 x[Cfg::RING ? 1 : XD][Cfg::RING ? 1 : MT];
+  const uint32_t ring = sm100::smem_u32(red) + warp * XD * MT * 512 + lane * 16;
   auto load_x = [&](int slot, int i) {
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-      x[slot][mt] = m0 + mt * 8 + g < ep.M ? __ldcg(reinterpret_cast<const uint4*>(xp + (size_t)mt * 8 * lda + (size_t)i * step))
-                                           : make_uint4(0u, 0u, 0u, 0u);
+    for (int mt = 0; mt < MT; ++mt) {
+      const bool in = m0 + mt * 8 + g < ep.M;
+      const uint16_t* src = xp + (size_t)(in ? mt * 8 : 0) * lda + (size_t)i * step;
+      if constexpr (Cfg::RING)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + (slot * MT + mt) * 512), "l"(in ? src : A), "r"(in ? 16 : 0)
+                     : "memory");
+      else
+        x[Cfg::RING ? 0 : slot][Cfg::RING ? 0 : mt] = in ? __ldcg(reinterpret_cast<const uint4*>(src)) : make_uint4(0u, 0u, 0u, 0u);
+    }
   };
 #pragma unroll
-  for (int p = 0; p < XD; ++p)
+  for (int p = 0; p < XD; ++p) {
     if (p < blocks) load_x(p, p);
+    if constexpr (Cfg::RING) asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  constexpr int QUADS = gr_paired<MODE>() ? 2 * NT : 4 * NT;         // output quads of a row
+  GrAhead ahead;
+  if constexpr (MODE != EPI_HEADS && MT <= 4) {
+    const int row = threadIdx.x / QUADS;
+    if (row < Cfg::ROWS && m0 + row < ep.M) ahead.load<MODE>(ep, m0 + row, n0 + (threadIdx.x - row * QUADS) * 4);
+  }
 
   float acc[NT][MT][4];
 #pragma unroll
@@ -104,23 +216,46 @@ gemm_rows_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[nt][mt][j] = 0.f;
 
+  int slot = 0;
   for (int i = 0; i < blocks; i += WD) {
 #pragma unroll
     for (int p = 0; p < WD; ++p) {
       if (i + p >= blocks) break;
-      const int s = p % XD;
+      if constexpr (Cfg::RING) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(XD - 1) : "memory");
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const uint4 lo = w[p][nt][0], hi = w[p][nt][1];
+        for (int mt = 0; mt < MT; ++mt) {        // one fragment at a time: registers are for sums and weights
+          uint4 v;
+          asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                       : "r"(ring + (slot * MT + mt) * 512)
+                       : "memory");
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) mma16816<F16>(acc[nt][mt], lo.x, hi.x, lo.y, hi.y, x[s][mt].x, x[s][mt].y);
+          for (int nt = 0; nt < NT; ++nt) {
+            const uint4 lo = w[p][nt][0], hi = w[p][nt][1];
+            mma16816<F16>(acc[nt][mt], lo.x, hi.x, lo.y, hi.y, v.x, v.y);
+            mma16816<F16>(acc[nt][mt], lo.z, hi.z, lo.w, hi.w, v.z, v.w);
+          }
+        }
+      } else {
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) mma16816<F16>(acc[nt][mt], lo.z, hi.z, lo.w, hi.w, x[s][mt].z, x[s][mt].w);
+        for (int nt = 0; nt < NT; ++nt) {
+          const uint4 lo = w[p][nt][0], hi = w[p][nt][1];
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) mma16816<F16>(acc[nt][mt], lo.x, hi.x, lo.y, hi.y, x[p][mt].x, x[p][mt].y);
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) mma16816<F16>(acc[nt][mt], lo.z, hi.z, lo.w, hi.w, x[p][mt].z, x[p][mt].w);
+        }
       }
       if (i + p + WD < blocks) load_w(p, i + p + WD);
-      if (i + p + XD < blocks) load_x(s, i + p + XD);
+      if (i + p + XD < blocks) load_x(Cfg::RING ? slot : p, i + p + XD);
+      if constexpr (Cfg::RING) {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        slot = slot + 1 == XD ? 0 : slot + 1;
+      }
     }
   }
+  if constexpr (Cfg::RING) __syncthreads();      // every warp is done with its part of the ring
 
   float* mine = red + warp * Cfg::ROWS * PITCH;
 #pragma unroll
@@ -143,26 +278,47 @@ gemm_rows_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
     }
     return v;
   };
-  constexpr int QUADS = gr_paired<MODE>() ? 2 * NT : 4 * NT;         // output quads of a row
+  if constexpr (MODE == EPI_HEADS) {
+    static_assert(NT == 1 && Cfg::ROWS * 4 <= GR_THREADS, "one quad a thread");
+    const int row = threadIdx.x >> 2, q = threadIdx.x & 3;
+    const bool in = row < Cfg::ROWS && m0 + row < ep.M;
+    heads_quad<Cfg::ROWS>(ep, in ? m0 + row : -1, row, n0, q, in ? total(row, q * 4) : make_float4(0.f, 0.f, 0.f, 0.f));
+    return;
+  }
   for (int u = threadIdx.x; u < Cfg::ROWS * QUADS; u += GR_THREADS) {
-    const int row = u / QUADS, q = u - row * QUADS, m = m0 + row;
+    const int row = u / QUADS, q = u - row * QUADS, m = m0 + row, n = n0 + q * 4;
     if (m >= ep.M) break;
+    if (MT > 4 || u != threadIdx.x) ahead.load<MODE>(ep, m, n);
     if constexpr (gr_paired<MODE>()) {
       const int c = (q >> 2) * 32 + (q & 3) * 4;                     // gate tile 2 (q / 4), its up tile 16 columns on
       const float4 gate = total(row, c), up = total(row, c + 16);
-      const int n = n0 + q * 4;
-      if constexpr (MODE == EPI_SWIGLU) epi_swiglu_quad(ep, m, n, gate, up);
+      if constexpr (MODE == EPI_SWIGLU) epi_swiglu_quad(ep, m, n, gate, up, ahead.a, ahead.b);
       else epi_glu_quad(ep, m, n, gate, up);
     } else {
       const float4 v = total(row, q * 4);
-      const int n = n0 + q * 4;
-      if constexpr (MODE == EPI_QKV_ROPE) epi_qkv_quad(ep, rope_row_ctx(ep, m), m, n, v);
-      else if constexpr (MODE == EPI_RESID) epi_resid_quad(ep, m, n, v);
+      if constexpr (MODE == EPI_QKV_ROPE)
+        epi_qkv_quad(ep, ahead.rr, m, n, v, make_float2(ahead.a.x, ahead.a.y), make_float2(ahead.a.z, ahead.a.w));
+      else if constexpr (MODE == EPI_RESID) epi_resid_quad(ep, m, n, v, ahead.a, ahead.b);
       else if constexpr (MODE == EPI_RELU2) epi_relu2_quad(ep, m, n, v);
       else if constexpr (MODE == EPI_ACT) epi_act_quad(ep, m, n, v);
       else epi_store_quad(ep, m, n, v);
     }
   }
+}
+
+template <int NT, int MT, int MODE, bool F16>
+__global__ void __launch_bounds__(GR_THREADS, 2)
+gemm_rows_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
+  extern __shared__ float red[];
+  rows_product<NT, MT, MODE, F16>(A, W, ep, K, red);
+}
+
+// clusters of the CTAs that share 128 columns
+template <int MT, bool F16>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(GR_THREADS, 2)
+gemm_rows_heads_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
+  extern __shared__ float red[];
+  rows_product<1, MT, EPI_HEADS, F16>(A, W, ep, K, red);
 }
 
 template <int NT, int MT, int MODE>
@@ -174,6 +330,14 @@ cudaError_t launch(const void* a, const void* w, const GemmEpilogue& ep, int K, 
                      reinterpret_cast<const uint16_t*>(w), ep, K);
 }
 
+template <int MT>
+cudaError_t launch_heads(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {
+  using Cfg = GrCfg<1, MT>;
+  return arcb_launch(act_f16 ? gemm_rows_heads_kernel<MT, true> : gemm_rows_heads_kernel<MT, false>,
+                     dim3(ep.N / 16, (ep.M + Cfg::ROWS - 1) / Cfg::ROWS), dim3(GR_THREADS), Cfg::SMEM, stream,
+                     reinterpret_cast<const uint16_t*>(a), reinterpret_cast<const uint16_t*>(w), ep, K);
+}
+
 template <int MODE>
 cudaError_t launch_mode(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {
   constexpr int N1 = gr_paired<MODE>() ? 2 : 1;
@@ -183,13 +347,25 @@ cudaError_t launch_mode(const void* a, const void* w, const GemmEpilogue& ep, in
   return launch<2, 8, MODE>(a, w, ep, K, act_f16, stream);
 }
 
-// the widest form's partial sums need more than the default 48 KB of shared memory
+// forms that need more than the default 48 KB of shared memory
+template <typename K>
+cudaError_t opt_in(K kernel, int bytes) {
+  return bytes > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
+}
 template <int MODE>
 cudaError_t init_mode() {
-  const int bytes = GrCfg<2, 8>::SMEM;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<2, 8, MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(gemm_rows_kernel<2, 8, MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaError_t e = opt_in(gemm_rows_kernel<2, 8, MODE, true>, GrCfg<2, 8>::SMEM);
+  if (e == cudaSuccess) e = opt_in(gemm_rows_kernel<2, 8, MODE, false>, GrCfg<2, 8>::SMEM);
+  if (e == cudaSuccess) e = opt_in(gemm_rows_kernel<2, 4, MODE, true>, GrCfg<2, 4>::SMEM);
+  if (e == cudaSuccess) e = opt_in(gemm_rows_kernel<2, 4, MODE, false>, GrCfg<2, 4>::SMEM);
+  return e;
+}
+cudaError_t init_heads() {
+  cudaError_t e = opt_in(gemm_rows_heads_kernel<8, true>, GrCfg<1, 8>::SMEM);
+  if (e == cudaSuccess) e = opt_in(gemm_rows_heads_kernel<8, false>, GrCfg<1, 8>::SMEM);
+  if (e == cudaSuccess) e = opt_in(gemm_rows_heads_kernel<4, true>, GrCfg<1, 4>::SMEM);
+  if (e == cudaSuccess) e = opt_in(gemm_rows_heads_kernel<4, false>, GrCfg<1, 4>::SMEM);
+  return e;
 }
 
 }  // namespace
@@ -202,17 +378,22 @@ int arcb_gemm_rows_init() {
   if ((e = init_mode<EPI_SWIGLU>()) != cudaSuccess) return (int)e;
   if ((e = init_mode<EPI_RELU2>()) != cudaSuccess) return (int)e;
   if ((e = init_mode<EPI_ACT>()) != cudaSuccess) return (int)e;
-  return (int)init_mode<EPI_GLU>();
+  if ((e = init_mode<EPI_GLU>()) != cudaSuccess) return (int)e;
+  return (int)init_heads();
 }
 
 // Up to 64 rows: the weights' 16-row fragments meet eight 8-row activation fragments, and the activations of a CTA
 // (64 rows x K) are re-read from L2 by every CTA; the step of the latent-attention model with 48 rows takes 3 % less
 // with it.  One row tile more would read the weights twice.
-bool arcb_gemm_rows_applies(const GemmEpilogue& ep, int K, int act_f16) {
+bool arcb_gemm_rows_applies(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16) {
   if (ep.M > 64 || act_f16 == 2 || K % 32 || ep.N % 128) return false;
   const GroupArgs& g = ep.grp;
-  if (g.tile_src || g.tile_group || g.n_tiles || g.panels || (g.n_group && g.n_group % 32)) return false;
-  return ep.mode != EPI_HEADS;
+  if (g.tile_src || g.tile_group || g.n_tiles || g.panels || (g.n_group && g.n_group % 32) || g.lda % 8 || g.a_group % 8) return false;
+  // 16-byte accesses; what is not aligned meets the tensor maps' refusal
+  const uintptr_t all = (uintptr_t)a | (uintptr_t)w | (uintptr_t)ep.x | (uintptr_t)ep.y | (uintptr_t)ep.out16 | (uintptr_t)ep.bias | (uintptr_t)ep.pj.out;
+  if (all & 15) return false;
+  // normed heads span CTAs of one cluster of 128 columns
+  return ep.mode != EPI_HEADS || !(ep.pj.q_norm || ep.pj.k_norm) || ep.pj.dimp <= 128;
 }
 
 int arcb_launch_gemm_rows(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {
@@ -225,6 +406,12 @@ int arcb_launch_gemm_rows(const void* a, const void* w, const GemmEpilogue& ep, 
     case EPI_RELU2: e = launch_mode<EPI_RELU2>(a, w, ep, K, act_f16, stream); break;
     case EPI_ACT: e = launch_mode<EPI_ACT>(a, w, ep, K, act_f16, stream); break;
     case EPI_GLU: e = launch_mode<EPI_GLU>(a, w, ep, K, act_f16, stream); break;
+    case EPI_HEADS:
+      e = ep.M <= 8    ? launch_heads<1>(a, w, ep, K, act_f16, stream)
+          : ep.M <= 16 ? launch_heads<2>(a, w, ep, K, act_f16, stream)
+          : ep.M <= 32 ? launch_heads<4>(a, w, ep, K, act_f16, stream)
+                       : launch_heads<8>(a, w, ep, K, act_f16, stream);
+      break;
   }
   arcb_count_launch(1);
   return (int)e;
