@@ -5,8 +5,8 @@
 //                      accumulators in TMEM (the epilogue drains one while the next tile fills the
 //                      other), operands staged by TMA (128-byte swizzle) through an mbarrier ring;
 //                      warp 0 = TMA producer, warp 1 = MMA issuer, warps 2-9 = epilogue.
-//   gemm_simt_kernel : CUDA-core tile kernel for skinny M (weight streaming) and as
-//                      the cross-check of the tensor-core path.
+//   gemm_simt_kernel, gemm_simt_wide_kernel : CUDA-core tile kernels, for 32-bit operands, for K the tensor-core kernels do
+//                      not take and as their cross-check.
 #include <cstdlib>
 
 #include "gemm.cuh"
@@ -1171,6 +1171,32 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 // ---------------------------------------------------------------------------
 constexpr int SM_BM = 32, SM_BN = 128, SM_BK = 32;
 
+// columns n .. n + 3 and n + 64 .. n + 67 of row m through the epilogue
+template <int MODE>
+__device__ __forceinline__ void simt_store(const GemmEpilogue& ep, int m, int n, float4 lo, float4 hi) {
+  if constexpr (MODE == EPI_SWIGLU) {
+    epi_swiglu_quad(ep, m, n, lo, hi);
+  } else if constexpr (MODE == EPI_GLU) {
+    epi_glu_quad(ep, m, n, lo, hi);
+  } else if constexpr (MODE == EPI_ACT) {
+    epi_act_quad(ep, m, n, lo);
+    epi_act_quad(ep, m, n + 64, hi);
+  } else if constexpr (MODE == EPI_QKV_ROPE) {
+    const RopeRow rr = rope_row_ctx(ep, m);
+    epi_qkv_quad(ep, rr, m, n, lo);
+    epi_qkv_quad(ep, rr, m, n + 64, hi);
+  } else if constexpr (MODE == EPI_RESID) {
+    epi_resid_quad(ep, m, n, lo);
+    epi_resid_quad(ep, m, n + 64, hi);
+  } else if constexpr (MODE == EPI_RELU2) {
+    epi_relu2_quad(ep, m, n, lo);
+    epi_relu2_quad(ep, m, n + 64, hi);
+  } else {
+    epi_store_quad(ep, m, n, lo);
+    epi_store_quad(ep, m, n + 64, hi);
+  }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(256)
 gemm_simt_kernel(const void* __restrict__ Av, const void* __restrict__ Wv, GemmEpilogue ep,
@@ -1244,30 +1270,95 @@ gemm_simt_kernel(const void* __restrict__ Av, const void* __restrict__ Wv, GemmE
   for (int i = 0; i < 2; ++i) {
     const int m = m0 + 2 * ty + i;
     if (m >= ep.M) continue;
-    const float4 lo = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    const float4 hi = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
-    const int n = n0 + 4 * tx;
-    if constexpr (MODE == EPI_SWIGLU) {
-      epi_swiglu_quad(ep, m, n, lo, hi);
-    } else if constexpr (MODE == EPI_GLU) {
-      epi_glu_quad(ep, m, n, lo, hi);
-    } else if constexpr (MODE == EPI_ACT) {
-      epi_act_quad(ep, m, n, lo);
-      epi_act_quad(ep, m, n + 64, hi);
-    } else if constexpr (MODE == EPI_QKV_ROPE) {
-      const RopeRow rr = rope_row_ctx(ep, m);
-      epi_qkv_quad(ep, rr, m, n, lo);
-      epi_qkv_quad(ep, rr, m, n + 64, hi);
-    } else if constexpr (MODE == EPI_RESID) {
-      epi_resid_quad(ep, m, n, lo);
-      epi_resid_quad(ep, m, n + 64, hi);
-    } else if constexpr (MODE == EPI_RELU2) {
-      epi_relu2_quad(ep, m, n, lo);
-      epi_relu2_quad(ep, m, n + 64, hi);
-    } else {
-      epi_store_quad(ep, m, n, lo);
-      epi_store_quad(ep, m, n + 64, hi);
+    simt_store<MODE>(ep, m, n0 + 4 * tx, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]),
+                     make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]));
+  }
+}
+
+// CUDA-core kernel for more rows: BM x 128 x 16 tiles, 256 threads, each thread BM / 16 rows x (4 + 4) columns, two-wide
+// multiply-adds, the next tile's global loads in flight while one is multiplied.  Bound by the multiply-add pipes (148 SMs
+// x 128 lanes); a thread of the 32-row kernel reads two shared-memory words per 16 multiply-adds, here 16 (12) per 64 (32).
+// Every sum runs over K in ascending order in one accumulator, as in the 32-row kernel: same bits.
+// B200, fp32, TFLOP/s, 32-row kernel / here: 1.6 k rows, N 1280, K 1280 and 5120 9 / 35 (64-row tiles, 260 CTAs), N 3200 and
+// 5248, K 1280 9 / 43 (128-row tiles).
+template <int BM, int MODE>
+__global__ void __launch_bounds__(256, 2)
+gemm_simt_wide_kernel(const void* Av, const void* Wv, GemmEpilogue ep, int K, int a_fmt) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int BK = 16, TM = BM / 16, LA = BM / 64, LB = 2, PA = BM + 4, PB = 128 + 4;
+  __shared__ __align__(16) float As[2][BK][PA];
+  __shared__ __align__(16) float Bs[2][BK][PB];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * 128;
+  const GroupArgs& g = ep.grp;
+  if (g.n_tiles && (m0 >> 7) >= *g.n_tiles) return;
+  const int a_row0 = g.tile_src ? g.tile_src[m0 >> 7] + (m0 & 127) : m0;
+  const long long a_rows = g.a_rows ? g.a_rows : ep.M;
+  const size_t lda = g.lda ? g.lda : K;
+  const size_t w_row0 = (size_t)n0 + (g.tile_group ? (size_t)g.tile_group[m0 >> 7] * g.group_rows : 0);
+  float4 ra[LA], rb[LB];
+  const int lr = tid >> 2, lk = (tid & 3) * 4;
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < LA; ++i)
+      ra[i] = a_row0 + lr + 64 * i < a_rows ? ld_act4(Av, (size_t)(a_row0 + lr + 64 * i) * lda + k0 + lk, a_fmt) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < LB; ++i) rb[i] = ld_act4(Wv, (w_row0 + lr + 64 * i) * K + k0 + lk, a_fmt);
+  };
+  auto stage = [&](int s) {
+#pragma unroll
+    for (int i = 0; i < LA; ++i) {
+      As[s][lk][lr + 64 * i] = ra[i].x; As[s][lk + 1][lr + 64 * i] = ra[i].y;
+      As[s][lk + 2][lr + 64 * i] = ra[i].z; As[s][lk + 3][lr + 64 * i] = ra[i].w;
     }
+#pragma unroll
+    for (int i = 0; i < LB; ++i) {
+      Bs[s][lk][lr + 64 * i] = rb[i].x; Bs[s][lk + 1][lr + 64 * i] = rb[i].y;
+      Bs[s][lk + 2][lr + 64 * i] = rb[i].z; Bs[s][lk + 3][lr + 64 * i] = rb[i].w;
+    }
+  };
+  uint64_t acc[TM][4];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+  fetch(0);
+  stage(0);
+  __syncthreads();
+  for (int k0 = 0, s = 0; k0 < K; k0 += BK, s ^= 1) {
+    const bool more = k0 + BK < K;
+    if (more) fetch(k0 + BK);
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      float a[TM];
+#pragma unroll
+      for (int h = 0; h < TM / 4; ++h) *reinterpret_cast<float4*>(a + 4 * h) = *reinterpret_cast<const float4*>(&As[s][k][64 * h + 4 * ty]);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&Bs[s][k][4 * tx]);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&Bs[s][k][64 + 4 * tx]);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        uint64_t aa;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a[i]));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][0]) : "l"(aa), "l"(b0.x));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][1]) : "l"(aa), "l"(b0.y));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][2]) : "l"(aa), "l"(b1.x));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][3]) : "l"(aa), "l"(b1.y));
+      }
+    }
+    if (more) stage(s ^ 1);
+    __syncthreads();
+  }
+  auto quad = [&](uint64_t lo, uint64_t hi) {
+    float4 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(lo));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.z), "=f"(v.w) : "l"(hi));
+    return v;
+  };
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + (i >> 2) * 64 + 4 * ty + (i & 3);
+    if (m < ep.M) simt_store<MODE>(ep, m, n0 + 4 * tx, quad(acc[i][0], acc[i][1]), quad(acc[i][2], acc[i][3]));
   }
 }
 
@@ -1617,9 +1708,11 @@ static int launch_gemm_mode(const void* a16, const void* w16, const GemmEpilogue
     arcb_count_launch(1);
     return (int)le;
   }
-  dim3 grid(N / SM_BN, (M + SM_BM - 1) / SM_BM);
-  const cudaError_t le = arcb_launch(gemm_simt_kernel<MODE>, grid, dim3(256), 0, stream,
-                                     a16, w16, ep, K, act_f16);
+  // 32-row tiles for few rows only; 128-row tiles once they are two waves (two CTAs fit an SM), 64-row tiles below
+  auto simt = [&](auto kernel, int bm) { return arcb_launch(kernel, dim3(N / SM_BN, (M + bm - 1) / bm), dim3(256), 0, stream, a16, w16, ep, K, act_f16); };
+  const cudaError_t le = M <= SM_BM ? simt(gemm_simt_kernel<MODE>, SM_BM)
+                         : (long long)(N / SM_BN) * ((M + 127) / 128) >= 2 * num_sms() ? simt(gemm_simt_wide_kernel<128, MODE>, 128)
+                                                                                         : simt(gemm_simt_wide_kernel<64, MODE>, 64);
   arcb_count_launch(1);
   return (int)le;
 }

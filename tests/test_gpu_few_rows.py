@@ -116,6 +116,23 @@ def test_few_row_products(lib, M, N, K, fmt):
     assert ((got[0][:M].double() - ref).abs() <= bound + (ref.abs() + x0[:M].double().abs() + bias.double().abs()) * 2 ** -22).all()
 
 
+@pytest.mark.parametrize("M,N,K", [(32, 128, 32), (33, 128, 32), (64, 384, 96), (65, 256, 64), (700, 1280, 320), (2500, 2048, 96)])
+def test_cuda_core_products(lib, M, N, K):
+    """32-row tiles, 64-row tiles from 33 rows on and 128-row tiles from two waves on: every sum runs over K in order, so the
+    same rows give the same bits through any of them."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = to_act(torch.randn(M, K, device="cuda", generator=g), _lib.ACT_F16)
+    w = to_act((torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).to(torch.bfloat16).float(), _lib.ACT_F16)
+    y, few = (torch.full((M + 1, N), 7.0, device="cuda") for _ in range(2))
+    _lib.check(lib.arcb_op_gemm(a.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, K, _lib.ACT_F16, _lib.GEMM_SIMT, stream()))
+    for m in range(0, M, 32):
+        rows = min(32, M - m)
+        _lib.check(lib.arcb_op_gemm(a[m:].data_ptr(), w.data_ptr(), few[m:].data_ptr(), rows, N, K, _lib.ACT_F16, _lib.GEMM_SIMT, stream()))
+    assert torch.equal(y, few) and (y[M] == 7).all()
+    ref = a.double() @ w.double().T
+    assert ((y[:M].double() - ref).abs() <= (a.double().abs() @ w.double().abs().T) * 2 ** -24 * K).all()
+
+
 # widths whose norms hold a row in one to eight registers a thread, and one beyond; a vocabulary off and on quads of columns
 @pytest.mark.parametrize("width,vocab", [(500, 333), (1000, 332), (2050, 96), (4100, 64)])
 def test_layered_steps_of_few_rows(width, vocab):
