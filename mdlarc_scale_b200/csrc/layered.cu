@@ -322,6 +322,7 @@ extern "C" int arcb_engine_create_layered(const arcb_model_desc* md, const arcb_
   if (!arcb_device_ok()) return arcb_fail(ARCB_E_UNSUPPORTED, "current device is not compute capability 10.x");
   CKL(arcb_gemm_init(), "gemm init (shared-memory opt-in / cuTensorMapEncodeTiled lookup)");
   CKL(arcb_mlstm_chunk_init(), "chunkwise recurrence init (shared-memory opt-in)");
+  CKL(arcb_mlstm_walk_init(), "recurrence init (shared-memory opt-in)");
   CKL(arcb_attn_prefill_gqa_init(), "prefill attention init (shared-memory opt-in)");
   CKL(arcb_attn_latent_init(), "latent attention init (shared-memory opt-in)");
   arcb_engine* e = new arcb_engine();

@@ -42,3 +42,4 @@ int arcb_mlstm_chunk_init();
 int arcb_launch_mlstm_chunk(const MlstmArgs& a, cudaStream_t stream);
 int arcb_launch_mlstm_step(const MlstmArgs& a, cudaStream_t stream);
 void arcb_count_launch(long long n);
+int arcb_mlstm_walk_init();
