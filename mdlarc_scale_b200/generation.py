@@ -31,6 +31,17 @@ class Request:
     slot: int = -1
     produced: int = 0            # tokens picked so far (host count; an upper bound once the end token is out)
     output: list[int] = field(default_factory=list)
+    tokens: np.ndarray | None = field(default=None, compare=False)     # the prompt as one array, from submit()
+
+
+def _token_array(prompt) -> np.ndarray:
+    try:
+        tokens = np.array(prompt, np.int64)
+        if tokens.ndim == 1:
+            return tokens
+    except (TypeError, ValueError, OverflowError, RuntimeError):
+        pass
+    return np.array([int(t) for t in prompt], object)     # elements that only int() understands, or refuses
 
 
 class Scheduler:
@@ -57,26 +68,35 @@ class Scheduler:
             raise ValueError("a prompt needs at least one token")
         if n + self.max_new - 1 > self.session.t_max:
             raise ValueError(f"prompt of {n} tokens plus {self.max_new} new ones exceeds the session's {self.session.t_max} positions")
-        if min(request.prompt) < 0 or max(request.prompt) >= self.engine.vocab_size:
+        tokens = _token_array(request.prompt)
+        if tokens.min() < 0 or tokens.max() >= self.engine.vocab_size:
             raise ValueError("a prompt token lies outside the vocabulary")
+        request.tokens = tokens.astype(np.int64)
         self.waiting.append(request)
 
+    # The device state of all admitted requests is set, and the results of all ended ones are read, together: with a few
+    # launches and copies for each (35 to 90 us) the GPU waited 10 of 68 ms for the host at 150 requests.
     def _admit(self) -> None:
+        admitted = []
         while self.waiting and self.session.free_slots:
             r = self.waiting.popleft()
             r.slot = self.session.acquire()
-            self.session.out_tokens[r.slot].fill_(-1)
-            self.session.sample_stream[r.slot] = r.rid & 0x7FFFFFFF
-            self.filling.append(r)
+            admitted.append(r)
+        if not admitted:
+            return
+        self.filling += admitted
+        at = torch.tensor([[r.slot for r in admitted], [r.rid & 0x7FFFFFFF for r in admitted]]).to(self.engine.device, non_blocking=True)
+        self.session.out_tokens.index_fill_(0, at[0], -1)
+        self.session.sample_stream.index_copy_(0, at[0], at[1].to(torch.int32))
 
     def _prefill(self) -> None:
         room, call, armed = self.session.max_prefill_tokens, [], []
         for r in self.filling:
-            n = min(room, len(r.prompt) - r.fed)
+            n = min(room, len(r.tokens) - r.fed)
             if n <= 0:
                 break
-            last = r.fed + n == len(r.prompt)
-            call.append(Segment(r.slot, r.prompt[r.fed:r.fed + n], arm=last))
+            last = r.fed + n == len(r.tokens)
+            call.append(Segment(r.slot, r.tokens[r.fed:r.fed + n], arm=last))
             r.fed += n
             room -= n
             if last:
@@ -97,17 +117,26 @@ class Scheduler:
                 self.session.lens[r.slot] += n
 
     def _retire(self) -> None:
-        ended = self.session.finished() if self.end_token >= 0 else None
-        for r in list(self.decoding):
-            if r.produced < self.max_new and (ended is None or not ended[r.slot]):
-                continue
-            row = self.session.out_tokens[r.slot].cpu().tolist()
+        flags = self.session.finished() if self.end_token >= 0 else None
+        ended = [r for r in self.decoding if r.produced >= self.max_new or (flags is not None and flags[r.slot])]
+        if not ended:
+            return
+        rows = self.session.out_tokens.cpu()
+        for r in ended:
+            row = rows[r.slot].tolist()
             if self.end_token in row:
                 row = row[:row.index(self.end_token) + 1]
             r.output = row
-            if self.session.step_logits is not None:
-                self.step_logits[r.rid] = self.session.step_logits[r.slot, :len(row)].clone()
-            self.decoding.remove(r)
+        if self.session.step_logits is not None:
+            # one copy for them all, as long as the longest; each request's logits are a view of it
+            longest = max(len(r.output) for r in ended)
+            at = torch.tensor([r.slot for r in ended]).to(self.engine.device, non_blocking=True)
+            logits = self.session.step_logits[:, :longest].index_select(0, at)
+            for i, r in enumerate(ended):
+                self.step_logits[r.rid] = logits[i, :len(r.output)]
+        gone = {id(r) for r in ended}
+        self.decoding = [r for r in self.decoding if id(r) not in gone]
+        for r in ended:
             self.session.release(r.slot)
             self.done.append(r)
 
@@ -139,7 +168,7 @@ def generate(engine: EngineBase, prompts, max_new: int, end_token: int | None = 
                       top_k, seed, return_logits)
     try:
         for i, p in enumerate(prompts):
-            sched.submit(Request(i, [int(t) for t in p]))
+            sched.submit(Request(i, p if isinstance(p, list) else [int(t) for t in p]))
         out = [r.output for r in sched.run()]
         return (out, sched.step_logits) if return_logits else out
     finally:

@@ -105,3 +105,106 @@ def test_pack_segments():
     assert last == sorted(last, reverse=True)
     with pytest.raises(ValueError):
         pack_segments([Segment(0, [1], [1])], [0])
+
+
+class _CpuSession:
+    """What the scheduler uses of a session; slot s of a request with prompt p generates p[-1], p[-1] + 1, ..."""
+
+    def __init__(self, n_slots, t_max, max_new, max_prefill_tokens, **kw):
+        self.t_max, self.max_prefill_tokens, self.n, self.end = t_max, max_prefill_tokens, n_slots, kw["end_token"]
+        self.out_tokens = torch.full((n_slots, max_new), 99, dtype=torch.int32)
+        self.sample_stream = torch.from_numpy(kw["sample_stream"]).to(torch.int32)
+        self.step_logits = torch.zeros(n_slots, max_new, 3) if kw["want_step_logits"] else None
+        self.lens, self.free, self.made, self.fed, self.streams = [0] * n_slots, list(range(n_slots)), [0] * n_slots, {}, []
+
+    free_slots = property(lambda self: len(self.free))
+
+    def acquire(self):
+        return self.free.pop()
+
+    def release(self, slot):
+        self.free.append(slot)
+
+    def _put(self, slot):
+        t = self.fed[slot][-1] + self.made[slot]
+        self.out_tokens[slot, self.made[slot]] = t
+        if self.step_logits is not None:
+            self.step_logits[slot, self.made[slot]] = float(t)
+        self.made[slot] += 1
+
+    def prefill_segments(self, segments):
+        for s in segments:
+            self.fed[s.slot] = (self.fed[s.slot] if self.lens[s.slot] else []) + [int(t) for t in s.tokens]
+            self.lens[s.slot] += len(s.tokens)
+            if s.arm:
+                assert (self.out_tokens[s.slot] == -1).all()
+                self.streams.append((self.fed[s.slot], int(self.sample_stream[s.slot])))
+                self.made[s.slot] = 0
+                self._put(s.slot)
+
+    def decode(self, n):
+        for slot in set(range(self.n)) - set(self.free):
+            for _ in range(n):
+                row = self.out_tokens[slot, :self.made[slot]].tolist()
+                if 0 < self.made[slot] < self.out_tokens.shape[1] and self.end not in row:
+                    self._put(slot)
+
+    def finished(self):
+        return np.array([self.end in self.out_tokens[s].tolist() for s in range(self.n)], np.int32)
+
+    def poll(self):
+        return 0
+
+    def close(self):
+        pass
+
+
+class _CpuEngine:
+    device, vocab_size = torch.device("cpu"), 1000
+
+    def new_session(self, n_slots, t_max, max_new, max_prefill_tokens, **kw):
+        self.session = _CpuSession(n_slots, t_max, max_new, max_prefill_tokens, **kw)
+        self.session.lens = _Lens(self.session)
+        return self.session
+
+
+class _Lens(list):
+    """Lengths (and the fake's counts) that start again when a slot is given back, as a session's do."""
+
+    def __init__(self, session):
+        super().__init__([0] * session.n)
+        release = session.release
+
+        def back(slot):
+            self[slot] = session.made[slot] = 0
+            release(slot)
+        session.release = back
+
+
+@pytest.mark.parametrize("max_batch", [2, 8])
+@pytest.mark.parametrize("end", [None, 40])
+def test_scheduler_admits_and_retires_together(max_batch, end):
+    """More requests than slots, prompts in portions, ends at different steps, every kind of sequence a prompt may be."""
+    from mdlarc_scale_b200.generation import generate
+    prompts = [[1, 2, 36], (7, 8), np.array([5] * 30 + [38]), torch.tensor([3, 4]), [torch.tensor(9), np.int32(100)], [True, 39.0], range(5, 8)]
+    engine = _CpuEngine()
+    out, logits = generate(engine, prompts, 20, end_token=end, max_batch=max_batch, prefill_tokens=16, return_logits=True)
+    for i, p in enumerate(prompts):
+        last = int(p[-1])
+        want = list(range(last, last + 20))
+        if end in want:
+            want = want[:want.index(end) + 1]
+        assert out[i] == want and logits[i].shape == (len(want), 3) and logits[i][:, 0].tolist() == want
+    assert sorted(engine.session.streams) == sorted(([int(t) for t in p], i) for i, p in enumerate(prompts))
+
+
+@pytest.mark.parametrize("prompt,error", [([], ValueError), ([1, 1000], ValueError), ([-1], ValueError), ([2 ** 70], ValueError),
+                                          ([[1, 2]], TypeError), ([None], TypeError), ([1] * 400, None)])
+def test_scheduler_refuses_bad_prompts(prompt, error):
+    from mdlarc_scale_b200.generation import Request, Scheduler, generate
+    if error:
+        with pytest.raises(error):
+            generate(_CpuEngine(), [prompt], 3)
+        return
+    with pytest.raises(ValueError):
+        Scheduler(_CpuEngine(), 3, 100, 1).submit(Request(0, prompt))
