@@ -379,7 +379,7 @@ static int run_layer(arcb_session* s, int l, int rows, const int* pos, const int
   __nv_bfloat16* vbase = kbase + (size_t)B * d * T;
 
   GemmEpilogue ep{};
-  ep.M = rows; ep.act_f16 = f16; ep.err = e->d_err;
+  ep.M = rows; ep.act_f16 = f16; ep.err = e->d_err; ep.step = !prefill;
   // QKV projection + 3D RoPE + cache write
   ep.mode = EPI_QKV_ROPE; ep.N = 3 * d; ep.out16 = s->q16;
   ep.pos = pos; ep.slot = slot; ep.seq = seq; ep.kcache = kbase; ep.vcache = vbase;
@@ -426,13 +426,14 @@ static int run_layer(arcb_session* s, int l, int rows, const int* pos, const int
   // out_proj + residual
   GemmEpilogue er{};
   er.mode = EPI_RESID; er.M = rows; er.N = d; er.x = s->x; er.bias = nullptr; er.act_f16 = f16; er.err = e->d_err;
+  er.step = !prefill;
   er.splitk_scratch = prefill ? nullptr : s->gemm_scratch;   // sized for the decode step's rows only
   CKL(arcb_launch_gemm(s->attn16, L.w_out, er, d, f16, use_tc_for(e, rows, d, d), stream), "out_proj gemm");
   plain_edges.off();
   CKL(arcb_launch_rmsnorm(s->x, L.ln2_w, s->xn16, rows, d, c.norm_eps, f16, stream), "ln2");
   // gate | up + SwiGLU
   GemmEpilogue eg{};
-  eg.mode = EPI_SWIGLU; eg.M = rows; eg.N = 2 * dff; eg.bias = L.b_gu; eg.out16 = s->h16; eg.act_f16 = f16; eg.err = e->d_err;
+  eg.mode = EPI_SWIGLU; eg.M = rows; eg.N = 2 * dff; eg.bias = L.b_gu; eg.out16 = s->h16; eg.act_f16 = f16; eg.err = e->d_err; eg.step = !prefill;
   CKL(arcb_launch_gemm(s->xn16, L.w_gu, eg, d, f16, use_tc_for(e, rows, 2 * dff, d), stream), "gate/up gemm");
   // down + bias + residual
   er.bias = L.b_down;
@@ -637,7 +638,7 @@ extern "C" int arcb_op_gemm(const void* a16, const void* w, float* y, int32_t M,
     tc = false;
   }
   GemmEpilogue ep{};
-  ep.mode = EPI_STORE_F32; ep.M = M; ep.N = N; ep.y = y;
+  ep.mode = EPI_STORE_F32; ep.M = M; ep.N = N; ep.y = y; ep.step = 1;
   CKL(arcb_launch_gemm(a16, w, ep, K, act_format == ARCB_ACT_F16, tc, (cudaStream_t)stream, variant), "gemm");
   return ARCB_OK;
 }
@@ -654,7 +655,7 @@ extern "C" int arcb_op_gemm_residual(const void* a16, const void* w, const float
     tc = false;
   }
   GemmEpilogue ep{};
-  ep.mode = EPI_RESID; ep.M = M; ep.N = N; ep.x = x; ep.bias = bias;
+  ep.mode = EPI_RESID; ep.M = M; ep.N = N; ep.x = x; ep.bias = bias; ep.step = 1;
   CKL(arcb_launch_gemm(a16, w, ep, K, act_format == ARCB_ACT_F16, tc, (cudaStream_t)stream, variant), "gemm");
   return ARCB_OK;
 }

@@ -103,6 +103,7 @@ struct GemmEpilogue {
   float* y;      // EPI_STORE_F32: [M][N]
   float* x;      // EPI_RESID: residual stream [M][N], updated in place
   const float* bias;  // EPI_RESID: [N] or null; EPI_SWIGLU: [N] packed like the weight rows
+  int step;      // the rows are one step of as many sequences, not rows of prompts: sums over K may be divided by the row count
   float* splitk_scratch;  // EPI_RESID, optional: >= 128 * ceil(M / 128) * N floats; allows the split-K kernel for few-row launches
   void* out16;   // EPI_QKV_ROPE: q16 [M][d]; EPI_SWIGLU: h16 [M][N/2]
   // EPI_QKV_ROPE
@@ -398,4 +399,81 @@ __device__ __forceinline__ void epi_glu_quad(const GemmEpilogue& e, int m, int n
     if (e.act_f16 == 1 && fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))) > 65504.f) arcb_count_saturation(e.err);
   }
   st_act4(e.out16, at, v, e.act_f16);
+}
+
+// What a quad's epilogue needs besides its sums, fetched while the products are still on their way.
+struct QuadAhead {
+  float4 a, b;
+  RopeRow rr;
+  template <int MODE>
+  __device__ __forceinline__ void load(const GemmEpilogue& ep, int m, int n) {
+    if constexpr (MODE == EPI_RESID) {
+      a = resid_old(ep, m, n);
+      b = bias_quad(ep, n);
+    } else if constexpr (MODE == EPI_SWIGLU) {
+      a = bias_quad(ep, n);
+      b = bias_quad(ep, n + 64);
+    } else if constexpr (MODE == EPI_QKV_ROPE) {
+      rr = rope_row_ctx(ep, m);
+      float2 c0, c1;
+      qkv_cs(ep, rr, n, c0, c1);
+      a = make_float4(c0.x, c0.y, c1.x, c1.y);
+    }
+  }
+};
+
+// Columns n .. n + 3 of row m (-1: none) of a fused mixer projection (ProjArgs).  head_sum(sum of squares, whether it is
+// wanted, columns of the head, column of the quad in it) adds the squares of the row's head; it is called by all threads or
+// by none.
+template <typename HeadSum>
+__device__ __forceinline__ void epi_heads_quad(const GemmEpilogue& ep, int m, int n, float4 v, HeadSum&& head_sum) {
+  const ProjArgs& p = ep.pj;
+  const bool gates = p.off_gate >= 0 && n >= p.off_gate;
+  const bool is_q = !gates && n < p.H * p.dimp;
+  const bool is_g = !gates && p.off_g >= 0 && n >= p.off_g;
+  const bool is_v = !gates && !is_g && p.off_v >= 0 && n >= p.off_v;
+  const bool is_k = !gates && !is_q && !is_g && !is_v && p.off_k >= 0;
+  const int sec0 = is_q ? p.off_q : is_k ? p.off_k : is_v ? p.off_v : p.off_g;
+  const int width = (is_q || is_k) ? p.dimp : p.vdimp;
+  const float* gain = is_q ? p.q_norm : is_k ? p.k_norm : nullptr;
+  // biases of whole heads exist in attention layers; the recurrence's bias vector only serves its gates
+  const float* bias = p.recurrent && !gates ? nullptr : p.bias;
+  if (bias) {
+    const float4 b = __ldg(reinterpret_cast<const float4*>(bias + n));
+    v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+  }
+  float post = 1.f;
+  const int in_head = (n - sec0) & (width - 1);
+  if (p.q_norm || p.k_norm) {
+    const float sum = head_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w), gain != nullptr && m >= 0, width, in_head);
+    if (gain) post = 1.f / sqrtf(sum / (float)p.dim + p.eps);
+  }
+  if (m < 0) return;
+  if (gates) {
+    const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n + i - p.off_gate < 2 * p.H) p.gates[(size_t)m * 2 * p.H + n + i - p.off_gate] = x[i];
+    return;
+  }
+  if (!is_q && !is_g && !is_v && !is_k) return;  // padding columns behind the last section
+  if (is_g && n >= p.off_g + p.H * p.vdimp) return;
+  if (is_v && p.off_g < 0 && n >= p.off_v + p.G * p.vdimp) return;
+  if (is_g) {
+    v = make_float4(sigmoid_f(v.x), sigmoid_f(v.y), sigmoid_f(v.z), sigmoid_f(v.w));
+  } else {
+    if (is_q) post *= query_gain(p, p.pos ? max(p.pos[m], 0) : 0);
+    v.x *= post; v.y *= post; v.z *= post; v.w *= post;
+    if (gain) {
+      const float4 g = __ldg(reinterpret_cast<const float4*>(gain + in_head));
+      v.x *= g.x; v.y *= g.y; v.z *= g.z; v.w *= g.w;
+    }
+  }
+  uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + (size_t)m * p.N + n;
+  if (!p.recurrent && (is_k || is_v)) {
+    const long long cr = proj_cache_row(p, m);
+    if (cr < 0) return;
+    dst = reinterpret_cast<uint16_t*>(is_k ? p.kcache : p.vcache) + (size_t)(cr + (long long)((n - sec0) / width) * p.t_max) * width + in_head;
+  }
+  *reinterpret_cast<uint2*>(dst) = make_uint2(pack2_act_chk(v.x, v.y, ep.act_f16, ep.err), pack2_act_chk(v.z, v.w, ep.act_f16, ep.err));
 }

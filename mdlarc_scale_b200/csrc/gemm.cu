@@ -10,6 +10,7 @@
 #include <cstdlib>
 
 #include "gemm.cuh"
+#include "gemm_mid.cuh"
 #include "gemm_rows.cuh"
 #include "launch.cuh"
 #include "ptx_sm100.cuh"
@@ -1498,6 +1499,7 @@ static cudaError_t set_tc2_smem_attr() {
 int arcb_gemm_init() {
   cudaError_t e;
   if (const int r = arcb_gemm_rows_init()) return r;
+  if (const int r = arcb_gemm_mid_init()) return r;
   if ((e = set_tc_smem_attr<EPI_STORE_F32>()) != cudaSuccess) return (int)e;
   if ((e = set_tc_smem_attr<EPI_QKV_ROPE>()) != cudaSuccess) return (int)e;
   if ((e = set_tc_smem_attr<EPI_RESID>()) != cudaSuccess) return (int)e;
@@ -1724,6 +1726,7 @@ int arcb_launch_gemm(const void* a16, const void* w16, const GemmEpilogue& ep, i
   if (N % 128 != 0 || K % 32 != 0) return -1;
   if (use_tc && (act_f16 == 2 || !arcb_gemm_tc_supported(M, N, K))) return -1;
   if (use_tc && tc_variant == 0 && arcb_gemm_rows_applies(a16, w16, ep, K, act_f16)) return arcb_launch_gemm_rows(a16, w16, ep, K, act_f16, stream);
+  if (use_tc && tc_variant == 0 && arcb_gemm_mid_applies(a16, w16, ep, K, act_f16)) return arcb_launch_gemm_mid(a16, w16, ep, K, act_f16, stream);
   switch (ep.mode) {
     case EPI_STORE_F32: return launch_gemm_mode<EPI_STORE_F32>(a16, w16, ep, K, act_f16, use_tc, tc_variant, stream);
     case EPI_QKV_ROPE: return launch_gemm_mode<EPI_QKV_ROPE>(a16, w16, ep, K, act_f16, use_tc, tc_variant, stream);

@@ -66,92 +66,22 @@ __device__ __forceinline__ int gr_col(int blk, int nt) {
   return (blk * NT + nt) * 16;
 }
 
-// What a quad's epilogue needs besides its sums, fetched while the products are still on their way.
-struct GrAhead {
-  float4 a, b;
-  RopeRow rr;
-  template <int MODE>
-  __device__ __forceinline__ void load(const GemmEpilogue& ep, int m, int n) {
-    if constexpr (MODE == EPI_RESID) {
-      a = resid_old(ep, m, n);
-      b = bias_quad(ep, n);
-    } else if constexpr (MODE == EPI_SWIGLU) {
-      a = bias_quad(ep, n);
-      b = bias_quad(ep, n + 64);
-    } else if constexpr (MODE == EPI_QKV_ROPE) {
-      rr = rope_row_ctx(ep, m);
-      float2 c0, c1;
-      qkv_cs(ep, rr, n, c0, c1);
-      a = make_float4(c0.x, c0.y, c1.x, c1.y);
-    }
-  }
-};
-
-// Quad q of a CTA's 16 columns of a fused mixer projection (ProjArgs), row m (-1: none).  A head's 64 or 128 columns lie
-// in 4 or 8 CTAs of one cluster, which exchange their rows' sums of squares through shared memory.
+// A head's 64 or 128 columns lie in 4 or 8 CTAs of one cluster, which exchange their rows' sums of squares through shared
+// memory; every thread of the cluster takes part.
 template <int ROWS>
-__device__ __forceinline__ void heads_quad(const GemmEpilogue& ep, int m, int row, int n0, int q, float4 v) {
-  const ProjArgs& p = ep.pj;
+__device__ __forceinline__ float cluster_head_sum(float ss, int row, int q, bool wanted, int width, int in_head) {
   __shared__ float part[ROWS];
-  const int n = n0 + q * 4;
-  const bool gates = p.off_gate >= 0 && n0 >= p.off_gate;
-  const bool is_q = !gates && n0 < p.H * p.dimp;
-  const bool is_g = !gates && p.off_g >= 0 && n0 >= p.off_g;
-  const bool is_v = !gates && !is_g && p.off_v >= 0 && n0 >= p.off_v;
-  const bool is_k = !gates && !is_q && !is_g && !is_v && p.off_k >= 0;
-  const int sec0 = is_q ? p.off_q : is_k ? p.off_k : is_v ? p.off_v : p.off_g;
-  const int width = (is_q || is_k) ? p.dimp : p.vdimp;
-  const float* gain = is_q ? p.q_norm : is_k ? p.k_norm : nullptr;
-  // biases of whole heads exist in attention layers; the recurrence's bias vector only serves its gates
-  const float* bias = p.recurrent && !gates ? nullptr : p.bias;
-  if (bias) {
-    const float4 b = __ldg(reinterpret_cast<const float4*>(bias + n));
-    v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+  ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+  if (q == 0 && row < ROWS) part[row] = ss;
+  sm100::cluster_sync_all();
+  float sum = 0.f;
+  if (wanted) {
+    const uint32_t first = sm100::cluster_ctarank() - (uint32_t)(in_head >> 4);
+    for (int c = 0; c < width >> 4; ++c) sum += sm100::ld_shared_cluster_f32(sm100::smem_u32(part + row), first + c);
   }
-  float post = 1.f;
-  if (p.q_norm || p.k_norm) {                    // the same for the whole cluster
-    float ss = (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
-    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-    if (q == 0 && row < ROWS) part[row] = ss;
-    sm100::cluster_sync_all();
-    if (gain && m >= 0) {
-      const uint32_t first = sm100::cluster_ctarank() - (((n0 - sec0) & (width - 1)) >> 4);
-      float sum = 0.f;
-      for (int c = 0; c < width >> 4; ++c) sum += sm100::ld_shared_cluster_f32(sm100::smem_u32(part + row), first + c);
-      post = 1.f / sqrtf(sum / (float)p.dim + p.eps);
-    }
-    sm100::cluster_sync_all();                   // nobody leaves while its sums are read
-  }
-  if (m < 0) return;
-  if (gates) {
-    const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (n + i - p.off_gate < 2 * p.H) p.gates[(size_t)m * 2 * p.H + n + i - p.off_gate] = x[i];
-    return;
-  }
-  if (!is_q && !is_g && !is_v && !is_k) return;  // padding columns behind the last section
-  if (is_g && n0 >= p.off_g + p.H * p.vdimp) return;
-  if (is_v && p.off_g < 0 && n0 >= p.off_v + p.G * p.vdimp) return;
-  const int in_head = (n - sec0) & (width - 1);
-  if (is_g) {
-    v = make_float4(sigmoid_f(v.x), sigmoid_f(v.y), sigmoid_f(v.z), sigmoid_f(v.w));
-  } else {
-    if (is_q) post *= query_gain(p, p.pos ? max(p.pos[m], 0) : 0);
-    v.x *= post; v.y *= post; v.z *= post; v.w *= post;
-    if (gain) {
-      const float4 g = __ldg(reinterpret_cast<const float4*>(gain + in_head));
-      v.x *= g.x; v.y *= g.y; v.z *= g.z; v.w *= g.w;
-    }
-  }
-  uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + (size_t)m * p.N + n;
-  if (!p.recurrent && (is_k || is_v)) {
-    const long long cr = proj_cache_row(p, m);
-    if (cr < 0) return;
-    dst = reinterpret_cast<uint16_t*>(is_k ? p.kcache : p.vcache) + (size_t)(cr + (long long)((n - sec0) / width) * p.t_max) * width + in_head;
-  }
-  *reinterpret_cast<uint2*>(dst) = make_uint2(pack2_act_chk(v.x, v.y, ep.act_f16, ep.err), pack2_act_chk(v.z, v.w, ep.act_f16, ep.err));
+  sm100::cluster_sync_all();                     // nobody leaves while its sums are read
+  return sum;
 }
 
 template <int NT, int MT, int MODE, bool F16>
@@ -202,7 +132,7 @@ __device__ __forceinline__ void rows_product(const uint16_t* A, const uint16_t* 
     if constexpr (Cfg::RING) asm volatile("cp.async.commit_group;" ::: "memory");
   }
   constexpr int QUADS = gr_paired<MODE>() ? 2 * NT : 4 * NT;         // output quads of a row
-  GrAhead ahead;
+  QuadAhead ahead;
   if constexpr (MODE != EPI_HEADS && MT <= 4) {
     const int row = threadIdx.x / QUADS;
     if (row < Cfg::ROWS && m0 + row < ep.M) ahead.load<MODE>(ep, m0 + row, n0 + (threadIdx.x - row * QUADS) * 4);
@@ -282,7 +212,8 @@ __device__ __forceinline__ void rows_product(const uint16_t* A, const uint16_t* 
     static_assert(NT == 1 && Cfg::ROWS * 4 <= GR_THREADS, "one quad a thread");
     const int row = threadIdx.x >> 2, q = threadIdx.x & 3;
     const bool in = row < Cfg::ROWS && m0 + row < ep.M;
-    heads_quad<Cfg::ROWS>(ep, in ? m0 + row : -1, row, n0, q, in ? total(row, q * 4) : make_float4(0.f, 0.f, 0.f, 0.f));
+    epi_heads_quad(ep, in ? m0 + row : -1, n0 + q * 4, in ? total(row, q * 4) : make_float4(0.f, 0.f, 0.f, 0.f),
+                   [&](float ss, bool wanted, int width, int in_head) { return cluster_head_sum<Cfg::ROWS>(ss, row, q, wanted, width, in_head); });
     return;
   }
   for (int u = threadIdx.x; u < Cfg::ROWS * QUADS; u += GR_THREADS) {

@@ -755,7 +755,7 @@ struct Rows {
 int lm_store32(arcb_session* s, const void* a, const void* w, int K, int N, int rows, float* out, bool step, cudaStream_t stream) {
   const LayeredModel& m = *s->eng->lm;
   GemmEpilogue er{};
-  er.mode = EPI_RESID; er.M = rows; er.N = N; er.x = out; er.overwrite = 1; er.act_f16 = m.fmt; er.err = s->eng->d_err;
+  er.mode = EPI_RESID; er.M = rows; er.N = N; er.x = out; er.overwrite = 1; er.act_f16 = m.fmt; er.err = s->eng->d_err; er.step = step;
   er.splitk_scratch = step && N <= m.n_wide_max ? s->ls->gemm_scratch : nullptr;
   CKL(lm_gemm(m, a, w, er, K, stream), "gemm");
   return ARCB_OK;
@@ -768,6 +768,7 @@ int lm_residual(arcb_session* s, const void* a, const void* w, int K, int rows, 
   er.mode = EPI_RESID; er.M = rows; er.N = m.wp; er.act_f16 = m.fmt; er.err = s->eng->d_err;
   er.x = m.sandwich() ? s->ls->y : s->ls->x;
   er.overwrite = m.sandwich() ? 1 : 0;
+  er.step = step;
   er.splitk_scratch = step ? s->ls->gemm_scratch : nullptr;
   CKL(lm_gemm(m, a, w, er, K, stream), "residual gemm");
   return ARCB_OK;
@@ -800,7 +801,7 @@ int lm_latent(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
   p.cq = ls->cq; p.cache = ls->k[l]; p.pos = R.pos; p.seq = R.seq; p.t_max = T; p.n_seqs = B; p.fmt = m.fmt; p.err = s->eng->d_err;
   CKL(arcb_launch_latent_prep(p, stream), "latent prep");
   GemmEpilogue eq{};
-  eq.mode = EPI_ACT; eq.M = R.n; eq.N = L.n_proj; eq.out16 = ls->proj; eq.act_f16 = m.fmt; eq.err = s->eng->d_err;
+  eq.mode = EPI_ACT; eq.M = R.n; eq.N = L.n_proj; eq.out16 = ls->proj; eq.act_f16 = m.fmt; eq.err = s->eng->d_err; eq.step = R.pa == nullptr;
   if (rot) eq.rot = RotArgs{rot, R.pos, L.rotp / 2, qh, L.dimp, T};
   CKL(lm_gemm(m, ls->cq, L.w_uq, eq, L.q_rankp, stream), "query gemm");
 
@@ -858,7 +859,7 @@ int lm_mlp(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
   const arcb_layer_desc& d = L.d;
   const bool step = R.pa == nullptr;
   GemmEpilogue eu{};
-  eu.M = R.n; eu.out16 = ls->hid; eu.act_f16 = m.fmt; eu.err = s->eng->d_err;
+  eu.M = R.n; eu.out16 = ls->hid; eu.act_f16 = m.fmt; eu.err = s->eng->d_err; eu.step = step;
   if (d.mlp == ARCB_MLP_RELU2) {
     eu.mode = EPI_RELU2; eu.N = L.ffp;
     CKL(lm_gemm(m, ls->xn, L.w_up, eu, m.wp, stream), "up gemm");
@@ -933,7 +934,7 @@ int lm_mixer(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
   p.pos = R.pos; p.seq = R.seq; p.kcache = ls->k[l]; p.vcache = ls->v[l]; p.t_max = T; p.n_seqs = B;
   p.out = ls->proj; p.gates = ls->gates; p.fmt = m.fmt; p.err = s->eng->d_err;
   GemmEpilogue ep{};
-  ep.M = R.n; ep.N = L.n_proj; ep.act_f16 = m.fmt; ep.err = s->eng->d_err;
+  ep.M = R.n; ep.N = L.n_proj; ep.act_f16 = m.fmt; ep.err = s->eng->d_err; ep.step = R.pa == nullptr;
   if (use_fused(m)) {
     ep.mode = EPI_HEADS; ep.pj = p;
     CKL(lm_gemm(m, ls->xn, L.w_proj, ep, m.wp, stream), "fused projection gemm");
@@ -1057,7 +1058,7 @@ int lm_head(arcb_session* s, int mode, int rows, const int* index, float* out, c
     a.x_scale = 1.f; a.x = ls->x; a.w = m.final_norm; a.xn = ls->hn; a.write_x = 0; a.row_index = index ? index + r0 : nullptr;
     CKL(arcb_launch_lm_norm(a, stream), "final norm");
     GemmEpilogue ep{};
-    ep.mode = EPI_STORE_F32; ep.M = n; ep.N = m.vp; ep.y = ls->logits; ep.act_f16 = m.fmt; ep.err = s->eng->d_err;
+    ep.mode = EPI_STORE_F32; ep.M = n; ep.N = m.vp; ep.y = ls->logits; ep.act_f16 = m.fmt; ep.err = s->eng->d_err; ep.step = mode == PICK_DECODE;
     CKL(lm_gemm(m, ls->hn, m.head, ep, m.wp, stream), "head gemm");
     PickArgs p{};
     p.mode = mode; p.rows = n; p.vocab = m.d.vocab; p.pitch = m.vp; p.logits = ls->logits; p.scale = m.d.logit_scale;

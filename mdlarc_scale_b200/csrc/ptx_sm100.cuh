@@ -289,6 +289,19 @@ __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t addr, uint32_t r
       : "memory");
   return v;
 }
+__device__ __forceinline__ float4 ld_shared_cluster_v4(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n"
+      ".reg .b32 a;\n"
+      "mapa.shared::cluster.u32 a, %4, %5;\n"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n"
+      "}\n"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
 __device__ __forceinline__ void st_shared_cluster_f32(uint32_t addr, uint32_t rank, float v) {
   asm volatile(
       "{\n"
