@@ -638,7 +638,7 @@ extern "C" int arcb_op_gemm(const void* a16, const void* w, float* y, int32_t M,
     tc = false;
   }
   GemmEpilogue ep{};
-  ep.mode = EPI_STORE_F32; ep.M = M; ep.N = N; ep.y = y; ep.step = 1;
+  ep.mode = EPI_STORE_F32; ep.M = M; ep.N = N; ep.y = y;
   CKL(arcb_launch_gemm(a16, w, ep, K, act_format == ARCB_ACT_F16, tc, (cudaStream_t)stream, variant), "gemm");
   return ARCB_OK;
 }

@@ -1725,8 +1725,8 @@ int arcb_launch_gemm(const void* a16, const void* w16, const GemmEpilogue& ep, i
   if (M <= 0) return 0;
   if (N % 128 != 0 || K % 32 != 0) return -1;
   if (use_tc && (act_f16 == 2 || !arcb_gemm_tc_supported(M, N, K))) return -1;
-  if (use_tc && tc_variant == 0 && arcb_gemm_rows_applies(a16, w16, ep, K, act_f16)) return arcb_launch_gemm_rows(a16, w16, ep, K, act_f16, stream);
   if (use_tc && tc_variant == 0 && arcb_gemm_mid_applies(a16, w16, ep, K, act_f16)) return arcb_launch_gemm_mid(a16, w16, ep, K, act_f16, stream);
+  if (use_tc && tc_variant == 0 && arcb_gemm_rows_applies(a16, w16, ep, K, act_f16)) return arcb_launch_gemm_rows(a16, w16, ep, K, act_f16, stream);
   switch (ep.mode) {
     case EPI_STORE_F32: return launch_gemm_mode<EPI_STORE_F32>(a16, w16, ep, K, act_f16, use_tc, tc_variant, stream);
     case EPI_QKV_ROPE: return launch_gemm_mode<EPI_QKV_ROPE>(a16, w16, ep, K, act_f16, use_tc, tc_variant, stream);

@@ -1,4 +1,4 @@
-// y = A[M,K] * W[N,K]^T for one tile of up to 256 rows (decode steps of mid-sized batches), epilogues of epilogue.cuh.
+// y = A[M,K] * W[N,K]^T for one tile of up to 256 rows (decode steps of mid-sized batches, wide heads), epilogues of epilogue.cuh.
 //
 // With 128 x 128 tiles of A rows and W rows, such a product is 8 to 65 CTAs that each pull (128 + 128) x K operands through
 // one SM's 110 GB/s, one after the other.  Here the product is transposed: 128 rows of W are the matrix instruction's rows
@@ -304,7 +304,11 @@ int arcb_gemm_mid_init() {
 // Decode steps only: how a sum is divided depends on the number of rows, and a prompt row's result does not depend on what
 // else its call holds.
 bool arcb_gemm_mid_applies(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16) {
-  if (!ep.step || ep.M <= 64 || ep.M > 256 || act_f16 == 2 || K % 64 || ep.N % 128) return false;
+  // Fewer rows are quicker on gemm_rows.cu up to 32 (us a launch here / there: 32 rows, 1280 x 1280 6.6 / 5.4, 5504 x 1024 8.7 / 7.0;
+  // 48 rows, 7.0 / 7.5 and 8.0 / 9.7), unless a CTA there has long sums of its own (24 rows, 1280 x 3456 7.8 / 10.5) or every SM
+  // several of its CTAs (16 rows, 32000 x 1280 17 / 24)
+  const bool here = ep.M > 32 || (ep.M > 16 && K >= 2560) || ep.N / 128 > 148;
+  if (!ep.step || !here || ep.M > 256 || act_f16 == 2 || K % 64 || ep.N % 128) return false;
   const GroupArgs& g = ep.grp;
   if (g.tile_src || g.tile_group || g.n_tiles || g.panels || g.n_group || g.lda % 8) return false;
   // 16-byte accesses of the epilogues' quads; what is not aligned meets the tensor maps' refusal

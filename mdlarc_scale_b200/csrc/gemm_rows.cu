@@ -12,8 +12,8 @@
 //     with the first activations, not behind the last sum;
 //   * the eight warps' sums meet in shared memory, always in the same order, and leave through the epilogues' quads.
 // B200, us a launch inside the captured step, tcgen05 tiles / here: 16 rows, QKV of width 1024 10.3 / 4.6, gate/up 10.6 / 5.4,
-// out and down 10.7 / 3.9; 1 row of width 256 6.1 to 6.8 / 1.9 to 2.4; 1 row, mixer projection of width 1280 14.2 / 6.5, its
-// 32 000-column head 26 / 18 (82 MB: 4.6 TB/s); 48 rows of width 1280, outputs 10.9 / 9.0, gated units 12.7 / 10.5.
+// out and down 10.7 / 3.9; 1 row of width 256 6.1 to 6.8 / 1.9 to 2.4; 1 row, mixer projection of width 1280 14.2 / 6.5.
+// Prompt portions of up to 64 rows, and steps that gemm_mid.cu does not take.
 #include "common.cuh"
 #include "gemm.cuh"
 #include "gemm_rows.cuh"
@@ -314,8 +314,8 @@ int arcb_gemm_rows_init() {
 }
 
 // Up to 64 rows: the weights' 16-row fragments meet eight 8-row activation fragments, and the activations of a CTA
-// (64 rows x K) are re-read from L2 by every CTA; the step of the latent-attention model with 48 rows takes 3 % less
-// with it.  One row tile more would read the weights twice.
+// (64 rows x K) are re-read from L2 by every CTA (48 rows of width 1280, tcgen05 tiles / here: outputs 10.9 / 9.0, gated units
+// 12.7 / 10.5 us).  One row tile more would read the weights twice.
 bool arcb_gemm_rows_applies(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16) {
   if (ep.M > 64 || act_f16 == 2 || K % 32 || ep.N % 128) return false;
   const GroupArgs& g = ep.grp;

@@ -117,20 +117,17 @@ def test_few_row_products(lib, M, N, K, fmt):
 
 
 @pytest.mark.parametrize("fmt", [_lib.ACT_F16, _lib.ACT_BF16])
-@pytest.mark.parametrize("M", [65, 80, 127, 128, 129, 150, 241, 256, 257])
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65, 127, 128, 129, 150, 241, 256, 257])
 @pytest.mark.parametrize("N,K", [(128, 64), (384, 256), (1024, 2752), (3072, 1024), (8448, 320), (19200, 256)])
 def test_mid_row_products(lib, M, N, K, fmt):
-    """One tile of 65 to 256 rows and one row beyond: fewer K blocks than CTAs of a cluster, uneven shares of them, clusters
-    of one to eight, more tiles than SMs."""
+    """Transposed tiles of up to 256 rows, and on the other side of their rule: fewer K blocks than CTAs of a cluster, uneven
+    shares of them, clusters of one to eight, more tiles than SMs."""
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     a = to_act(torch.randn(M, K, device="cuda", generator=g), fmt)
     w = to_act((torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).to(torch.bfloat16).float(), fmt)
     bias = torch.randn(N, device="cuda", generator=g)
     ref = a.double() @ w.double().T
     bound = (a.double().abs() @ w.double().abs().T) * 2 ** -24 * (K / 16 + 16)
-    y = torch.full((M + 1, N), 7.0, device="cuda")
-    _lib.check(lib.arcb_op_gemm(a.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, K, fmt, _lib.GEMM_AUTO, stream()))
-    assert ((y[:M].double() - ref).abs() <= bound).all() and (y[M] == 7).all()
     x0 = torch.randn(M + 1, N, device="cuda", generator=g)
     got = []
     for _ in range(2):
@@ -140,6 +137,25 @@ def test_mid_row_products(lib, M, N, K, fmt):
     assert torch.equal(got[0], got[1]) and torch.equal(got[0][M], x0[M])
     ref = ref + x0[:M].double() + bias.double()
     assert ((got[0][:M].double() - ref).abs() <= bound + (ref.abs() + x0[:M].double().abs() + bias.double().abs()) * 2 ** -22).all()
+
+
+@pytest.mark.parametrize("fmt", ["f16", "bf16"])
+@pytest.mark.parametrize("slots", [33, 80, 131])
+@pytest.mark.parametrize("name", ["mixed", "plain_heads", "wide_group", "unequal"])
+def test_mid_row_steps(name, slots, fmt):
+    """A decode step of that many sequences: heads of 64 and 128 columns with and without norms, gates, caches, vocabularies."""
+    from vodavik_util import CONFIGS
+    cfg = CONFIGS[name]
+    w = vo.random_weights(cfg, 5)
+    eng = registry.build_engine(cfg, w, "cuda:0", fmt)
+    s = eng.new_session(slots, 16, 1, 8 * slots, stop_on_end=False)
+    toks = [tokens(cfg, 2 + i % 6, 100 + i) for i in range(slots)]
+    at = [s.acquire() for _ in range(slots)]
+    s.step([Segment(a, t[:-1], []) for a, t in zip(at, toks)])
+    got = torch.cat(s.step([Segment(a, t[-1:], [0]) for a, t in zip(at, toks)]))
+    s.poll()
+    want = torch.stack([oracle_logits(cfg, w, t)[-1] for t in toks])
+    assert rel_error(got, want) < (1e-2 if fmt == "f16" else 6e-2)
 
 
 @pytest.mark.parametrize("M,N,K", [(32, 128, 32), (33, 128, 32), (64, 384, 96), (65, 256, 64), (700, 1280, 320), (2500, 2048, 96)])
