@@ -530,10 +530,173 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 //
 // 640 threads: warps 0-3 helpers (TMA producer, issuer A, issuer B, one idle), warps 4-7 / 8-11
 // tile A halves 0 / 1, warps 12-15 / 16-19 tile B halves 0 / 1.  Registers are re-divided after
-// start-up (setmaxnreg): the helper warpgroup keeps 24, the four softmax warpgroups get 112 each
-// (24 * 128 + 112 * 512 = 60 416 of the 65 536, so the increase can never wait for registers).
+// start-up (setmaxnreg): the helper warpgroup keeps 32, the four softmax warpgroups get 112 each
+// (32 * 128 + 112 * 512 = 96 * 640, what the block was launched with, so the increase never waits for good).
 // ---------------------------------------------------------------------------------------------
 constexpr int SPLIT_THREADS = 640;
+constexpr int SPLIT_SMEM_BYTES = SMEM_BYTES + 2 * Q_BYTES;   // Q tiles of two items
+
+// One CTA an SM takes items (query block x head) from a common counter, a head's blocks most expensive first.  An item's chain
+// (block description, Q and K, scores, softmax, P V, normaliser, store) is 15 us for 250 keys when nothing else runs beside it;
+// here the producer reads and fetches the next item while this one is worked on, and its first scores are computed behind
+// this one's last product.  A fixed division of the items measured 8 % slower on four prompts of 10 k tokens: what is even
+// (all heads' most expensive blocks first) does not keep keys in L2, what keeps them there is not even.
+// B200, us a launch, an item a CTA / this: 262 prompts of 250 tokens, 20 heads 543 / 370, 150 prompts of about 360
+// tokens 431 / 311, 20 of 2 k tokens 700 / 635, 4 of 10 k tokens 1740 / 1720; 37 prompts of 64 to 500 tokens, 12 heads 92.5 / 73.6;
+// 60 items in all (fewer than SMs) 26 / 27.
+struct FlashItem { int row0, rows, n_a, n_b, head; };    // rows < 0: the list has ended
+
+// Barriers of the items: Q full / empty by item parity.  Empty: two issuers and the 16 softmax warps, which also read the
+// item's description.
+struct ItemBars { uint32_t full, empty; };
+
+// Description of an item as warp 0 holds it: lane i has the counts of rows i, 32 + i, ...
+struct FlashWork {
+  int row0, rows, kv0, head, cnt[8];
+  __device__ __forceinline__ void load(int item, const AttnPrefillArgs& a) {
+    const int lane = threadIdx.x & 31;
+    head = item / a.n_qblocks;
+    const int blk = item - head * a.n_qblocks;
+    row0 = a.qblock_row0[blk];
+    rows = a.qblock_rows[blk];               // 1..256
+    kv0 = a.qblock_kv0[blk];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) cnt[i] = i * 32 + lane < rows ? a.kv_count[row0 + i * 32 + lane] : 0;
+  }
+};
+
+// Warp 0, all lanes; `w`: the CTA's first item.  Counts and descriptions reach the others through shared memory, ahead of Q's
+// barrier.
+__device__ __forceinline__ void flash_items_producer(const CUtensorMap* tmap_q, const CUtensorMap* tmap_k, const CUtensorMap* tmap_v,
+                                                     const Bars& B, const ItemBars& I, uint32_t q_smem, uint32_t kv_smem,
+                                                     const AttnPrefillArgs& a, FlashWork& w, FlashItem* s_item, int (*s_cnt)[2 * BQ]) {
+  const int lane = threadIdx.x & 31, total = a.n_qblocks * a.n_heads;
+  int tile = 0;                                  // key tiles of all items so far
+  bool more = true;
+  for (int k = 0;; ++k) {
+    int most[2] = {0, 0};
+    if (more) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) most[i >> 2] = max(most[i >> 2], w.cnt[i]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        most[0] = max(most[0], __shfl_xor_sync(0xffffffffu, most[0], o));
+        most[1] = max(most[1], __shfl_xor_sync(0xffffffffu, most[1], o));
+      }
+    }
+    const int n_a = (most[0] + BKV - 1) / BKV, n_b = (most[1] + BKV - 1) / BKV, n_tiles = max(n_a, n_b), par = k & 1;
+    const bool good = mbar_wait_bounded(I.empty + 8 * par, ((k >> 1) & 1) ^ 1);
+    if (!__all_sync(0xffffffffu, good)) {
+      if (lane == 0) arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_MMA);
+      return;
+    }
+    if (!more) {
+      if (lane == 0) {
+        s_item[par].rows = -1;
+        mbar_arrive(I.full + 8 * par);
+      }
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s_cnt[par][i * 32 + lane] = w.cnt[i];
+    if (lane == 0) s_item[par] = FlashItem{w.row0, w.rows, n_a, n_b, w.head};
+    __syncwarp();
+    int next = -1;
+    if (lane == 0) {
+      const bool two = w.rows > BQ;
+      const uint32_t dst = q_smem + par * 2 * Q_BYTES;
+      mbar_expect_tx(I.full + 8 * par, two ? 2 * Q_BYTES : Q_BYTES);
+      tma_load_2d(dst, tmap_q, w.head * HD, w.row0, I.full + 8 * par);
+      if (two) tma_load_2d(dst + Q_BYTES, tmap_q, w.head * HD, w.row0 + BQ, I.full + 8 * par);
+      int j = 0;
+      for (; j < n_tiles; ++j, ++tile) {
+        const int s = tile % KV_STAGES;
+        if (!mbar_wait_bounded(B.kv_empty + 8 * s, ((tile / KV_STAGES) & 1) ^ 1)) {
+          arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_MMA);
+          break;
+        }
+        const uint32_t kv = kv_smem + s * 2 * KV_TILE_BYTES;
+        mbar_expect_tx(B.kv_full + 8 * s, 2 * KV_TILE_BYTES);
+        tma_load_2d(kv, tmap_k, w.head * HD, w.kv0 + j * BKV, B.kv_full + 8 * s);
+        tma_load_2d(kv + KV_TILE_BYTES, tmap_v, w.head * HD, w.kv0 + j * BKV, B.kv_full + 8 * s);
+      }
+      if (j == n_tiles) next = atomicAdd(a.next, 1);
+      // `total` fetches a launch (every CTA's last one finds nothing): the last of them leaves the counter as it was
+      if (next == total - 1) *a.next = 0;
+    }
+    next = __shfl_sync(0xffffffffu, next, 0);
+    if (next < 0) return;
+    next += gridDim.x;
+    more = next < total;
+    if (more) w.load(next, a);
+  }
+}
+
+// One thread: the products of Q tile x, as flash_mma_issuer, over all items.
+__device__ __forceinline__ void flash_items_issuer(int x, const Bars& B, const ItemBars& I, uint32_t q_smem, uint32_t kv_smem,
+                                                   uint32_t tmem_base, const FlashItem* s_item, uint32_t idesc_qk,
+                                                   uint32_t idesc_pv, int* err) {
+  bool ok = true;
+  auto wait_or_flag = [&](uint32_t bar, uint32_t parity, int code) {
+    if (ok && !mbar_wait_bounded(bar, parity)) {
+      arcb_set_error(err, code);
+      ok = false;
+    }
+  };
+  int done = 0, tile = 0;                        // this Q tile's products, and key tiles, of the items before
+  for (int k = 0;; ++k) {
+    const int par = k & 1;
+    wait_or_flag(I.full + 8 * par, (k >> 1) & 1, ARCB_DEV_WAIT_TIMEOUT_TMA);
+    if (!ok || s_item[par].rows < 0) return;
+    const int n_a = s_item[par].n_a, n_b = s_item[par].n_b, n_x = x ? n_b : n_a, n_tiles = max(n_a, n_b);
+    const uint64_t dq = umma_desc_k_sw128(q_smem + (par * 2 + x) * Q_BYTES);
+    auto mma_s = [&](int j) {  // S_x = Q_x K(j)^T
+      const uint64_t dk = umma_desc_k_sw128(kv_smem + ((tile + j) % KV_STAGES) * 2 * KV_TILE_BYTES);
+#pragma unroll
+      for (int ks = 0; ks < HD / 16; ++ks) umma_f16(tmem_base + x * 128, dq + 2 * ks, dk + 2 * ks, idesc_qk, ks ? 1u : 0u);
+      umma_commit(B.s[x]);
+      if (j == n_x - 1) umma_commit(I.empty + 8 * par);
+    };
+    auto mma_o = [&](int j) {  // O_x (+)= P_x V(j); then this tile is done with K/V stage j
+      const int s = (tile + j) % KV_STAGES;
+      const uint64_t dv = umma_desc_mn_sw128(kv_smem + s * 2 * KV_TILE_BYTES + KV_TILE_BYTES);
+#pragma unroll
+      for (int ks = 0; ks < BKV / 16; ++ks)
+        umma_f16_ts(tmem_base + 256 + x * 64, tmem_base + TMEM_P + x * 64 + ks * 8, dv + (uint64_t)(ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
+      umma_commit(B.o[x]);
+      umma_commit(B.kv_empty + 8 * s);
+    };
+    for (int j = 0; j < n_x; ++j) {
+      wait_or_flag(B.kv_full + 8 * ((tile + j) % KV_STAGES), ((tile + j) / KV_STAGES) & 1, ARCB_DEV_WAIT_TIMEOUT_TMA);
+      if (done + j > 0) wait_or_flag(B.sfree[x], (done + j - 1) & 1, ARCB_DEV_WAIT_TIMEOUT_ACC);   // the scores before are copied out
+      if (!ok) return;
+      tc_fence_after();
+      mma_s(j);
+      if (j > 0) {
+        wait_or_flag(B.p[x], (done + j - 1) & 1, ARCB_DEV_WAIT_TIMEOUT_ACC);
+        if (!ok) return;
+        tc_fence_after();
+        mma_o(j - 1);
+      }
+    }
+    if (n_x > 0) {
+      wait_or_flag(B.p[x], (done + n_x - 1) & 1, ARCB_DEV_WAIT_TIMEOUT_ACC);
+      if (!ok) return;
+      tc_fence_after();
+      mma_o(n_x - 1);
+    } else {
+      mbar_arrive(I.empty + 8 * par);
+    }
+    // stages that only the other Q tile uses go back as soon as they have landed, in order
+    for (int j = n_x; j < n_tiles; ++j) {
+      wait_or_flag(B.kv_full + 8 * ((tile + j) % KV_STAGES), ((tile + j) / KV_STAGES) & 1, ARCB_DEV_WAIT_TIMEOUT_TMA);
+      if (!ok) return;
+      mbar_arrive(B.kv_empty + 8 * ((tile + j) % KV_STAGES));
+    }
+    done += n_x;
+    tile += n_tiles;
+  }
+}
 
 template <int POLY>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
@@ -541,22 +704,25 @@ attn_prefill_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
                           const __grid_constant__ CUtensorMap tmap_v, AttnPrefillArgs a, uint32_t idesc_qk,
                           uint32_t idesc_pv) {
   pdl_launch_dependents();
-  pdl_wait();   // the prologue below already reads the work list from global memory
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
-  __shared__ int s_max_cnt[16];
-  __shared__ float s_xchg[2][2][2][BQ];   // [tile parity][Q tile][half][row]: half-tile maxima, then row sums
+  __shared__ FlashItem s_item[2];
+  __shared__ int s_cnt[2][2 * BQ];
+  __shared__ float s_xchg[2][2][2][BQ];   // [exchange parity][Q tile][half][row]: half-tile maxima, then row sums
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t q_smem = base;
-  const uint32_t kv_smem = base + 2 * Q_BYTES;
+  const uint32_t kv_smem = base + 4 * Q_BYTES;
   const uint32_t bar0 = kv_smem + KV_STAGES * 2 * KV_TILE_BYTES;
-  uint8_t* bar_ptr = base_ptr + 2 * Q_BYTES + KV_STAGES * 2 * KV_TILE_BYTES;
+  uint8_t* bar_ptr = base_ptr + 4 * Q_BYTES + KV_STAGES * 2 * KV_TILE_BYTES;
   Bars B;
-  B.q = bar0;
-  B.kv_full = bar0 + 8;
-  B.kv_empty = bar0 + 8 + 8 * KV_STAGES;
-  B.s[0] = bar0 + 8 + 16 * KV_STAGES;
+  ItemBars I;
+  I.full = bar0;
+  I.empty = bar0 + 16;
+  B.kv_full = bar0 + 32;
+  B.kv_empty = B.kv_full + 8 * KV_STAGES;
+  B.s[0] = B.kv_full + 16 * KV_STAGES;
   B.s[1] = B.s[0] + 8;
   B.p[0] = B.s[0] + 16;
   B.p[1] = B.s[0] + 24;
@@ -568,27 +734,19 @@ attn_prefill_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 256);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int blk = blockIdx.x, h = blockIdx.y;
-  const int row0 = a.qblock_row0[blk];
-  const int rows = a.qblock_rows[blk];  // 1..256
-  const int kv0 = a.qblock_kv0[blk];
 
   const int wg = (warp >> 2) - 1;          // softmax warpgroup 0..3 (helpers: -1)
   const int grp = wg >> 1;                 // Q tile
   const int half = wg & 1;                 // which 64 keys of a tile / which 32 output dims
   const int quarter = warp & 3;            // TMEM lane quarter this warp may touch
   const int r = quarter * 32 + lane;       // row inside the Q tile
-  int my_cnt = 0;
-  if (warp >= 4) {
-    const int qr = grp * BQ + r;
-    if (qr < rows) my_cnt = a.kv_count[row0 + qr];
-    int mx = my_cnt;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) s_max_cnt[warp - 4] = mx;
-  }
-  if (threadIdx.x == 0) {
-    mbar_init(B.q, 1);
+  FlashWork first;
+  if (warp == 0) first.load(blockIdx.x, a);
+  if (threadIdx.x == 64) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(I.full + 8 * s, 1);
+      mbar_init(I.empty + 8 * s, 18);
+    }
     for (int s = 0; s < KV_STAGES; ++s) {
       mbar_init(B.kv_full + 8 * s, 1);
       mbar_init(B.kv_empty + 8 * s, 2);
@@ -613,169 +771,171 @@ attn_prefill_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  int cnt_a = 0, cnt_b = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    cnt_a = max(cnt_a, s_max_cnt[i]);
-    cnt_b = max(cnt_b, s_max_cnt[8 + i]);
-  }
-  const int n_a = (cnt_a + BKV - 1) / BKV;
-  const int n_b = (cnt_b + BKV - 1) / BKV;
-  const int n_tiles = max(n_a, n_b);
 
   if (warp < 4) {
-    reg_dealloc_24();
+    reg_dealloc_32();
     if (warp == 0) {
-      if (lane == 0 && n_tiles > 0)
-        flash_tma_producer(&tmap_q, &tmap_k, &tmap_v, B, q_smem, kv_smem, h, row0, rows, kv0, n_tiles, a.err);
+      flash_items_producer(&tmap_q, &tmap_k, &tmap_v, B, I, q_smem, kv_smem, a, first, s_item, s_cnt);
     } else if (warp <= 2) {
-      if (lane == 0 && n_tiles > 0)
-        flash_mma_issuer(warp - 1, B, q_smem, kv_smem, tmem_base, n_a, n_b, idesc_qk, idesc_pv, a.err);
+      if (lane == 0) flash_items_issuer(warp - 1, B, I, q_smem, kv_smem, tmem_base, s_item, idesc_qk, idesc_pv, a.err);
     }
   } else {
     reg_alloc_112();
     // ---- softmax / output threads: row r of Q tile grp, key half `half` ----
-    const int n_mine = grp ? n_b : n_a;
     const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t t_s = t_lane + grp * 128 + half * 64;
     const uint32_t t_o = t_lane + 256 + grp * 64 + half * 32;
     const uint32_t t_p = t_lane + TMEM_P + grp * 64 + half * 32;
     const uint32_t xbar = xbar0 + 8 * (grp * 4 + quarter);
     const float sc = 0.125f * LOG2E;
-    float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
     uint32_t xphase = 0;
     // both threads of a row publish a value and read the partner's; false if the partner never came
-    auto exchange = [&](int slot, float mine, float& theirs) -> bool {
-      s_xchg[slot][grp][half][r] = mine;
+    auto exchange = [&](float mine, float& theirs) -> bool {
+      s_xchg[xphase][grp][half][r] = mine;
       mbar_arrive(xbar);
       const bool good = mbar_wait_bounded(xbar, xphase);
+      theirs = s_xchg[xphase][grp][half ^ 1][r];
       xphase ^= 1u;
-      theirs = s_xchg[slot][grp][half ^ 1][r];
       return good;
     };
-    for (int j = 0; j < n_mine; ++j) {
-      if (ok && !mbar_wait_bounded(B.s[grp], j & 1)) {
-        arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_ACC);
-        ok = false;
+    int done = 0;                          // key tiles of the items before
+    for (int k = 0; ok; ++k) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(I.full + 8 * (k & 1), (k >> 1) & 1))) {
+        arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_TMA);
+        break;
       }
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t sv[2][32];
-      tmem_ld_32x32(t_s, sv[0]);
-      tmem_ld_32x32(t_s + 32, sv[1]);
-      tmem_wait_ld_dep(sv[0]);
-      tmem_wait_ld_dep(sv[1]);
-      // this thread's share of S is in registers
-      tc_fence_before();
-      mbar_arrive(B.sfree[grp]);
-      const int n_valid = min(max(my_cnt - j * BKV, 0), BKV) - half * 64;   // visible keys within this half (may be <= 0)
-      if (!__all_sync(0xffffffffu, n_valid >= 64)) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (c * 32 + i >= n_valid) sv[c][i] = 0xff800000u;   // -inf: exp2 gives exactly 0
-      }
-      float mx2[2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        mx2[c] = fmaxf(__uint_as_float(sv[c][0]), __uint_as_float(sv[c][1]));
-#pragma unroll
-        for (int i = 2; i < 32; i += 2) mx2[c] = max3_f32(mx2[c], __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
-      }
-      float other;
-      bool good = exchange(j & 1, fmaxf(mx2[0], mx2[1]), other);
-      if (!good) arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_ACC);
-      ok = __all_sync(0xffffffffu, good);
-      if (!ok) break;
-      const float mx = fmaxf(fmaxf(mx2[0], mx2[1]), other) * sc;   // the same value in both threads of the row
-      float alpha = 1.f;
-      if (mx > m_ref + RESCALE_THRESHOLD) {  // also the first visible tile (m_ref = -inf)
-        alpha = (m_ref == -INFINITY) ? 0.f : ex2_fast(m_ref - mx);
-        m_ref = mx;
-      }
-      l *= alpha;
-      const float m_safe = (m_ref == -INFINITY) ? 0.f : m_ref;
-      const uint64_t sc2 = pack_f32x2(sc, sc), nm2 = pack_f32x2(-m_safe, -m_safe);
-      uint32_t pr[4][8];
-      // the 64 probabilities of this half-tile are summed as packed halves in a balanced tree (they are
-      // at most 2^8 each and almost always at most 1, so the tree stays far inside the half range) and
-      // leave half precision once per tile; the running row sum is fp32
-      __half2 gsum[4];
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        __half2 p[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int k = g * 8 + e;                    // this half's keys 2k, 2k + 1 = its P column k
-          float t0, t1;
-          shift2_f32(sv[k >> 4][(2 * k) & 31], sv[k >> 4][((2 * k) & 31) + 1], sc2, nm2, t0, t1);
-          p[e] = ex2_on_fma<POLY>(e) ? ex2_poly_half2(__floats2half2_rn(t0, t1))
-                                     : __floats2half2_rn(ex2_fast(t0), ex2_fast(t1));
+      if (s_item[k & 1].rows < 0) break;
+      const int n_mine = grp ? s_item[k & 1].n_b : s_item[k & 1].n_a, head = s_item[k & 1].head;
+      const int qr = grp * BQ + r;
+      const int my_cnt = s_cnt[k & 1][qr];
+      const int out_row = qr < s_item[k & 1].rows ? s_item[k & 1].row0 + qr : -1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(I.empty + 8 * (k & 1));
+      float m_ref = -INFINITY, l = 0.f;
+      for (int j = 0; j < n_mine; ++j) {
+        if (ok && !mbar_wait_bounded(B.s[grp], (done + j) & 1)) {
+          arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_ACC);
+          ok = false;
         }
-        gsum[g] = __hadd2(__hadd2(__hadd2(p[0], p[1]), __hadd2(p[2], p[3])),
-                          __hadd2(__hadd2(p[4], p[5]), __hadd2(p[6], p[7])));
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t sv[2][32];
+        tmem_ld_32x32(t_s, sv[0]);
+        tmem_ld_32x32(t_s + 32, sv[1]);
+        tmem_wait_ld_dep(sv[0]);
+        tmem_wait_ld_dep(sv[1]);
+        // this thread's share of S is in registers
+        tc_fence_before();
+        mbar_arrive(B.sfree[grp]);
+        const int n_valid = min(max(my_cnt - j * BKV, 0), BKV) - half * 64;   // visible keys within this half (may be <= 0)
+        if (!__all_sync(0xffffffffu, n_valid >= 64)) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) pr[g][e] = h2_bits(p[e]);
-      }
-      const float2 ts = __half22float2(__hadd2(__hadd2(gsum[0], gsum[1]), __hadd2(gsum[2], gsum[3])));
-      l += ts.x + ts.y;
-      if (j > 0) {
-        // PV(j-1) must have retired before P is overwritten and O rescaled
-        good = mbar_wait_bounded(B.o[grp], (j - 1) & 1);
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (c * 32 + i >= n_valid) sv[c][i] = 0xff800000u;   // -inf: exp2 gives exactly 0
+        }
+        float mx2[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          mx2[c] = fmaxf(__uint_as_float(sv[c][0]), __uint_as_float(sv[c][1]));
+#pragma unroll
+          for (int i = 2; i < 32; i += 2) mx2[c] = max3_f32(mx2[c], __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
+        }
+        float other;
+        bool good = exchange(fmaxf(mx2[0], mx2[1]), other);
         if (!good) arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_ACC);
         ok = __all_sync(0xffffffffu, good);
         if (!ok) break;
-        tc_fence_after();
+        const float mx = fmaxf(fmaxf(mx2[0], mx2[1]), other) * sc;   // the same value in both threads of the row
+        float alpha = 1.f;
+        if (mx > m_ref + RESCALE_THRESHOLD) {  // also the first visible tile (m_ref = -inf)
+          alpha = (m_ref == -INFINITY) ? 0.f : ex2_fast(m_ref - mx);
+          m_ref = mx;
+        }
+        l *= alpha;
+        const float m_safe = (m_ref == -INFINITY) ? 0.f : m_ref;
+        const uint64_t sc2 = pack_f32x2(sc, sc), nm2 = pack_f32x2(-m_safe, -m_safe);
+        uint32_t pr[4][8];
+        // the 64 probabilities of this half-tile are summed as packed halves in a balanced tree (they are
+        // at most 2^8 each and almost always at most 1, so the tree stays far inside the half range) and
+        // leave half precision once per tile; the running row sum is fp32
+        __half2 gsum[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          __half2 p[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int k = g * 8 + e;                    // this half's keys 2k, 2k + 1 = its P column k
+            float t0, t1;
+            shift2_f32(sv[k >> 4][(2 * k) & 31], sv[k >> 4][((2 * k) & 31) + 1], sc2, nm2, t0, t1);
+            p[e] = ex2_on_fma<POLY>(e) ? ex2_poly_half2(__floats2half2_rn(t0, t1))
+                                       : __floats2half2_rn(ex2_fast(t0), ex2_fast(t1));
+          }
+          gsum[g] = __hadd2(__hadd2(__hadd2(p[0], p[1]), __hadd2(p[2], p[3])),
+                            __hadd2(__hadd2(p[4], p[5]), __hadd2(p[6], p[7])));
+#pragma unroll
+          for (int e = 0; e < 8; ++e) pr[g][e] = h2_bits(p[e]);
+        }
+        const float2 ts = __half22float2(__hadd2(__hadd2(gsum[0], gsum[1]), __hadd2(gsum[2], gsum[3])));
+        l += ts.x + ts.y;
+        if (j > 0) {
+          // PV(j-1) must have retired before P is overwritten and O rescaled
+          good = mbar_wait_bounded(B.o[grp], (done + j - 1) & 1);
+          if (!good) arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_ACC);
+          ok = __all_sync(0xffffffffu, good);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+          // this thread's 32 output dims of the row were accumulated against the old reference maximum
+          uint32_t oreg[32];
+          tmem_ld_32x32(t_o, oreg);
+          tmem_wait_ld_dep(oreg);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
+          tmem_st_32x32(t_o, oreg);
+        }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) tmem_st_32x8(t_p + g * 8, pr[g]);
+        // P (and a rescaled O) are complete in tensor memory before the MMA warp is told
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(B.p[grp]);
       }
-      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-        // this thread's 32 output dims of the row were accumulated against the old reference maximum
-        uint32_t oreg[32];
+      // the row's normaliser is the sum of the two halves' private sums
+      float l_other = 0.f;
+      if (ok && n_mine > 0) {
+        bool good = exchange(l, l_other);
+        good = mbar_wait_bounded(B.o[grp], (done + n_mine - 1) & 1) && good;
+        if (!good) arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_ACC);
+        ok = __all_sync(0xffffffffu, good);
+      }
+      const float l_row = half ? l_other + l : l + l_other;   // same order of addition in both threads
+      const float inv = (ok && l_row > 0.f) ? 1.f / l_row : 0.f;
+      uint16_t* dst = reinterpret_cast<uint16_t*>(a.out16) + ((size_t)max(out_row, 0) * a.n_heads + head) * HD + half * 32;
+      uint32_t oreg[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) oreg[i] = 0u;
+      if (ok && n_mine > 0) {
+        tc_fence_after();
         tmem_ld_32x32(t_o, oreg);
         tmem_wait_ld_dep(oreg);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
-        tmem_st_32x32(t_o, oreg);
       }
+      if (out_row >= 0) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g) tmem_st_32x8(t_p + g * 8, pr[g]);
-      // P (and a rescaled O) are complete in tensor memory before the MMA warp is told
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(B.p[grp]);
-    }
-    // the row's normaliser is the sum of the two halves' private sums
-    float l_other = 0.f;
-    if (ok && n_mine > 0) {
-      bool good = exchange(n_mine & 1, l, l_other);
-      good = mbar_wait_bounded(B.o[grp], (n_mine - 1) & 1) && good;
-      if (!good) arcb_set_error(a.err, ARCB_DEV_WAIT_TIMEOUT_ACC);
-      ok = __all_sync(0xffffffffu, good);
-    }
-    const float l_row = half ? l_other + l : l + l_other;   // same order of addition in both threads
-    const int qr = grp * BQ + r;
-    const float inv = (ok && l_row > 0.f) ? 1.f / l_row : 0.f;
-    uint16_t* dst = reinterpret_cast<uint16_t*>(a.out16) + ((size_t)(row0 + qr) * a.n_heads + h) * HD + half * 32;
-    uint32_t oreg[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) oreg[i] = 0u;
-    if (ok && n_mine > 0) {
-      tc_fence_after();
-      tmem_ld_32x32(t_o, oreg);
-      tmem_wait_ld_dep(oreg);
-    }
-    if (qr < rows) {
-#pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-        uint4 v;
-        v.x = pack2_act(__uint_as_float(oreg[i]) * inv, __uint_as_float(oreg[i + 1]) * inv, 1);
-        v.y = pack2_act(__uint_as_float(oreg[i + 2]) * inv, __uint_as_float(oreg[i + 3]) * inv, 1);
-        v.z = pack2_act(__uint_as_float(oreg[i + 4]) * inv, __uint_as_float(oreg[i + 5]) * inv, 1);
-        v.w = pack2_act(__uint_as_float(oreg[i + 6]) * inv, __uint_as_float(oreg[i + 7]) * inv, 1);
-        *reinterpret_cast<uint4*>(dst + i) = v;
+        for (int i = 0; i < 32; i += 8) {
+          uint4 v;
+          v.x = pack2_act(__uint_as_float(oreg[i]) * inv, __uint_as_float(oreg[i + 1]) * inv, 1);
+          v.y = pack2_act(__uint_as_float(oreg[i + 2]) * inv, __uint_as_float(oreg[i + 3]) * inv, 1);
+          v.z = pack2_act(__uint_as_float(oreg[i + 4]) * inv, __uint_as_float(oreg[i + 5]) * inv, 1);
+          v.w = pack2_act(__uint_as_float(oreg[i + 6]) * inv, __uint_as_float(oreg[i + 7]) * inv, 1);
+          *reinterpret_cast<uint4*>(dst + i) = v;
+        }
       }
+      done += n_mine;
     }
   }
   tc_fence_before();
@@ -815,7 +975,7 @@ int flash_split() {
 
 template <int POLY>
 cudaError_t set_split_smem_attr() {
-  return cudaFuncSetAttribute(attn_prefill_split_kernel<POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+  return cudaFuncSetAttribute(attn_prefill_split_kernel<POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM_BYTES);
 }
 
 template <int SOFTMAX, int POLY>
@@ -843,7 +1003,7 @@ int arcb_attn_prefill_init() {
 
 int arcb_launch_attn_prefill(const AttnPrefillArgs& a, cudaStream_t stream) {
   if (a.n_qblocks <= 0) return 0;
-  if (a.n_kv_rows <= 0 || a.n_rows <= 0) return -1;
+  if (a.n_kv_rows <= 0 || a.n_rows <= 0 || !a.next) return -1;
   const uint64_t d = (uint64_t)a.n_heads * HD;
   CUtensorMap tq, tk, tv;
   int r = arcb_make_tmap_2d_16b(&tq, a.q16, (uint64_t)a.n_rows, d, BQ, HD, a.act_f16);
@@ -856,11 +1016,14 @@ int arcb_launch_attn_prefill(const AttnPrefillArgs& a, cudaStream_t stream) {
   const uint32_t idesc_qk = umma_idesc_f16(BQ, BKV, fmt, fmt, 0, 0);
   const uint32_t idesc_pv = umma_idesc_f16(BQ, HD, fmt, fmt, 0, 1);  // B = V is MN-major
   dim3 grid(a.n_qblocks, a.n_heads);
+  const long long items = (long long)a.n_qblocks * a.n_heads;
+  if (items > 0x7fffffffLL) return -1;
+  const unsigned ctas = (unsigned)(items < arcb_num_sms() ? items : arcb_num_sms());
   cudaError_t le = cudaSuccess;
 #define ARCB_LAUNCH_FLASH(SM, PL) \
   le = arcb_launch(attn_prefill_kernel<SM, PL>, grid, dim3(N_THREADS), SMEM_BYTES, stream, tq, tk, tv, a, idesc_qk, idesc_pv)
 #define ARCB_LAUNCH_SPLIT(PL) \
-  le = arcb_launch(attn_prefill_split_kernel<PL>, grid, dim3(SPLIT_THREADS), SMEM_BYTES, stream, tq, tk, tv, a, idesc_qk, idesc_pv)
+  le = arcb_launch(attn_prefill_split_kernel<PL>, dim3(ctas), dim3(SPLIT_THREADS), SPLIT_SMEM_BYTES, stream, tq, tk, tv, a, idesc_qk, idesc_pv)
   if (!a.act_f16) {
     ARCB_LAUNCH_FLASH(0, 0);
   } else if (flash_split()) {

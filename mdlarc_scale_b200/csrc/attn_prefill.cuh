@@ -15,6 +15,7 @@ struct AttnPrefillArgs {
   int n_qblocks, n_rows, n_kv_rows, n_heads;
   int act_f16;
   int* err;
+  int* next;                // item counter of the persistent kernel: 0, and 0 again when the launch is done; one launch at a time
 };
 
 bool arcb_attn_prefill_available();

@@ -403,7 +403,7 @@ static int run_layer(arcb_session* s, int l, int rows, const int* pos, const int
     fa.seq = seq; fa.kv_count = kv_count; fa.qblock_row0 = pa->d_qblock_row0; fa.qblock_rows = pa->d_qblock_rows;
     fa.qblock_kv0 = pa->d_qblock_kv0;
     fa.n_qblocks = pa->n_qblocks; fa.n_rows = rows; fa.n_kv_rows = pa->n_kv_rows; fa.n_heads = c.n_heads;
-    fa.act_f16 = f16; fa.err = e->d_err;
+    fa.act_f16 = f16; fa.err = e->d_err; fa.next = s->st.n_finished + 1;
     CKL(arcb_launch_attn_prefill(fa, stream), "prefill attention");
   } else {
     AttnStreamArgs aa{};
@@ -462,6 +462,7 @@ extern "C" int arcb_prefill(arcb_session* s, const arcb_prefill_args* a, void* s
     CK(cudaMemsetAsync(s->state_ints, 0, s->n_state_ints * 4, stream));
     s->state_cleared = true;
   }
+  CK(cudaMemsetAsync(s->st.n_finished + 1, 0, 4, stream));   // the prefill attention's item counter, should a launch have failed
   const bool use_ex = c.use_example_embedding && a->d_example_ids;
   if (a->n_first > 0) {
     if (s->graph_exec && s->use_examples != use_ex) {  // the recorded step baked the other choice in

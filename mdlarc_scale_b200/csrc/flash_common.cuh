@@ -38,6 +38,7 @@ __device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cas
 __device__ __forceinline__ __half2 h2_from_bits(uint32_t b) { return *reinterpret_cast<__half2*>(&b); }
 
 // Re-division of the CTA's registers between warpgroups (all four warps of a warpgroup execute it)
+__device__ __forceinline__ void reg_dealloc_32() { asm volatile("setmaxnreg.dec.sync.aligned.u32 32;"); }
 __device__ __forceinline__ void reg_dealloc_24() { asm volatile("setmaxnreg.dec.sync.aligned.u32 24;"); }
 __device__ __forceinline__ void reg_alloc_112() { asm volatile("setmaxnreg.inc.sync.aligned.u32 112;"); }
 

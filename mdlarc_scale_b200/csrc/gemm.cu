@@ -1572,6 +1572,7 @@ static cudaError_t launch_tc2(const CUtensorMap& ta, const CUtensorMap& tb, cons
 }
 
 int arcb_gemm_max_pairs() { return max_pairs(); }
+int arcb_num_sms() { return num_sms(); }
 
 // Column tile of the split-K residual kernel for an M x N x K launch, or 0 when it does not apply:
 // the launch must leave most SMs without a 128 x 128 tile, K must be long enough to be worth
