@@ -1498,8 +1498,6 @@ static cudaError_t set_tc2_smem_attr() {
 // any stream capture).
 int arcb_gemm_init() {
   cudaError_t e;
-  if (const int r = arcb_gemm_rows_init()) return r;
-  if (const int r = arcb_gemm_mid_init()) return r;
   if ((e = set_tc_smem_attr<EPI_STORE_F32>()) != cudaSuccess) return (int)e;
   if ((e = set_tc_smem_attr<EPI_QKV_ROPE>()) != cudaSuccess) return (int)e;
   if ((e = set_tc_smem_attr<EPI_RESID>()) != cudaSuccess) return (int)e;

@@ -12,6 +12,9 @@
 // 2048 x 8192 38.7 / 14.6, 8320 x 2048 15.0 / 14.2, 32000 x 2048 53 / 34.
 #include <cuda.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "common.cuh"
 #include "gemm.cuh"
 #include "gemm_mid.cuh"
@@ -224,9 +227,51 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   }
 }
 
-// clusters of 2 to 8 CTAs, one CTA an SM, that run at once on each device
 constexpr int GM_DEVICES = 64;
-int g_clusters[GM_DEVICES][GM_SPLIT_MAX + 1];
+
+int current_device() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < GM_DEVICES ? dev : 0;
+}
+
+// Shared-memory opt-in of a kernel at its first launch on a device: doing it for all forms when an engine is created loads
+// kernels that most programs never use (0.3 ms each).
+template <typename K>
+cudaError_t opt_in(K kernel, std::atomic<unsigned long long>& done) {
+  const unsigned long long bit = 1ull << current_device();
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_MAX);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
+// clusters of `splits` CTAs, one CTA an SM, that run at once on this device
+int clusters_at_once(int splits) {
+  static std::mutex mu;
+  static int known[GM_DEVICES][GM_SPLIT_MAX + 1];                    // count + 1, 0: not asked yet
+  static std::atomic<unsigned long long> opted{0};
+  std::lock_guard<std::mutex> lock(mu);
+  int& slot = known[current_device()][splits];
+  if (slot) return slot - 1;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = splits;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(splits * 148);
+  cfg.blockDim = dim3(GM_THREADS);
+  cfg.dynamicSmemBytes = GM_SMEM_MAX;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (opt_in(gemm_mid_kernel<EPI_RESID, 8>, opted) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, gemm_mid_kernel<EPI_RESID, 8>, &cfg) != cudaSuccess) {
+    n = 0;
+    cudaGetLastError();
+  }
+  slot = n + 1;
+  return n;
+}
 
 // The split with the shortest time: a launch's and a tile's fixed cost (about 4 us a wave), operands at one SM's 110 KB a us,
 // and 2 us for the exchange, as long as all clusters run at once.  Tiles beyond one wave run two CTAs an SM where shared
@@ -234,14 +279,12 @@ int g_clusters[GM_DEVICES][GM_SPLIT_MAX + 1];
 GmShape gm_shape(int M, int N, int K) {
   GmShape best{};
   best.rows = (M + 15) / 16 * 16;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= GM_DEVICES) dev = 0;
   const int tiles = N / 128, num_k = K / 64, stage = GM_W_BYTES + best.rows * 128;
   const bool two = tiles > 148 && 2 * stage + 2048 <= GM_SMEM_HALF && best.rows * 512 + 2048 <= GM_SMEM_HALF;
   best.splits = 1;
   double best_time = 0.;
   for (int s = 1; s <= GM_SPLIT_MAX && s <= num_k; ++s) {
-    if (s > 1 && tiles > g_clusters[dev][s]) continue;
+    if (s > 1 && (tiles * s > 148 || tiles > clusters_at_once(s))) continue;
     const int waves = s > 1 ? 1 : two ? (tiles + 295) / 296 : (tiles + 147) / 148;
     const double time = waves * (4. + (num_k + s - 1) / s * (stage / 110e3) * (two ? 2 : 1)) + (s > 1 ? 2. : 0.);
     if (s == 1 || time < best_time) { best.splits = s; best_time = time; }
@@ -259,47 +302,20 @@ int launch(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_
   if (!r) r = arcb_make_tmap_2d_16b(&ta, a, (uint64_t)ep.M, (uint64_t)(ep.grp.lda ? ep.grp.lda : K), sh.rows, 64, act_f16);
   if (r) return 1000 + r;
   const uint32_t idesc = umma_idesc_f16(128, sh.rows, act_f16 ? 0 : 1, act_f16 ? 0 : 1);
-  auto kernel = sh.splits == 1 ? gemm_mid_kernel<MODE, 1> : sh.splits <= 4 ? gemm_mid_kernel<MODE, 4> : gemm_mid_kernel<MODE, 8>;
-  const cudaError_t e = arcb_launch_cluster(kernel, sh.splits, dim3(ep.N / 128 * sh.splits), dim3(GM_THREADS), sh.smem(), stream, tw, ta, ep,
-                                            K / 64, idesc, sh);
+  static std::atomic<unsigned long long> opted[3];
+  auto run = [&](auto kernel, std::atomic<unsigned long long>& done) {
+    const cudaError_t e = opt_in(kernel, done);
+    return e != cudaSuccess ? e : arcb_launch_cluster(kernel, sh.splits, dim3(ep.N / 128 * sh.splits), dim3(GM_THREADS), sh.smem(), stream, tw, ta, ep,
+                                                      K / 64, idesc, sh);
+  };
+  const cudaError_t e = sh.splits == 1   ? run(gemm_mid_kernel<MODE, 1>, opted[0])
+                        : sh.splits <= 4 ? run(gemm_mid_kernel<MODE, 4>, opted[1])
+                                         : run(gemm_mid_kernel<MODE, 8>, opted[2]);
   arcb_count_launch(1);
   return (int)e;
 }
 
-template <int MODE>
-cudaError_t opt_in() {
-  cudaError_t e = cudaFuncSetAttribute(gemm_mid_kernel<MODE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_MAX);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_mid_kernel<MODE, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_MAX);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_mid_kernel<MODE, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_MAX);
-  return e;
-}
-
 }  // namespace
-
-int arcb_gemm_mid_init() {
-  const cudaError_t all[] = {opt_in<EPI_STORE_F32>(), opt_in<EPI_QKV_ROPE>(), opt_in<EPI_RESID>(), opt_in<EPI_SWIGLU>(), opt_in<EPI_RELU2>(),
-                             opt_in<EPI_HEADS>(), opt_in<EPI_ACT>(), opt_in<EPI_GLU>()};
-  for (const cudaError_t e : all)
-    if (e != cudaSuccess) return (int)e;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= GM_DEVICES) return 0;
-  for (int s = 2; s <= GM_SPLIT_MAX; ++s) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = s;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(s * 148);
-    cfg.blockDim = dim3(GM_THREADS);
-    cfg.dynamicSmemBytes = GM_SMEM_MAX;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_mid_kernel<EPI_RESID, 8>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
-    g_clusters[dev][s] = n;
-  }
-  return 0;
-}
 
 // Decode steps only: how a sum is divided depends on the number of rows, and a prompt row's result does not depend on what
 // else its call holds.

@@ -4,4 +4,3 @@
 
 bool arcb_gemm_mid_applies(const void* a16, const void* w16, const GemmEpilogue& ep, int K, int act_f16);
 int arcb_launch_gemm_mid(const void* a16, const void* w16, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream);
-int arcb_gemm_mid_init();   // shared-memory opt-in, once per device and outside any capture

@@ -14,6 +14,8 @@
 // B200, us a launch inside the captured step, tcgen05 tiles / here: 16 rows, QKV of width 1024 10.3 / 4.6, gate/up 10.6 / 5.4,
 // out and down 10.7 / 3.9; 1 row of width 256 6.1 to 6.8 / 1.9 to 2.4; 1 row, mixer projection of width 1280 14.2 / 6.5.
 // Prompt portions of up to 64 rows, and steps that gemm_mid.cu does not take.
+#include <atomic>
+
 #include "common.cuh"
 #include "gemm.cuh"
 #include "gemm_rows.cuh"
@@ -252,11 +254,28 @@ gemm_rows_heads_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, in
   rows_product<1, MT, EPI_HEADS, F16>(A, W, ep, K, red);
 }
 
+// Shared-memory opt-in of a form that needs more than the default 48 KB, at its first launch on a device: doing it for all
+// forms when an engine is created loads kernels that most programs never use.
+template <typename K>
+cudaError_t opt_in(K kernel, int bytes, std::atomic<unsigned long long>& done) {
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  const unsigned long long bit = 1ull << dev;
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
 template <int NT, int MT, int MODE>
 cudaError_t launch(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {
   using Cfg = GrCfg<NT, MT>;
   const dim3 grid(ep.N / (16 * NT), (ep.M + Cfg::ROWS - 1) / Cfg::ROWS);
   auto kernel = act_f16 ? gemm_rows_kernel<NT, MT, MODE, true> : gemm_rows_kernel<NT, MT, MODE, false>;
+  static std::atomic<unsigned long long> opted[2];
+  const cudaError_t e = opt_in(kernel, Cfg::SMEM, opted[act_f16 ? 1 : 0]);
+  if (e != cudaSuccess) return e;
   return arcb_launch(kernel, grid, dim3(GR_THREADS), Cfg::SMEM, stream, reinterpret_cast<const uint16_t*>(a),
                      reinterpret_cast<const uint16_t*>(w), ep, K);
 }
@@ -264,8 +283,11 @@ cudaError_t launch(const void* a, const void* w, const GemmEpilogue& ep, int K, 
 template <int MT>
 cudaError_t launch_heads(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {
   using Cfg = GrCfg<1, MT>;
-  return arcb_launch(act_f16 ? gemm_rows_heads_kernel<MT, true> : gemm_rows_heads_kernel<MT, false>,
-                     dim3(ep.N / 16, (ep.M + Cfg::ROWS - 1) / Cfg::ROWS), dim3(GR_THREADS), Cfg::SMEM, stream,
+  auto kernel = act_f16 ? gemm_rows_heads_kernel<MT, true> : gemm_rows_heads_kernel<MT, false>;
+  static std::atomic<unsigned long long> opted[2];
+  const cudaError_t e = opt_in(kernel, Cfg::SMEM, opted[act_f16 ? 1 : 0]);
+  if (e != cudaSuccess) return e;
+  return arcb_launch(kernel, dim3(ep.N / 16, (ep.M + Cfg::ROWS - 1) / Cfg::ROWS), dim3(GR_THREADS), Cfg::SMEM, stream,
                      reinterpret_cast<const uint16_t*>(a), reinterpret_cast<const uint16_t*>(w), ep, K);
 }
 
@@ -278,40 +300,7 @@ cudaError_t launch_mode(const void* a, const void* w, const GemmEpilogue& ep, in
   return launch<2, 8, MODE>(a, w, ep, K, act_f16, stream);
 }
 
-// forms that need more than the default 48 KB of shared memory
-template <typename K>
-cudaError_t opt_in(K kernel, int bytes) {
-  return bytes > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
-}
-template <int MODE>
-cudaError_t init_mode() {
-  cudaError_t e = opt_in(gemm_rows_kernel<2, 8, MODE, true>, GrCfg<2, 8>::SMEM);
-  if (e == cudaSuccess) e = opt_in(gemm_rows_kernel<2, 8, MODE, false>, GrCfg<2, 8>::SMEM);
-  if (e == cudaSuccess) e = opt_in(gemm_rows_kernel<2, 4, MODE, true>, GrCfg<2, 4>::SMEM);
-  if (e == cudaSuccess) e = opt_in(gemm_rows_kernel<2, 4, MODE, false>, GrCfg<2, 4>::SMEM);
-  return e;
-}
-cudaError_t init_heads() {
-  cudaError_t e = opt_in(gemm_rows_heads_kernel<8, true>, GrCfg<1, 8>::SMEM);
-  if (e == cudaSuccess) e = opt_in(gemm_rows_heads_kernel<8, false>, GrCfg<1, 8>::SMEM);
-  if (e == cudaSuccess) e = opt_in(gemm_rows_heads_kernel<4, true>, GrCfg<1, 4>::SMEM);
-  if (e == cudaSuccess) e = opt_in(gemm_rows_heads_kernel<4, false>, GrCfg<1, 4>::SMEM);
-  return e;
-}
-
 }  // namespace
-
-int arcb_gemm_rows_init() {
-  cudaError_t e;
-  if ((e = init_mode<EPI_STORE_F32>()) != cudaSuccess) return (int)e;
-  if ((e = init_mode<EPI_QKV_ROPE>()) != cudaSuccess) return (int)e;
-  if ((e = init_mode<EPI_RESID>()) != cudaSuccess) return (int)e;
-  if ((e = init_mode<EPI_SWIGLU>()) != cudaSuccess) return (int)e;
-  if ((e = init_mode<EPI_RELU2>()) != cudaSuccess) return (int)e;
-  if ((e = init_mode<EPI_ACT>()) != cudaSuccess) return (int)e;
-  if ((e = init_mode<EPI_GLU>()) != cudaSuccess) return (int)e;
-  return (int)init_heads();
-}
 
 // Up to 64 rows: the weights' 16-row fragments meet eight 8-row activation fragments, and the activations of a CTA
 // (64 rows x K) are re-read from L2 by every CTA (48 rows of width 1280, tcgen05 tiles / here: outputs 10.9 / 9.0, gated units
