@@ -211,8 +211,8 @@ __device__ __forceinline__ void rows_product(const uint16_t* A, const uint16_t* 
     return v;
   };
   if constexpr (MODE == EPI_HEADS) {
-    static_assert(NT == 1 && Cfg::ROWS * 4 <= GR_THREADS, "one quad a thread");
-    const int row = threadIdx.x >> 2, q = threadIdx.x & 3;
+    static_assert(Cfg::ROWS * QUADS <= GR_THREADS, "one quad a thread");
+    const int row = threadIdx.x / QUADS, q = threadIdx.x % QUADS;    // norms need NT = 1: quads of a row in neighbouring lanes of four
     const bool in = row < Cfg::ROWS && m0 + row < ep.M;
     epi_heads_quad(ep, in ? m0 + row : -1, n0 + q * 4, in ? total(row, q * 4) : make_float4(0.f, 0.f, 0.f, 0.f),
                    [&](float ss, bool wanted, int width, int in_head) { return cluster_head_sum<Cfg::ROWS>(ss, row, q, wanted, width, in_head); });
@@ -280,6 +280,11 @@ cudaError_t launch(const void* a, const void* w, const GemmEpilogue& ep, int K, 
                      reinterpret_cast<const uint16_t*>(w), ep, K);
 }
 
+// Up to 16 rows: 32 columns a CTA once 16 make more CTAs than run at once (two an SM), for 9 rows and more some earlier, where
+// re-reading the activations counts.  us a launch, 16 / 32 columns: 1 row, 4608 x 1280 4.2 / 4.6, 5120 x 1280 5.7 / 5.0, 8192 x 2048
+// 9.0 / 7.7; 16 rows, 1280 x 1280 3.5 / 4.2, 3200 x 1280 4.8 / 4.6, 5120 x 1280 7.2 / 5.8.
+bool wide_columns(const GemmEpilogue& ep) { return ep.M <= 16 && ep.N / 16 > (ep.M <= 8 ? 296 : 192); }
+
 template <int MT>
 cudaError_t launch_heads(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {
   using Cfg = GrCfg<1, MT>;
@@ -294,6 +299,7 @@ cudaError_t launch_heads(const void* a, const void* w, const GemmEpilogue& ep, i
 template <int MODE>
 cudaError_t launch_mode(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {
   constexpr int N1 = gr_paired<MODE>() ? 2 : 1;
+  if (N1 == 1 && wide_columns(ep)) return ep.M <= 8 ? launch<2, 1, MODE>(a, w, ep, K, act_f16, stream) : launch<2, 2, MODE>(a, w, ep, K, act_f16, stream);
   if (ep.M <= 8) return launch<N1, 1, MODE>(a, w, ep, K, act_f16, stream);
   if (ep.M <= 16) return launch<N1, 2, MODE>(a, w, ep, K, act_f16, stream);
   if (ep.M <= 32) return launch<2, 4, MODE>(a, w, ep, K, act_f16, stream);
@@ -327,6 +333,10 @@ int arcb_launch_gemm_rows(const void* a, const void* w, const GemmEpilogue& ep, 
     case EPI_ACT: e = launch_mode<EPI_ACT>(a, w, ep, K, act_f16, stream); break;
     case EPI_GLU: e = launch_mode<EPI_GLU>(a, w, ep, K, act_f16, stream); break;
     case EPI_HEADS:
+      if (!ep.pj.q_norm && !ep.pj.k_norm && wide_columns(ep)) {
+        e = ep.M <= 8 ? launch<2, 1, EPI_HEADS>(a, w, ep, K, act_f16, stream) : launch<2, 2, EPI_HEADS>(a, w, ep, K, act_f16, stream);
+        break;
+      }
       e = ep.M <= 8    ? launch_heads<1>(a, w, ep, K, act_f16, stream)
           : ep.M <= 16 ? launch_heads<2>(a, w, ep, K, act_f16, stream)
           : ep.M <= 32 ? launch_heads<4>(a, w, ep, K, act_f16, stream)

@@ -93,7 +93,7 @@ def test_splits_merged_in_a_cluster(lib, splits, T):
 
 @pytest.mark.parametrize("fmt", [_lib.ACT_F16, _lib.ACT_BF16])
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64, 65])
-@pytest.mark.parametrize("N,K", [(128, 64), (384, 256), (1280, 704), (1024, 3392)])
+@pytest.mark.parametrize("N,K", [(128, 64), (384, 256), (1280, 704), (1024, 3392), (3072, 256), (3200, 704), (4736, 96), (4864, 704)])
 def test_few_row_products(lib, M, N, K, fmt):
     """Row tiles of 8, 16, 32 and 64 and one row beyond; K of fewer blocks than warps, and of more than are in flight."""
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
@@ -145,7 +145,17 @@ def test_mid_row_products(lib, M, N, K, fmt):
 def test_mid_row_steps(name, slots, fmt):
     """A decode step of that many sequences: heads of 64 and 128 columns with and without norms, gates, caches, vocabularies."""
     from vodavik_util import CONFIGS
-    cfg = CONFIGS[name]
+    steps_match(CONFIGS[name], slots, fmt)
+
+
+@pytest.mark.parametrize("fmt", ["f16", "bf16"])
+@pytest.mark.parametrize("slots", [1, 8, 9, 16, 17])
+def test_steps_with_wide_projections(slots, fmt):
+    """Recurrent projections (no norms) of more 16-column tiles than CTAs run at once, beside attention's normed ones."""
+    steps_match(config(128, 77, [mlstm(20, 64, 64), attention(30, 5, 64, 64, ff=4800)]), slots, fmt)
+
+
+def steps_match(cfg, slots, fmt):
     w = vo.random_weights(cfg, 5)
     eng = registry.build_engine(cfg, w, "cuda:0", fmt)
     s = eng.new_session(slots, 16, 1, 8 * slots, stop_on_end=False)
