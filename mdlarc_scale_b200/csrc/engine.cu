@@ -430,7 +430,7 @@ static int run_layer(arcb_session* s, int l, int rows, const int* pos, const int
   er.splitk_scratch = prefill ? nullptr : s->gemm_scratch;   // sized for the decode step's rows only
   CKL(arcb_launch_gemm(s->attn16, L.w_out, er, d, f16, use_tc_for(e, rows, d, d), stream), "out_proj gemm");
   plain_edges.off();
-  CKL(arcb_launch_rmsnorm(s->x, L.ln2_w, s->xn16, rows, d, c.norm_eps, f16, stream), "ln2");
+  CKL(arcb_launch_rmsnorm(s->x, L.ln2_w, s->xn16, rows, d, c.norm_eps, f16, !prefill, stream), "ln2");
   // gate | up + SwiGLU
   GemmEpilogue eg{};
   eg.mode = EPI_SWIGLU; eg.M = rows; eg.N = 2 * dff; eg.bias = L.b_gu; eg.out16 = s->h16; eg.act_f16 = f16; eg.err = e->d_err; eg.step = !prefill;
@@ -439,7 +439,7 @@ static int run_layer(arcb_session* s, int l, int rows, const int* pos, const int
   er.bias = L.b_down;
   CKL(arcb_launch_gemm(s->h16, L.w_down, er, dff, f16, use_tc_for(e, rows, d, dff), stream), "down gemm");
   if (l + 1 < c.n_layers)
-    CKL(arcb_launch_rmsnorm(s->x, e->layers[l + 1].ln1_w, s->xn16, rows, d, c.norm_eps, f16, stream), "ln1");
+    CKL(arcb_launch_rmsnorm(s->x, e->layers[l + 1].ln1_w, s->xn16, rows, d, c.norm_eps, f16, !prefill, stream), "ln1");
   return ARCB_OK;
 }
 
@@ -517,7 +517,7 @@ static int record_decode_step(arcb_session* s, cudaStream_t stream) {
     if (r) return r;
   }
   HeadArgs ha{};
-  ha.mode = HEAD_DECODE; ha.rows = B; ha.d = c.d_model; ha.eps = c.norm_eps; ha.x = s->x;
+  ha.mode = HEAD_DECODE; ha.step = 1; ha.rows = B; ha.d = c.d_model; ha.eps = c.norm_eps; ha.x = s->x;
   ha.lnf_w = e->lnf_w; ha.lm_head = e->lm_head;
   CKL(arcb_launch_head(ha, s->st, stream), "head(decode)");
   return ARCB_OK;
@@ -605,7 +605,7 @@ extern "C" int arcb_session_attention_probe(arcb_session* s, float* ms) {
 extern "C" int arcb_op_rmsnorm(const float* x, const float* w, void* out16, int32_t rows, int32_t d,
                                float eps, int32_t act_format, void* stream) {
   if (!x || !w || !out16 || d % 4) return arcb_fail(ARCB_E_ARG, "bad rmsnorm arguments");
-  CKL(arcb_launch_rmsnorm(x, w, out16, rows, d, eps, act_format == ARCB_ACT_F16, (cudaStream_t)stream), "rmsnorm");
+  CKL(arcb_launch_rmsnorm(x, w, out16, rows, d, eps, act_format == ARCB_ACT_F16, true, (cudaStream_t)stream), "rmsnorm");
   return ARCB_OK;
 }
 
@@ -707,7 +707,7 @@ extern "C" int arcb_op_head(const float* x, const int32_t* row_index, const floa
                             float* logits, int32_t* argmax, int32_t rows, int32_t d, float eps, void* stream) {
   if (!x || !lnf_w || !lm_head || d % 4) return arcb_fail(ARCB_E_ARG, "bad head arguments");
   HeadArgs ha{};
-  ha.mode = HEAD_PLAIN; ha.rows = rows; ha.d = d; ha.eps = eps; ha.x = x; ha.row_index = row_index;
+  ha.mode = HEAD_PLAIN; ha.step = 1; ha.rows = rows; ha.d = d; ha.eps = eps; ha.x = x; ha.row_index = row_index;
   ha.lnf_w = lnf_w; ha.lm_head = lm_head; ha.logits = logits; ha.argmax = argmax;
   DecodeState st{};
   CKL(arcb_launch_head(ha, st, (cudaStream_t)stream), "head");

@@ -774,10 +774,10 @@ int lm_residual(arcb_session* s, const void* a, const void* w, int K, int rows, 
   return ARCB_OK;
 }
 
-int lm_norm(arcb_session* s, const float* w, int rows, float x_scale, float* dense, cudaStream_t stream) {
+int lm_norm(arcb_session* s, const float* w, const Rows& R, float x_scale, float* dense, cudaStream_t stream) {
   const LayeredModel& m = *s->eng->lm;
   LmNormArgs a{};
-  a.kind = m.d.norm; a.rows = rows; a.width = m.d.width; a.pitch = m.wp; a.fmt = m.fmt; a.eps = m.d.norm_eps;
+  a.kind = m.d.norm; a.rows = R.n; a.width = m.d.width; a.pitch = m.wp; a.fmt = m.fmt; a.eps = m.d.norm_eps; a.step = R.pa == nullptr;
   a.x_scale = x_scale; a.x = s->ls->x; a.w = w; a.xn = s->ls->xn; a.write_x = 1; a.dense = dense;
   CKL(arcb_launch_lm_norm(a, stream), "norm");
   return ARCB_OK;
@@ -828,7 +828,7 @@ int lm_latent(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
       const int n = R.n - r0 < ls->lat_rows ? R.n - r0 : ls->lat_rows;
       const void* qr = q + (size_t)r0 * L.n_proj * m.es;
       GemmEpilogue el{};
-      el.mode = EPI_ACT; el.M = n; el.N = L.hp * L.kvp; el.out16 = ls->qlat; el.act_f16 = m.fmt; el.err = s->eng->d_err;
+      el.mode = EPI_ACT; el.M = n; el.N = L.hp * L.kvp; el.out16 = ls->qlat; el.act_f16 = m.fmt; el.err = s->eng->d_err; el.step = R.pa == nullptr;
       el.grp.n_group = L.kvp; el.grp.a_group = qh; el.grp.lda = L.n_proj;
       CKL(lm_gemm(m, qr, L.w_ukt, el, L.dimp, stream), "latent query gemm");
       AttnLatentArgs a{};
@@ -842,7 +842,7 @@ int lm_latent(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
       else
         CKL(arcb_launch_attn_latent_stream(a, stream), "latent attention");
       GemmEpilogue ev{};
-      ev.mode = EPI_ACT; ev.M = n; ev.N = L.k_out; ev.act_f16 = m.fmt; ev.err = s->eng->d_err;
+      ev.mode = EPI_ACT; ev.M = n; ev.N = L.k_out; ev.act_f16 = m.fmt; ev.err = s->eng->d_err; ev.step = R.pa == nullptr;
       ev.out16 = reinterpret_cast<uint8_t*>(ls->mix) + (size_t)r0 * L.k_out * m.es;
       ev.grp.n_group = L.vdimp; ev.grp.a_group = L.kvp; ev.grp.lda = L.hp * L.kvp;
       CKL(lm_gemm(m, ls->olat, reinterpret_cast<const uint8_t*>(L.w_ukv) + (size_t)L.hp * L.dimp * L.kvp * m.es, ev, L.kvp, stream), "value gemm");
@@ -991,7 +991,7 @@ int lm_layers_sandwich(arcb_session* s, const Rows& R, float* residuals, cudaStr
   const int n_runs = (int)m.runs.size();
   LmNormArgs first{};
   first.kind = m.d.norm; first.rows = R.n; first.width = m.d.width; first.pitch = m.wp; first.fmt = m.fmt; first.eps = m.d.norm_eps;
-  first.x_scale = 1.f; first.x = ls->x; first.w = m.layers[m.runs[0].layer].norm1; first.xn = ls->xn;
+  first.x_scale = 1.f; first.x = ls->x; first.w = m.layers[m.runs[0].layer].norm1; first.xn = ls->xn; first.step = R.pa == nullptr;
   CKL(arcb_launch_lm_norm(first, stream), "norm");
   for (int l = 0; l < n_runs; ++l) {
     const LmLayer& L = m.layers[m.runs[l].layer];
@@ -1035,11 +1035,11 @@ int lm_layers(arcb_session* s, const Rows& R, float* residuals, cudaStream_t str
     int r = lm_mixer(s, l, R, stream);
     if (r) return r;
     // the norm leaves x already multiplied by the factor of the next sublayer's sum
-    r = lm_norm(s, L.norm1, R.n, last && !L.ffp ? 1.f : m.d.residual_alpha, L.ffp ? nullptr : dense, stream);
+    r = lm_norm(s, L.norm1, R, last && !L.ffp ? 1.f : m.d.residual_alpha, L.ffp ? nullptr : dense, stream);
     if (r) return r;
     if (L.ffp) {
       r = lm_mlp(s, l, R, stream);
-      if (!r) r = lm_norm(s, L.norm2, R.n, last ? 1.f : m.d.residual_alpha, dense, stream);
+      if (!r) r = lm_norm(s, L.norm2, R, last ? 1.f : m.d.residual_alpha, dense, stream);
       if (r) return r;
     }
   }
@@ -1056,6 +1056,7 @@ int lm_head(arcb_session* s, int mode, int rows, const int* index, float* out, c
     LmNormArgs a{};
     a.kind = m.d.norm; a.rows = n; a.width = m.d.width; a.pitch = m.wp; a.fmt = m.fmt; a.eps = m.d.norm_eps;
     a.x_scale = 1.f; a.x = ls->x; a.w = m.final_norm; a.xn = ls->hn; a.write_x = 0; a.row_index = index ? index + r0 : nullptr;
+    a.step = mode == PICK_DECODE;
     CKL(arcb_launch_lm_norm(a, stream), "final norm");
     GemmEpilogue ep{};
     ep.mode = EPI_STORE_F32; ep.M = n; ep.N = m.vp; ep.y = ls->logits; ep.act_f16 = m.fmt; ep.err = s->eng->d_err; ep.step = mode == PICK_DECODE;

@@ -14,10 +14,11 @@ namespace {
 
 constexpr int ROWS_PER_CTA = 4;
 
-// Launches of at most this many rows give a row a CTA instead of a warp: with fewer rows than the machine has warps a
+// Steps of at most this many rows give a row a CTA instead of a warp: with fewer rows than the machine has warps a
 // row's time is one warp's chain of loads, sums and stores.  B200, centred norm of 1 row of 1280 columns, us
 // per launch inside the captured step, warp / CTA per row: 7.2 / 2.2.  Many rows are bound by bytes, and the warp form reads
-// them at the HBM rate.
+// them at the HBM rate.  A prompt's rows always have a warp each: the two forms add in different orders, and a prompt's results
+// do not depend on what else its call holds.
 constexpr int CTA_ROW_MAX = 2048;
 constexpr int CTA_THREADS = 128;
 
@@ -789,7 +790,7 @@ int arcb_launch_lm_norm(const LmNormArgs& a, cudaStream_t stream) {
   if (a.pitch % 128) return -1;
   auto cta = [&](auto kernel) { return arcb_launch(kernel, dim3(a.rows), dim3(CTA_THREADS), 0, stream, a); };
   const int steps = (a.pitch + CTA_THREADS * 4 - 1) / (CTA_THREADS * 4);
-  const cudaError_t e = a.rows > CTA_ROW_MAX || steps > 8
+  const cudaError_t e = !a.step || a.rows > CTA_ROW_MAX || steps > 8
                             ? arcb_launch(lm_norm_kernel, dim3((a.rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), dim3(ROWS_PER_CTA * 32), 0, stream, a)
                         : steps <= 1 ? cta(lm_norm_cta_kernel<1>)
                         : steps <= 2 ? cta(lm_norm_cta_kernel<2>)

@@ -46,6 +46,7 @@ struct LmNormArgs {
   int write_x;
   const int* row_index;    // optional gather of rows of x (write_x 0)
   float* dense;            // optional [rows][width]: y, without padding
+  int step;                // rows of a step: the order of a row's sums may depend on their number
 };
 
 // Sandwich norms, one sublayer to the next: x += norm(y) * w_out, then xn = norm(x) * w_in in the activation format.

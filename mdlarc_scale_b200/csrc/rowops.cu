@@ -11,11 +11,12 @@ namespace {
 
 constexpr int ROWS_PER_CTA = 4;
 
-// One CTA per row instead of one warp: launches of at most this many rows leave most of the machine idle
+// One CTA per row instead of one warp in steps: launches of at most this many rows leave most of the machine idle
 // otherwise, and a row's time is then one warp's chain of loads and shuffles (1280 columns: 40 floats a lane).
 // B200, us per launch inside the captured step, warp / CTA per row: norm of 6 rows of 1280 columns 4.8 / 1.8, of 128 rows
-// of 1024 3.8 / 1.8; head of 16 rows of 1024 21.5 / 4.0, step begin 9.1 / 2.9.  2048 such CTAs are one wave; above that the
-// warp form reads at the HBM rate.
+// of 1024 3.8 / 1.8; head of 16 rows of 1024 21.5 / 4.0, step begin 9.1 / 2.9.  2048 CTAs of 128 threads are one wave (the
+// head's of 256 threads two); above that the warp form reads at the HBM rate.  The two add in different orders, so a prompt's
+// rows, whose results do not depend on what else their call holds, always have a warp each.
 constexpr int CTA_ROW_MAX = 2048;
 constexpr int CTA_THREADS = 128;
 constexpr int CTA_MAX_D = CTA_THREADS * 4 * 4;   // columns a CTA holds in registers
@@ -483,15 +484,15 @@ __global__ void pack_rows_kernel(const float* __restrict__ src, void* __restrict
 
 }  // namespace
 
-static bool cta_per_row(int rows, int d) { return rows <= CTA_ROW_MAX && d <= CTA_MAX_D; }
+static bool cta_per_row(bool step, int rows, int d) { return step && rows <= CTA_ROW_MAX && d <= CTA_MAX_D; }
 
 int arcb_launch_rmsnorm(const float* x, const float* w, void* out16, int rows, int d, float eps,
-                        int act_f16, cudaStream_t stream) {
+                        int act_f16, bool step, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (d % 4) return -1;
   uint16_t* out = reinterpret_cast<uint16_t*>(out16);
   auto cta = [&](auto kernel) { return arcb_launch(kernel, dim3(rows), dim3(CTA_THREADS), 0, stream, x, w, out, d, eps, act_f16); };
-  const cudaError_t e = !cta_per_row(rows, d) ? arcb_launch(rmsnorm_kernel, dim3((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
+  const cudaError_t e = !cta_per_row(step, rows, d) ? arcb_launch(rmsnorm_kernel, dim3((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
                                                             dim3(ROWS_PER_CTA * 32), 0, stream, x, w, out, rows, d, eps, act_f16)
                         : d <= CTA_THREADS * 4 ? cta(rmsnorm_cta_kernel<1>)
                         : d <= CTA_THREADS * 8 ? cta(rmsnorm_cta_kernel<2>)
@@ -510,7 +511,7 @@ int arcb_launch_embed_norm(const EmbedArgs& a, cudaStream_t stream) {
 
 int arcb_launch_decode_begin(const DecodeState& st, const EmbedArgs& a, cudaStream_t stream) {
   auto cta = [&](auto kernel) { return arcb_launch(kernel, dim3(st.n_seqs), dim3(CTA_THREADS), 0, stream, st, a); };
-  const cudaError_t e = !cta_per_row(st.n_seqs, a.d) ? arcb_launch(decode_begin_kernel, dim3((st.n_seqs + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
+  const cudaError_t e = !cta_per_row(true, st.n_seqs, a.d) ? arcb_launch(decode_begin_kernel, dim3((st.n_seqs + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
                                                                    dim3(ROWS_PER_CTA * 32), 0, stream, st, a)
                         : a.d <= CTA_THREADS * 4 ? cta(decode_begin_cta_kernel<1>)
                         : a.d <= CTA_THREADS * 8 ? cta(decode_begin_cta_kernel<2>)
@@ -522,7 +523,7 @@ int arcb_launch_decode_begin(const DecodeState& st, const EmbedArgs& a, cudaStre
 int arcb_launch_head(const HeadArgs& a, const DecodeState& st, cudaStream_t stream) {
   if (a.rows <= 0) return 0;
   auto cta = [&](auto kernel) { return arcb_launch(kernel, dim3(a.rows), dim3(HEAD_THREADS), 0, stream, a, st); };
-  const cudaError_t e = !cta_per_row(a.rows, a.d) ? arcb_launch(head_kernel, dim3((a.rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
+  const cudaError_t e = !cta_per_row(a.step != 0, a.rows, a.d) ? arcb_launch(head_kernel, dim3((a.rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA),
                                                                 dim3(ROWS_PER_CTA * 32), 0, stream, a, st)
                         : a.d <= HEAD_THREADS * 4 ? cta(head_cta_kernel<1>)
                                                   : cta(head_cta_kernel<2>);

@@ -56,13 +56,16 @@ struct HeadArgs {
   const float* lm_head;  // [14][d]
   float* logits;         // optional [rows][14]
   int* argmax;           // optional [rows]
+  int step;              // rows of a step (see arcb_launch_rmsnorm)
   // HEAD_FIRST only
   const int* first_seq; const int* prompt_len;
   const int* grid_x; const int* grid_y; const int* grid_in_output;
 };
 
+// `step`: the rows are one step of as many sequences, and the order of a row's sums may depend on their number; a prompt's rows
+// are summed in one order, whatever else the call holds.
 int arcb_launch_rmsnorm(const float* x, const float* w, void* out16, int rows, int d, float eps,
-                        int act_f16, cudaStream_t stream);
+                        int act_f16, bool step, cudaStream_t stream);
 int arcb_launch_embed_norm(const EmbedArgs& a, cudaStream_t stream);
 int arcb_launch_decode_begin(const DecodeState& st, const EmbedArgs& a, cudaStream_t stream);
 int arcb_launch_head(const HeadArgs& a, const DecodeState& st, cudaStream_t stream);
