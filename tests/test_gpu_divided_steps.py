@@ -1,0 +1,89 @@
+"""Decode steps of 33 to 256 sequences whose products divide their sums over K among the CTAs of a cluster: every epilogue, in
+clusters of two to four and of five to eight CTAs, at row counts off and on the slices that each CTA finishes."""
+import numpy as np
+import pytest
+import torch
+
+import logesun_util as lu
+import vodavik_util as vu
+from gpu_util import have_b200
+from mdlarc_scale_b200 import registry
+from mdlarc_scale_b200.engine import Engine
+from mdlarc_scale_b200.inference import generate_tokens
+from mdlarc_scale_b200.layered import Segment
+from oracle import arc_model as om
+from oracle import arc_tokens as at
+from oracle import logesun as lo
+from oracle import vodavik as vo
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_b200(), reason="needs a B200")]
+# The oracle with its operands rounded to halves moves a row by up to 8e-4 of the logits, to bfloat16 by up to 6e-3, and the grid
+# models' cache is bfloat16 in both: 6e-3, and three times that where everything is.  Mistakes planted in the oracle: the last
+# row's rotation one column off 1.9e-2 to 4.4e-2, a lost bias 3e-2 and more, a lost cache row 7e-2, up columns shifted 0.8.
+TOL = {"f16": 6e-3, "bf16": 1.8e-2}
+
+# Column tiles of 128 and K blocks of 64: qkv 12 x 4 and gate/up 11 x 4 of the first are never divided (256 sequences), qkv
+# 24 x 16 and gate/up 16 x 16 of the second make clusters of five to eight, qkv 30 x 20 and gate/up 53 x 20 of the third
+# of two to four.
+GRID = {"whole": dict(d_model=256, n_heads=4, d_ff=704, n_layers=2), "five to eight": dict(d_model=1024, n_heads=16, d_ff=1024, n_layers=2),
+        "two to four": dict(d_model=1280, n_heads=20, d_ff=3392, n_layers=1)}
+
+
+@pytest.mark.parametrize("fmt", ["f16", "bf16"])
+@pytest.mark.parametrize("rows", [33, 80, 129, 256])
+@pytest.mark.parametrize("model", sorted(GRID))
+def test_grid_steps(model, rows, fmt):
+    """Rotations, cache rows and the pairing of gate and up columns, over ragged caches; some rows end early and are held."""
+    cfg = om.Config(max_seq_len=512, num_examples=8, **GRID[model])
+    sd = om.round_bf16(om.perturb_state(om.init_state(cfg, seed=0), seed=1))
+    g = np.random.default_rng(rows)
+    new, lens = 6, g.integers(3, 40, rows)
+    forced = g.integers(0, 12, (rows, new)).astype(np.int32)
+    forced[:, 2] = 11
+    ends = {int(b): int(g.integers(0, new - 1)) for b in g.choice(rows, rows // 5, replace=False)}
+    for b, i in ends.items():
+        forced[b, i] = 13
+    prompts = [[10, *g.integers(0, 12, n - 2).tolist(), 12] for n in lens]
+    width = int(lens.max())
+    ids, pos, mask = np.zeros((rows, width), np.int64), np.zeros((rows, width, 3), np.int64), np.zeros((rows, width), bool)
+    full = np.zeros((rows, width + new), np.int64), np.zeros((rows, width + new, 3), np.int64)
+    for b, p in enumerate(prompts):
+        both = p + forced[b].tolist()
+        at_ = np.asarray(at.positions_3d(both))
+        ids[b, :len(p)], pos[b, :len(p)], mask[b, :len(p)] = p, at_[:len(p)], True
+        full[0][b, :len(both)], full[1][b, :len(both)] = both, at_
+    ex = g.integers(0, 8, rows)
+    eng = Engine(sd, cfg, "cuda:0", act_format=fmt)
+    got = generate_tokens(eng, ids, pos, mask, ex, new, stop_on_end=True, forced=forced, want_logits=True)
+    # causal: what is padded behind a sequence does not reach it
+    want = om.forward(sd, cfg, torch.from_numpy(full[0]), torch.from_numpy(full[1]), torch.from_numpy(ex))
+    seen = [(b, i) for b in range(rows) for i in range(1, ends.get(b, new - 1) + 1)]
+    b, i = (torch.tensor(x) for x in zip(*seen))
+    assert vu.rel_error(got.step_logits.cpu()[b, i], want[b, torch.from_numpy(lens)[b] - 1 + i]) < TOL[fmt]
+
+
+# With 20 K blocks of 64: fused projections and outputs of up to 29 column tiles in clusters of five to eight, the wide units and
+# the vocabulary in clusters of two to four; every expert is chosen, so no near tie decides
+LAYERED = {
+    "vodavik": (vo, vu.config(1280, 6100, [vu.attention(10, 2, 64, 64, ff=4500), vu.mlstm(5, 128, 128, ff=1000)])),
+    "logesun": (lo, lu.config(1280, 700, [lu.latent(10, 64, 32, 64, 256, 128, 40, lu.dense(3000)),
+                                          lu.latent(6, 64, 32, 64, 256, 128, 60, lu.moe(2, 2, 64, shared=900))])),
+}
+
+
+@pytest.mark.parametrize("fmt", ["f16", "bf16"])
+@pytest.mark.parametrize("slots", [48, 130, 256])
+@pytest.mark.parametrize("name", sorted(LAYERED))
+def test_layered_steps(name, slots, fmt):
+    oracle, cfg = LAYERED[name]
+    w = oracle.random_weights(cfg, 5)
+    eng = registry.build_engine(cfg, w, "cuda:0", fmt)
+    s = eng.new_session(slots, 16, 1, 8 * slots, stop_on_end=False)
+    toks = [vu.tokens(cfg, 2 + i % 6, 100 + i) for i in range(slots)]
+    at_ = [s.acquire() for _ in range(slots)]
+    s.step([Segment(a, t[:-1], []) for a, t in zip(at_, toks)])
+    got = torch.cat(s.step([Segment(a, t[-1:], [0]) for a, t in zip(at_, toks)]))
+    s.poll()
+    w64 = {k: v.double() for k, v in w.items()}
+    want = torch.stack([oracle.Sequence(cfg, w64, torch.float64).step(t)[-1] for t in toks])
+    assert vu.rel_error(got, want) < TOL[fmt]
