@@ -121,24 +121,29 @@ class Scheduler:
         ended = [r for r in self.decoding if r.produced >= self.max_new or (flags is not None and flags[r.slot])]
         if not ended:
             return
+        if self.end_token < 0:      # all of them have max_new tokens: copied while the GPU is still at the last steps
+            self._keep_logits(ended, [self.max_new] * len(ended))
         rows = self.session.out_tokens.cpu()
         for r in ended:
             row = rows[r.slot].tolist()
             if self.end_token in row:
                 row = row[:row.index(self.end_token) + 1]
             r.output = row
-        if self.session.step_logits is not None:
-            # one copy for them all, as long as the longest; each request's logits are a view of it
-            longest = max(len(r.output) for r in ended)
-            at = torch.tensor([r.slot for r in ended]).to(self.engine.device, non_blocking=True)
-            logits = self.session.step_logits[:, :longest].index_select(0, at)
-            for i, r in enumerate(ended):
-                self.step_logits[r.rid] = logits[i, :len(r.output)]
+        if self.end_token >= 0:
+            self._keep_logits(ended, [len(r.output) for r in ended])
         gone = {id(r) for r in ended}
         self.decoding = [r for r in self.decoding if id(r) not in gone]
         for r in ended:
             self.session.release(r.slot)
             self.done.append(r)
+
+    def _keep_logits(self, requests: list[Request], lengths: list[int]) -> None:
+        """Each request's rows in memory of their own: one that is kept keeps no other's, nor rows it has not picked from."""
+        if self.session.step_logits is None:
+            return
+        slots = self.session.step_logits.unbind(0)
+        for r, n in zip(requests, lengths):
+            self.step_logits[r.rid] = slots[r.slot].narrow(0, 0, n).clone()
 
     def run(self) -> list[Request]:
         """Until every submitted request is done; returns them in submission order."""

@@ -208,3 +208,16 @@ def test_scheduler_refuses_bad_prompts(prompt, error):
         return
     with pytest.raises(ValueError):
         Scheduler(_CpuEngine(), 3, 100, 1).submit(Request(0, prompt))
+
+
+@pytest.mark.parametrize("end", [None, 40])
+def test_step_logits_of_a_request_hold_its_own_rows(end):
+    """A request that ends early beside a long one is not stored at the long one's length, and keeps nothing of it alive."""
+    from mdlarc_scale_b200.generation import generate
+    out, logits = generate(_CpuEngine(), [[38], [2], [39], [5]], 30, end_token=end, return_logits=True)
+    stores = set()
+    for i, row in enumerate(out):
+        assert logits[i].shape == (len(row), 3) and logits[i][:, 0].tolist() == row
+        assert logits[i].untyped_storage().nbytes() == len(row) * 3 * 4
+        stores.add(logits[i].untyped_storage().data_ptr())
+    assert len(stores) == len(out)
