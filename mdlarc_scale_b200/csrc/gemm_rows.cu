@@ -314,7 +314,7 @@ cudaError_t launch_mode(const void* a, const void* w, const GemmEpilogue& ep, in
 // tiles of more rows, and a prompt row's result does not depend on what else its call holds (40 rows of a prompt, width 1280,
 // gated units: 10.5 us there).
 bool arcb_gemm_rows_applies(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16) {
-  if (!ep.step || ep.M > 64 || act_f16 == 2 || K % 32 || ep.N % 128) return false;
+  if (!ep.step || ep.M > 64 || act_f16 == 2 || K % 64 || ep.N % 128) return false;   // other K: the CUDA-core kernels, as beyond 64 rows
   const GroupArgs& g = ep.grp;
   if (g.tile_src || g.tile_group || g.n_tiles || g.panels || (g.n_group && g.n_group % 32) || g.lda % 8 || g.a_group % 8) return false;
   // 16-byte accesses; what is not aligned meets the tensor maps' refusal
