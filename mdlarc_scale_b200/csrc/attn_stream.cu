@@ -9,6 +9,7 @@
 // With n_splits > 1 every split writes (m, l, acc[64]) to scratch and a second kernel merges
 // the splits; with n_splits == 1 the normalised output is written directly.
 #include "attn_stream.cuh"
+#include "gemm.cuh"
 #include "launch.cuh"
 #include "ptx_sm100.cuh"
 
@@ -422,7 +423,7 @@ int arcb_launch_attn_stream(const AttnStreamArgs& a, cudaStream_t stream) {
     return (int)e;
   }
   if (a.n_splits > 1 && !a.scratch) return -1;
-  if (coop && (n_work >= 296 || a.n_splits == 1))
+  if (coop && (attn_cta_per_item(n_work, arcb_num_sms()) || a.n_splits == 1))
     e = arcb_launch(attn_stream_coop_kernel<COOP_WARPS, COOP_ROWS, 4, false>, dim3((unsigned)n_work), dim3(COOP_WARPS * 32), 0, stream, a);
   else
     e = arcb_launch(attn_stream_kernel, dim3((unsigned)blocks), dim3(WARPS_PER_CTA * 32), 0, stream, a);

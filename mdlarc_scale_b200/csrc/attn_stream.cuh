@@ -1,8 +1,8 @@
 // Launcher of the streaming (one query per item) attention kernel; see attn_stream.cu.
 #pragma once
 #include "common.cuh"
+#include "step_rules.cuh"
 
-constexpr int ATTN_CLUSTER_MAX = 8;      // splits that are merged inside the launch
 constexpr int ATTN_SCRATCH_STRIDE = 68;  // floats per (item, head, split): 64 acc, m, l, pad
 
 struct AttnStreamArgs {

@@ -194,21 +194,10 @@ static bool engine_complete(const arcb_engine* e) {
 // ---------------------------------------------------------------------------
 // session
 // ---------------------------------------------------------------------------
-// Split count of decode attention for a cache of t_max rows: up to eight splits of at least two CTA iterations (256 rows),
-// which one launch merges in clusters.  An SM holds four of its CTAs, so a launch takes as long as its waves of 592 times
-// the rows of a split: the count with the shortest such time is taken, within the first wave if that is 10 % less than with
-// fewer splits, beyond it only if it is 30 % less (2048 items: 39 us unsplit, 48 in two splits).
 // `requested` > 0 is the caller's choice (and the only one that may need scratch).
 static int choose_splits(const arcb_engine* e, int n_seqs, int requested, int t_max) {
   if (requested > 0) return requested > 64 ? 64 : requested;
-  const long long work = (long long)n_seqs * e->cfg.n_heads;
-  int best = 1;
-  double best_time = 0.;
-  for (int s = 1; s <= ATTN_CLUSTER_MAX && (s == 1 || 256LL * s <= t_max); ++s) {
-    const double time = (double)((work * s + 591) / 592) / s;
-    if (s == 1 || time < (work * s <= 592 ? 0.9 : 0.7) * best_time) { best = s; best_time = time; }
-  }
-  return best;
+  return attn_splits((long long)n_seqs * e->cfg.n_heads, t_max, arcb_num_sms());
 }
 static int scratch_splits(int requested) { return requested > 64 ? 64 : requested > 1 ? requested : 1; }
 

@@ -20,29 +20,13 @@
 #include "gemm_mid.cuh"
 #include "launch.cuh"
 #include "ptx_sm100.cuh"
+#include "step_rules.cuh"
 
 using namespace sm100;
 
 namespace {
 
 constexpr int GM_THREADS = 256;
-constexpr int GM_W_BYTES = 128 * 128;            // 128 weight rows x 64 columns
-constexpr int GM_SMEM_MAX = 222 * 1024, GM_SMEM_HALF = 111 * 1024;
-constexpr int GM_SPLIT_MAX = 8;
-
-struct GmShape {
-  int rows;          // rows of A, rounded up to 16: columns of the instruction
-  int splits;        // CTAs of a cluster
-  int stages;
-  // Never less than lets CTAs of an SM outgrow its tensor memory: with one of a cluster waiting for columns that another
-  // cluster holds, whose peer waits in turn, neither would end.
-  int smem() const {
-    const int ring = stages * (GM_W_BYTES + rows * 128), part = rows * 512, least = (rows > 128 ? 100 : 58) * 1024;
-    const int need = (ring > part ? ring : part) + 1024 + 16 * stages + 64;
-    return need > least ? need : least;
-  }
-};
-
 // SMAX: no more CTAs in a cluster (1, 4 or 8); what a thread sums is requested before the first addition.
 template <int MODE, int SMAX>
 __global__ void __launch_bounds__(GM_THREADS, SMAX == 1 ? 2 : 1)
@@ -258,7 +242,7 @@ int clusters_at_once(int splits) {
   attr.val.clusterDim.x = splits;
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits * 148);
+  cfg.gridDim = dim3(splits * arcb_num_sms());
   cfg.blockDim = dim3(GM_THREADS);
   cfg.dynamicSmemBytes = GM_SMEM_MAX;
   cfg.attrs = &attr;
@@ -273,30 +257,9 @@ int clusters_at_once(int splits) {
   return n;
 }
 
-// The split with the shortest time: a launch's and a tile's fixed cost (about 4 us a wave), operands at one SM's 110 KB a us,
-// and 2 us for the exchange, as long as all clusters run at once.  Tiles beyond one wave run two CTAs an SM where shared
-// memory allows it.
-GmShape gm_shape(int M, int N, int K) {
-  GmShape best{};
-  best.rows = (M + 15) / 16 * 16;
-  const int tiles = N / 128, num_k = K / 64, stage = GM_W_BYTES + best.rows * 128;
-  const bool two = tiles > 148 && 2 * stage + 2048 <= GM_SMEM_HALF && best.rows * 512 + 2048 <= GM_SMEM_HALF;
-  best.splits = 1;
-  double best_time = 0.;
-  for (int s = 1; s <= GM_SPLIT_MAX && s <= num_k; ++s) {
-    if (s > 1 && (tiles * s > 148 || tiles > clusters_at_once(s))) continue;
-    const int waves = s > 1 ? 1 : two ? (tiles + 295) / 296 : (tiles + 147) / 148;
-    const double time = waves * (4. + (num_k + s - 1) / s * (stage / 110e3) * (two ? 2 : 1)) + (s > 1 ? 2. : 0.);
-    if (s == 1 || time < best_time) { best.splits = s; best_time = time; }
-  }
-  const int share = (num_k + best.splits - 1) / best.splits, room = ((two ? GM_SMEM_HALF : GM_SMEM_MAX) - 2048) / stage;
-  best.stages = share < room ? share : room;
-  return best;
-}
-
 template <int MODE>
 int launch(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {
-  const GmShape sh = gm_shape(ep.M, ep.N, K);
+  const GmShape sh = gm_shape(ep.M, ep.N, K, arcb_num_sms(), clusters_at_once);
   CUtensorMap tw, ta;
   int r = arcb_make_tmap_2d_16b(&tw, w, (uint64_t)ep.N, (uint64_t)K, 128, 64, act_f16);
   if (!r) r = arcb_make_tmap_2d_16b(&ta, a, (uint64_t)ep.M, (uint64_t)(ep.grp.lda ? ep.grp.lda : K), sh.rows, 64, act_f16);
@@ -320,11 +283,7 @@ int launch(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_
 // Decode steps only: how a sum is divided depends on the number of rows, and a prompt row's result does not depend on what
 // else its call holds.
 bool arcb_gemm_mid_applies(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16) {
-  // Fewer rows are quicker on gemm_rows.cu up to 32 (us a launch here / there: 32 rows, 1280 x 1280 6.6 / 5.4, 5504 x 1024 8.7 / 7.0;
-  // 48 rows, 7.0 / 7.5 and 8.0 / 9.7), unless a CTA there has long sums of its own (24 rows, 1280 x 3456 7.8 / 10.5) or every SM
-  // several of its CTAs (16 rows, 32000 x 1280 17 / 24)
-  const bool here = ep.M > 32 || (ep.M > 16 && K >= 2560) || ep.N / 128 > 148;
-  if (!ep.step || !here || ep.M > 256 || act_f16 == 2 || K % 64 || ep.N % 128) return false;
+  if (!ep.step || !mid_transposes(ep.M, ep.N, K, arcb_num_sms()) || act_f16 == 2 || K % 64 || ep.N % 128) return false;
   const GroupArgs& g = ep.grp;
   if (g.tile_src || g.tile_group || g.n_tiles || g.panels || g.n_group || g.lda % 8) return false;
   // 16-byte accesses of the epilogues' quads; what is not aligned meets the tensor maps' refusal

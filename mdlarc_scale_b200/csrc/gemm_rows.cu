@@ -21,6 +21,7 @@
 #include "gemm_rows.cuh"
 #include "launch.cuh"
 #include "ptx_sm100.cuh"
+#include "step_rules.cuh"
 
 namespace {
 
@@ -280,10 +281,7 @@ cudaError_t launch(const void* a, const void* w, const GemmEpilogue& ep, int K, 
                      reinterpret_cast<const uint16_t*>(w), ep, K);
 }
 
-// Up to 16 rows: 32 columns a CTA once 16 make more CTAs than run at once (two an SM), for 9 rows and more some earlier, where
-// re-reading the activations counts.  us a launch, 16 / 32 columns: 1 row, 4608 x 1280 4.2 / 4.6, 5120 x 1280 5.7 / 5.0, 8192 x 2048
-// 9.0 / 7.7; 16 rows, 1280 x 1280 3.5 / 4.2, 3200 x 1280 4.8 / 4.6, 5120 x 1280 7.2 / 5.8.
-bool wide_columns(const GemmEpilogue& ep) { return ep.M <= 16 && ep.N / 16 > (ep.M <= 8 ? 296 : 192); }
+bool wide_columns(const GemmEpilogue& ep) { return rows_wide_columns(ep.M, ep.N, arcb_num_sms()); }
 
 template <int MT>
 cudaError_t launch_heads(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16, cudaStream_t stream) {

@@ -1,0 +1,73 @@
+// Rules that choose kernels and splits of decode steps from sizes and from the number of SMs: host code without CUDA, so that
+// they are tested on any machine.
+#pragma once
+
+constexpr int ATTN_CLUSTER_MAX = 8;      // splits of decode attention that are merged inside the launch
+
+// Split count of decode attention for `work` items (sequences x heads) over a cache of t_max rows: up to eight splits of at least
+// two CTA iterations (256 rows), which one launch merges in clusters.  An SM holds four of its CTAs, so a launch takes as long as
+// its waves of 4 CTAs an SM times the rows of a split: the count with the shortest such time is taken, within the first wave if
+// that is 10 % less than with fewer splits, beyond it only if it is 30 % less (148 SMs, 2048 items: 39 us unsplit, 48 in two
+// splits).
+inline int attn_splits(long long work, int t_max, int sms) {
+  int best = 1;
+  double best_time = 0.;
+  for (int s = 1; s <= ATTN_CLUSTER_MAX && (s == 1 || 256LL * s <= t_max); ++s) {
+    const double time = (double)((work * s + 4 * sms - 1) / (4 * sms)) / s;
+    if (s == 1 || time < (work * s <= 4 * sms ? 0.9 : 0.7) * best_time) { best = s; best_time = time; }
+  }
+  return best;
+}
+
+// One split of decode attention, or more of them than a cluster merges, has a CTA an item (or a warp): from two CTAs an SM on
+// the former.
+inline bool attn_cta_per_item(long long n_work, int sms) { return n_work >= 2LL * sms; }
+
+// Few-row products: 32 columns a CTA once 16 make more CTAs than run at once (two an SM), for 9 rows and more some earlier, where
+// re-reading the activations counts.  B200 (148 SMs), us a launch, 16 / 32 columns: 1 row, 4608 x 1280 4.2 / 4.6, 5120 x 1280
+// 5.7 / 5.0, 8192 x 2048 9.0 / 7.7; 16 rows, 1280 x 1280 3.5 / 4.2, 3200 x 1280 4.8 / 4.6, 5120 x 1280 7.2 / 5.8.
+inline bool rows_wide_columns(int M, int N, int sms) { return M <= 16 && N / 16 > (M <= 8 ? 2 * sms : sms * 13 / 10); }
+
+// Transposed products instead of few-row ones.  Fewer rows are quicker on gemm_rows.cu up to 32 (us a launch transposed / there: 32
+// rows, 1280 x 1280 6.6 / 5.4, 5504 x 1024 8.7 / 7.0; 48 rows, 7.0 / 7.5 and 8.0 / 9.7), unless a CTA there has long sums of its
+// own (24 rows, 1280 x 3456 7.8 / 10.5) or every SM several of its CTAs (16 rows, 32000 x 1280 17 / 24)
+inline bool mid_transposes(int M, int N, int K, int sms) { return M <= 256 && (M > 32 || (M > 16 && K >= 2560) || N / 128 > sms); }
+
+constexpr int GM_W_BYTES = 128 * 128;            // 128 weight rows x 64 columns
+constexpr int GM_SMEM_MAX = 222 * 1024, GM_SMEM_HALF = 111 * 1024;
+constexpr int GM_SPLIT_MAX = 8;
+
+struct GmShape {
+  int rows;          // rows of A, rounded up to 16: columns of the instruction
+  int splits;        // CTAs of a cluster
+  int stages;
+  // Never less than lets CTAs of an SM outgrow its tensor memory: with one of a cluster waiting for columns that another
+  // cluster holds, whose peer waits in turn, neither would end.
+  int smem() const {
+    const int ring = stages * (GM_W_BYTES + rows * 128), part = rows * 512, least = (rows > 128 ? 100 : 58) * 1024;
+    const int need = (ring > part ? ring : part) + 1024 + 16 * stages + 64;
+    return need > least ? need : least;
+  }
+};
+
+// The split with the shortest time: a launch's and a tile's fixed cost (about 4 us a wave), operands at one SM's 110 KB a us,
+// and 2 us for the exchange, as long as all clusters run at once.  Tiles beyond one wave run two CTAs an SM where shared
+// memory allows it.  clusters_at_once(s): clusters of s CTAs that run at once.
+template <typename F>
+GmShape gm_shape(int M, int N, int K, int sms, F&& clusters_at_once) {
+  GmShape best{};
+  best.rows = (M + 15) / 16 * 16;
+  const int tiles = N / 128, num_k = K / 64, stage = GM_W_BYTES + best.rows * 128;
+  const bool two = tiles > sms && 2 * stage + 2048 <= GM_SMEM_HALF && best.rows * 512 + 2048 <= GM_SMEM_HALF;
+  best.splits = 1;
+  double best_time = 0.;
+  for (int s = 1; s <= GM_SPLIT_MAX && s <= num_k; ++s) {
+    if (s > 1 && (tiles * s > sms || tiles > clusters_at_once(s))) continue;
+    const int at_once = s == 1 && two ? 2 * sms : sms, waves = s > 1 ? 1 : (tiles + at_once - 1) / at_once;
+    const double time = waves * (4. + (num_k + s - 1) / s * (stage / 110e3) * (two ? 2 : 1)) + (s > 1 ? 2. : 0.);
+    if (s == 1 || time < best_time) { best.splits = s; best_time = time; }
+  }
+  const int share = (num_k + best.splits - 1) / best.splits, room = ((two ? GM_SMEM_HALF : GM_SMEM_MAX) - 2048) / stage;
+  best.stages = share < room ? share : room;
+  return best;
+}
