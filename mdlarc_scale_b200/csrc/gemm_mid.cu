@@ -232,11 +232,9 @@ cudaError_t opt_in(K kernel, std::atomic<unsigned long long>& done) {
 // clusters of `splits` CTAs, one CTA an SM, that run at once on this device
 int clusters_at_once(int splits) {
   static std::mutex mu;
-  static int known[GM_DEVICES][GM_SPLIT_MAX + 1];                    // count + 1, 0: not asked yet
+  static int known[GM_DEVICES][GM_SPLIT_MAX + 1];
   static std::atomic<unsigned long long> opted{0};
   std::lock_guard<std::mutex> lock(mu);
-  int& slot = known[current_device()][splits];
-  if (slot) return slot - 1;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = splits;
@@ -247,14 +245,12 @@ int clusters_at_once(int splits) {
   cfg.dynamicSmemBytes = GM_SMEM_MAX;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  int n = 0;
-  if (opt_in(gemm_mid_kernel<EPI_RESID, 8>, opted) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, gemm_mid_kernel<EPI_RESID, 8>, &cfg) != cudaSuccess) {
-    n = 0;
-    cudaGetLastError();
-  }
-  slot = n + 1;
-  return n;
+  return asked_once(known[current_device()][splits], [&](int& n) {
+    const bool ok = opt_in(gemm_mid_kernel<EPI_RESID, 8>, opted) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, gemm_mid_kernel<EPI_RESID, 8>, &cfg) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+  });
 }
 
 template <int MODE>

@@ -50,6 +50,17 @@ struct GmShape {
   }
 };
 
+// A device query that is asked until it succeeds: `slot` is 0 before that and the answer + 1 from then on.  query(n) says whether n
+// was written; the answer of one that fails is 0 for this time only.
+template <typename F>
+int asked_once(int& slot, F&& query) {
+  if (slot) return slot - 1;
+  int n = 0;
+  if (!query(n)) return 0;
+  slot = n + 1;
+  return n;
+}
+
 // The split with the shortest time: a launch's and a tile's fixed cost (about 4 us a wave), operands at one SM's 110 KB a us,
 // and 2 us for the exchange, as long as all clusters run at once.  Tiles beyond one wave run two CTAs an SM where shared
 // memory allows it.  clusters_at_once(s): clusters of s CTAs that run at once.

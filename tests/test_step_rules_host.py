@@ -19,6 +19,9 @@ void shape(int M, int N, int K, int sms, int at_once_ctas, int* out) {
   const GmShape s = gm_shape(M, N, K, sms, [&](int n) { return at_once_ctas / n; });
   out[0] = s.rows; out[1] = s.splits; out[2] = s.stages; out[3] = s.smem();
 }
+int ask(int* slot, int works, int answer, int* asked) {
+  return asked_once(*slot, [&](int& n) { ++*asked; n = answer; return works != 0; });
+}
 }
 """
 
@@ -82,3 +85,12 @@ def test_shapes_fit(rules, sms):
         # tensor memory: 128 columns up to 128 rows, 256 beyond, of 512; an SM has 228 KB of shared memory, a CTA takes 1 KB more than its own
         ctas = 228 * 1024 // (smem + 1024)
         assert ctas * (128 if rows <= 128 else 256) <= 512
+
+
+def test_a_failed_query_is_asked_again(rules):
+    """Clusters that run at once on a device: an error is no answer, and an answer (none at all included) is kept."""
+    for answer in (0, 22):
+        slot, asked = C.c_int(0), C.c_int(0)
+        ask = lambda works, n: rules.ask(C.byref(slot), works, n, C.byref(asked))  # noqa: E731
+        assert [ask(0, 9), ask(0, 9), ask(1, answer), ask(1, 5), ask(0, 5)] == [0, 0, answer, answer, answer]
+        assert asked.value == 3
