@@ -218,17 +218,6 @@ int current_device() {
   return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < GM_DEVICES ? dev : 0;
 }
 
-// Shared-memory opt-in of a kernel at its first launch on a device: doing it for all forms when an engine is created loads
-// kernels that most programs never use (0.3 ms each).
-template <typename K>
-cudaError_t opt_in(K kernel, std::atomic<unsigned long long>& done) {
-  const unsigned long long bit = 1ull << current_device();
-  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_MAX);
-  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
-  return e;
-}
-
 // clusters of `splits` CTAs, one CTA an SM, that run at once on this device
 int clusters_at_once(int splits) {
   static std::mutex mu;
@@ -246,7 +235,7 @@ int clusters_at_once(int splits) {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   return asked_once(known[current_device()][splits], [&](int& n) {
-    const bool ok = opt_in(gemm_mid_kernel<EPI_RESID, 8>, opted) == cudaSuccess &&
+    const bool ok = arcb_opt_in_smem(gemm_mid_kernel<EPI_RESID, 8>, GM_SMEM_MAX, opted) == cudaSuccess &&
                     cudaOccupancyMaxActiveClusters(&n, gemm_mid_kernel<EPI_RESID, 8>, &cfg) == cudaSuccess;
     if (!ok) cudaGetLastError();
     return ok;
@@ -263,7 +252,7 @@ int launch(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_
   const uint32_t idesc = umma_idesc_f16(128, sh.rows, act_f16 ? 0 : 1, act_f16 ? 0 : 1);
   static std::atomic<unsigned long long> opted[3];
   auto run = [&](auto kernel, std::atomic<unsigned long long>& done) {
-    const cudaError_t e = opt_in(kernel, done);
+    const cudaError_t e = arcb_opt_in_smem(kernel, GM_SMEM_MAX, done);
     return e != cudaSuccess ? e : arcb_launch_cluster(kernel, sh.splits, dim3(ep.N / 128 * sh.splits), dim3(GM_THREADS), sh.smem(), stream, tw, ta, ep,
                                                       K / 64, idesc, sh);
   };

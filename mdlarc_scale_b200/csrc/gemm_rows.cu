@@ -243,7 +243,7 @@ __device__ __forceinline__ void rows_product(const uint16_t* A, const uint16_t* 
 template <int NT, int MT, int MODE, bool F16>
 __global__ void __launch_bounds__(GR_THREADS, 2)
 gemm_rows_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
-  extern __shared__ float red[];
+  extern __shared__ __align__(16) float red[];     // float4 and 16-byte asynchronous copies
   rows_product<NT, MT, MODE, F16>(A, W, ep, K, red);
 }
 
@@ -251,22 +251,8 @@ gemm_rows_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
 template <int MT, bool F16>
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(GR_THREADS, 2)
 gemm_rows_heads_kernel(const uint16_t* A, const uint16_t* W, GemmEpilogue ep, int K) {
-  extern __shared__ float red[];
+  extern __shared__ __align__(16) float red[];     // float4 and 16-byte asynchronous copies
   rows_product<1, MT, EPI_HEADS, F16>(A, W, ep, K, red);
-}
-
-// Shared-memory opt-in of a form that needs more than the default 48 KB, at its first launch on a device: doing it for all
-// forms when an engine is created loads kernels that most programs never use.
-template <typename K>
-cudaError_t opt_in(K kernel, int bytes, std::atomic<unsigned long long>& done) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  const unsigned long long bit = 1ull << dev;
-  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
-  return e;
 }
 
 template <int NT, int MT, int MODE>
@@ -275,7 +261,7 @@ cudaError_t launch(const void* a, const void* w, const GemmEpilogue& ep, int K, 
   const dim3 grid(ep.N / (16 * NT), (ep.M + Cfg::ROWS - 1) / Cfg::ROWS);
   auto kernel = act_f16 ? gemm_rows_kernel<NT, MT, MODE, true> : gemm_rows_kernel<NT, MT, MODE, false>;
   static std::atomic<unsigned long long> opted[2];
-  const cudaError_t e = opt_in(kernel, Cfg::SMEM, opted[act_f16 ? 1 : 0]);
+  const cudaError_t e = arcb_opt_in_smem(kernel, Cfg::SMEM, opted[act_f16 ? 1 : 0]);
   if (e != cudaSuccess) return e;
   return arcb_launch(kernel, grid, dim3(GR_THREADS), Cfg::SMEM, stream, reinterpret_cast<const uint16_t*>(a),
                      reinterpret_cast<const uint16_t*>(w), ep, K);
@@ -288,7 +274,7 @@ cudaError_t launch_heads(const void* a, const void* w, const GemmEpilogue& ep, i
   using Cfg = GrCfg<1, MT>;
   auto kernel = act_f16 ? gemm_rows_heads_kernel<MT, true> : gemm_rows_heads_kernel<MT, false>;
   static std::atomic<unsigned long long> opted[2];
-  const cudaError_t e = opt_in(kernel, Cfg::SMEM, opted[act_f16 ? 1 : 0]);
+  const cudaError_t e = arcb_opt_in_smem(kernel, Cfg::SMEM, opted[act_f16 ? 1 : 0]);
   if (e != cudaSuccess) return e;
   return arcb_launch(kernel, dim3(ep.N / 16, (ep.M + Cfg::ROWS - 1) / Cfg::ROWS), dim3(GR_THREADS), Cfg::SMEM, stream,
                      reinterpret_cast<const uint16_t*>(a), reinterpret_cast<const uint16_t*>(w), ep, K);

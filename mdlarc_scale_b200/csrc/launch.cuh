@@ -12,6 +12,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <utility>
 
 bool arcb_pdl_enabled();
@@ -53,4 +54,17 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t arcb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                Args&&... args) {
   return arcb_launch_cluster(kernel, 1, grid, block, smem, stream, std::forward<Args>(args)...);
+}
+
+// Shared-memory opt-in of a kernel that needs more than the default 48 KB, at its first launch on a device (`done`: a bit each):
+// doing it for all forms when an engine is created loads kernels that most programs never use (0.3 ms each).
+template <typename K>
+inline cudaError_t arcb_opt_in_smem(K kernel, int bytes, std::atomic<unsigned long long>& done) {
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  int dev = 0;
+  const unsigned long long bit = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? 1ull << dev : 0;   // 0: every launch
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
