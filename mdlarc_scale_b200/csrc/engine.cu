@@ -89,6 +89,7 @@ extern "C" int arcb_engine_create(const arcb_config* cfg, arcb_engine** out) {
   arcb_engine* e = new arcb_engine();
   e->cfg = *cfg;
   cudaGetDevice(&e->device);
+  e->sms = arcb_num_sms();
   const size_t d = cfg->d_model, dff = cfg->d_ff;
   e->layers.resize(cfg->n_layers);
   e->loaded.assign((size_t)ARCB_T_COUNT * cfg->n_layers, 0);
@@ -194,12 +195,14 @@ static bool engine_complete(const arcb_engine* e) {
 // ---------------------------------------------------------------------------
 // session
 // ---------------------------------------------------------------------------
-// `requested` > 0 is the caller's choice (and the only one that may need scratch).
+// `requested` > 0 is the caller's choice.
 static int choose_splits(const arcb_engine* e, int n_seqs, int requested, int t_max) {
   if (requested > 0) return requested > 64 ? 64 : requested;
-  return attn_splits((long long)n_seqs * e->cfg.n_heads, t_max, arcb_num_sms());
+  return attn_splits((long long)n_seqs * e->cfg.n_heads, t_max, e->sms);
 }
-static int scratch_splits(int requested) { return requested > 64 ? 64 : requested > 1 ? requested : 1; }
+static int scratch_splits(const arcb_engine* e, int n_seqs, int requested) {
+  return attn_scratch_splits((long long)n_seqs * e->cfg.n_heads, requested, e->sms);
+}
 
 struct WsLayout {
   size_t x, xn, q, attn, h, k16, v16, scratch, gemm_scratch, ints, total;
@@ -234,7 +237,7 @@ extern "C" int64_t arcb_session_workspace_bytes(const arcb_engine* e, int32_t n_
                                                 int32_t max_prefill_tokens, int32_t attn_splits) {
   if (!e || n_seqs <= 0 || max_prefill_tokens < 0) return -1;
   if (e->lm) return lm_workspace_bytes(e, n_seqs, max_prefill_tokens, attn_splits);
-  return (int64_t)ws_layout(e, n_seqs, max_prefill_tokens, scratch_splits(attn_splits)).total;
+  return (int64_t)ws_layout(e, n_seqs, max_prefill_tokens, scratch_splits(e, n_seqs, attn_splits)).total;
 }
 
 extern "C" int64_t arcb_kv_cache_bytes(const arcb_engine* e, int32_t n_seqs, int32_t t_max) {
@@ -269,7 +272,7 @@ extern "C" int arcb_session_create(arcb_engine* e, const arcb_session_desc* dsc,
     return ARCB_OK;
   }
   const int splits = choose_splits(e, dsc->n_seqs, dsc->attn_splits, dsc->t_max);
-  const WsLayout w = ws_layout(e, dsc->n_seqs, dsc->max_prefill_tokens, scratch_splits(dsc->attn_splits));
+  const WsLayout w = ws_layout(e, dsc->n_seqs, dsc->max_prefill_tokens, scratch_splits(e, dsc->n_seqs, dsc->attn_splits));
   if ((size_t)dsc->workspace_bytes < w.total) return arcb_fail(ARCB_E_ARG, "workspace too small");
   arcb_session* s = new arcb_session();
   s->eng = e;
@@ -283,7 +286,7 @@ extern "C" int arcb_session_create(arcb_engine* e, const arcb_session_desc* dsc,
   s->h16 = reinterpret_cast<uint16_t*>(base + w.h);
   s->k16 = reinterpret_cast<uint16_t*>(base + w.k16);
   s->v16 = reinterpret_cast<uint16_t*>(base + w.v16);
-  s->attn_scratch = dsc->attn_splits > 1 ? reinterpret_cast<float*>(base + w.scratch) : nullptr;
+  s->attn_scratch = scratch_splits(e, dsc->n_seqs, dsc->attn_splits) > 1 ? reinterpret_cast<float*>(base + w.scratch) : nullptr;
   s->gemm_scratch = reinterpret_cast<float*>(base + w.gemm_scratch);
   int* ints = reinterpret_cast<int*>(base + w.ints);
   const int B = dsc->n_seqs;

@@ -43,6 +43,7 @@ struct LayerWeights {
 struct arcb_engine {
   arcb_config cfg;
   int device = 0;
+  int sms = 148;          // of its device
   std::vector<LayerWeights> layers;
   float* token_embed = nullptr;
   float* example_embed = nullptr;

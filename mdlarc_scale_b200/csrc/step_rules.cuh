@@ -4,12 +4,25 @@
 
 constexpr int ATTN_CLUSTER_MAX = 8;      // splits of decode attention that are merged inside the launch
 
+// One split of decode attention, or more of them than a cluster merges, has a CTA an item (or a warp): from two CTAs an SM on
+// the former.
+inline bool attn_cta_per_item(long long n_work, int sms) { return n_work >= 2LL * sms; }
+
 // Split count of decode attention for `work` items (sequences x heads) over a cache of t_max rows: up to eight splits of at least
 // two CTA iterations (256 rows), which one launch merges in clusters.  An SM holds four of its CTAs, so a launch takes as long as
 // its waves of 4 CTAs an SM times the rows of a split: the count with the shortest such time is taken, within the first wave if
 // that is 10 % less than with fewer splits, beyond it only if it is 30 % less (148 SMs, 2048 items: 39 us unsplit, 48 in two
 // splits).
+// Few items over a long cache leave most of the machine idle in eight splits: more of them, 2.7 CTAs an SM, and a merge launch.
+// It costs 5 us, and a split of eight 1 us for every 128 rows: B200, us a layer, eight splits / more: 12 heads over 10 k rows
+// 14.0 / 14.2, 12 k 16.3 / 14.9, 32 k 36.5 / 24.3; 16 heads 14.9 / 15.3, 17.6 / 15.6, 40.6 / 28.0; 20 heads 15.8 / 16.6, 18.4 / 18.1,
+// 41.9 / 33.1; 24 heads 16.5 / 16.9, 19.1 / 18.8, 43.7 / 36.9; 28 heads 17.0 / 19.4, 20.1 / 21.9, 45.8 / 42.8.
 inline int attn_splits(long long work, int t_max, int sms) {
+  if (t_max > 12288 && work * ATTN_CLUSTER_MAX <= sms * 13 / 10) {
+    const long long s = (sms * 27 / 10 + work - 1) / work;
+    const int many = s < 64 ? (int)s : 64;
+    if (many > ATTN_CLUSTER_MAX && attn_cta_per_item(work * many, sms)) return many;
+  }
   int best = 1;
   double best_time = 0.;
   for (int s = 1; s <= ATTN_CLUSTER_MAX && (s == 1 || 256LL * s <= t_max); ++s) {
@@ -19,9 +32,12 @@ inline int attn_splits(long long work, int t_max, int sms) {
   return best;
 }
 
-// One split of decode attention, or more of them than a cluster merges, has a CTA an item (or a warp): from two CTAs an SM on
-// the former.
-inline bool attn_cta_per_item(long long n_work, int sms) { return n_work >= 2LL * sms; }
+// Splits that a session's scratch is made for: the caller's choice, or the most that any cache is given; 1: none.
+inline int attn_scratch_splits(long long work, int requested, int sms) {
+  if (requested > 0) return requested > 64 ? 64 : requested;
+  const int s = attn_splits(work, 0x7fffffff, sms);
+  return s > ATTN_CLUSTER_MAX ? s : 1;
+}
 
 // Few-row products: 32 columns a CTA once 16 make more CTAs than run at once (two an SM), for 9 rows and more some earlier, where
 // re-reading the activations counts.  B200 (148 SMs), us a launch, 16 / 32 columns: 1 row, 4608 x 1280 4.2 / 4.6, 5120 x 1280

@@ -2,12 +2,16 @@
 choose them."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
 from gpu_util import have_b200, stream, to_act
 from mdlarc_scale_b200 import _lib, registry
+from mdlarc_scale_b200.engine import Engine
+from mdlarc_scale_b200.inference import generate_tokens
 from mdlarc_scale_b200.layered import Segment
+from oracle import arc_model as om
 from oracle import vodavik as vo
 from vodavik_util import attention, config, mlstm, oracle_logits, rel_error, tokens
 
@@ -89,6 +93,28 @@ def test_splits_merged_in_a_cluster(lib, splits, T):
         p = torch.softmax(torch.einsum("hd,htd->ht", q[i].double(), k[s, :, :n].double()) / 8, -1)
         ref = torch.einsum("ht,htd->hd", p, v[s, :, :n].double())
         assert ((outs[0][i].double() - ref).abs() <= ref.abs() * 2 ** -11 + 1e-5).all()
+
+
+@pytest.mark.parametrize("rows,t_max,scratch", [(2, 12290, True), (2, 12200, True), (1, 12400, False), (6, 12290, True), (7, 12290, False)])
+def test_few_sequences_over_a_long_cache(lib, rows, t_max, scratch):
+    """More splits than a cluster merges where four heads x `rows` leave the machine idle in eight (5 to 24 of them, beyond 12288
+    rows): a long and some short caches, against one split.  Both sum in 32 bits and round a layer's outputs to halves once:
+    a rounding turned over is 2^-11 of one element."""
+    cfg = om.make_config("tiny", max_seq_len=16384)
+    eng = Engine(om.round_bf16(om.perturb_state(om.init_state(cfg, seed=0), seed=1)), cfg, "cuda:0")
+    g = np.random.default_rng(rows)
+    new = 4
+    lens = np.array([t_max - new] + [40] * (rows - 1))
+    width = int(lens.max())
+    ids, mask = g.integers(0, 12, (rows, width)), np.arange(width)[None] < lens[:, None]
+    pos = np.stack([g.integers(0, m, (rows, width)) for m in (30, 30, 5)], -1)
+    forced = g.integers(0, 12, (rows, new)).astype(np.int32)
+    out = [generate_tokens(eng, ids, pos, mask, None, new, stop_on_end=False, forced=forced, want_logits=True, attn_splits=s).step_logits
+           for s in (0, 1, 0)]
+    assert torch.equal(out[0], out[2]) and bool(torch.isfinite(out[0]).all())
+    assert rel_error(out[0][:, 1:].flatten(0, 1), out[1][:, 1:].flatten(0, 1)) < 1e-3
+    sizes = [eng.new_session(rows, t_max, new, 64, attn_splits=s).workspace.numel() for s in (0, 1)]
+    assert (sizes[0] > sizes[1]) == scratch
 
 
 @pytest.mark.parametrize("fmt", [_lib.ACT_F16, _lib.ACT_BF16])

@@ -12,6 +12,7 @@ SOURCE = r"""
 #include "step_rules.cuh"
 extern "C" {
 int splits(long long work, int t_max, int sms) { return attn_splits(work, t_max, sms); }
+int scratch(long long work, int requested, int sms) { return attn_scratch_splits(work, requested, sms); }
 int cta_per_item(long long n, int sms) { return attn_cta_per_item(n, sms); }
 int wide(int M, int N, int sms) { return rows_wide_columns(M, N, sms); }
 int transposes(int M, int N, int K, int sms) { return mid_transposes(M, N, K, sms); }
@@ -33,6 +34,7 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", str(CSRC), str(d / "rules.cpp"), "-o", str(d / "rules.so")], check=True)
     lib = C.CDLL(str(d / "rules.so"))
     lib.splits.argtypes = [C.c_longlong, C.c_int, C.c_int]
+    lib.scratch.argtypes = [C.c_longlong, C.c_int, C.c_int]
     lib.cta_per_item.argtypes = [C.c_longlong, C.c_int]
     return lib
 
@@ -45,7 +47,8 @@ def shape(rules, M, N, K, sms, at_once=None):
 
 # what the choices were measured with
 MEASURED = {
-    "splits": [((2048, 400), 1), ((6 * 20, 5200), 4), ((4, 190), 1), ((20, 10240), 8), ((16 * 16, 1200), 2)],
+    "splits": [((2048, 400), 1), ((6 * 20, 5200), 4), ((4, 190), 1), ((20, 10240), 8), ((20, 12288), 8), ((20, 12289), 20), ((16, 32768), 25),
+               ((24, 16384), 17), ((25, 16384), 8), ((5, 20000), 64), ((4, 32768), 8), ((16 * 16, 1200), 2)],
     "wide": [((1, 4608), 0), ((1, 4736), 0), ((1, 4864), 1), ((16, 1280), 0), ((16, 3072), 0), ((16, 3200), 1), ((17, 32000), 0)],
     "transposes": [((32, 1280, 1280), 0), ((33, 1280, 1280), 1), ((24, 1280, 3456), 1), ((16, 32000, 1280), 1), ((16, 18944, 1280), 0),
                    ((256, 1280, 1280), 1), ((257, 1280, 1280), 0)],
@@ -69,6 +72,17 @@ def test_lines_move_with_the_sm_count(rules):
     assert rules.transposes(16, 75 * 128, 1280, 74) and not rules.transposes(16, 74 * 128, 1280, 74)
     # 24 tiles of 16 K blocks: clusters of six fill 148 SMs, fewer CTAs a cluster fit 74
     assert shape(rules, 40, 3072, 1024, 148)[1] == 6 and shape(rules, 40, 3072, 1024, 74)[1] in (1, 2, 3)
+
+
+@pytest.mark.parametrize("sms", [1, 66, 148, 160])
+def test_scratch_holds_every_choice(rules, sms):
+    """Splits that no cluster merges find scratch, whatever the cache, and have a CTA iteration of rows each."""
+    for work in range(1, 400):
+        room = rules.scratch(work, 0, sms)
+        for t_max in (1, 255, 256, 4096, 12288, 12289, 16384, 65536, 2 ** 31 - 1):
+            s = rules.splits(work, t_max, sms)
+            assert 1 <= s <= 64 and (s <= 8 or (s <= room and t_max >= 128 * s and rules.cta_per_item(work * s, sms)))
+        assert rules.scratch(work, 5, sms) == 5 and rules.scratch(work, 99, sms) == 64
 
 
 @pytest.mark.parametrize("sms", [1, 66, 132, 148, 160])
