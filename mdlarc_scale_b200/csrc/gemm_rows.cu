@@ -13,7 +13,7 @@
 //   * the eight warps' sums meet in shared memory, always in the same order, and leave through the epilogues' quads.
 // B200, us a launch inside the captured step, tcgen05 tiles / here: 16 rows, QKV of width 1024 10.3 / 4.6, gate/up 10.6 / 5.4,
 // out and down 10.7 / 3.9; 1 row of width 256 6.1 to 6.8 / 1.9 to 2.4; 1 row, mixer projection of width 1280 14.2 / 6.5.
-// Steps of up to 64 rows that gemm_mid.cu does not take.
+// Steps of up to 32 rows, and of up to 64 in products with column groups (step_rules.cuh draws the line to gemm_mid.cu).
 #include <atomic>
 
 #include "common.cuh"
@@ -286,19 +286,20 @@ cudaError_t launch_mode(const void* a, const void* w, const GemmEpilogue& ep, in
   if (N1 == 1 && wide_columns(ep)) return ep.M <= 8 ? launch<2, 1, MODE>(a, w, ep, K, act_f16, stream) : launch<2, 2, MODE>(a, w, ep, K, act_f16, stream);
   if (ep.M <= 8) return launch<N1, 1, MODE>(a, w, ep, K, act_f16, stream);
   if (ep.M <= 16) return launch<N1, 2, MODE>(a, w, ep, K, act_f16, stream);
-  if (ep.M <= 32) return launch<2, 4, MODE>(a, w, ep, K, act_f16, stream);
-  return launch<2, 8, MODE>(a, w, ep, K, act_f16, stream);
+  if constexpr (MODE == EPI_ACT)
+    if (ep.M > 32) return launch<2, 8, MODE>(a, w, ep, K, act_f16, stream);
+  return launch<2, 4, MODE>(a, w, ep, K, act_f16, stream);
 }
 
 }  // namespace
 
-// Up to 64 rows: the weights' 16-row fragments meet eight 8-row activation fragments, and the activations of a CTA
-// (64 rows x K) are re-read from L2 by every CTA (48 rows of width 1280, tcgen05 tiles / here: outputs 10.9 / 9.0, gated units
-// 12.7 / 10.5 us).  One row tile more would read the weights twice.  Steps only: K is added in other parts than in the tcgen05
-// tiles of more rows, and a prompt row's result does not depend on what else its call holds (40 rows of a prompt, width 1280,
-// gated units: 10.5 us there).
+// Steps only: K is added in other parts than in the tcgen05 tiles of more rows, and a prompt row's result does not depend on what else
+// its call holds (48 rows of width 1280, gated units: 10.5 us here, 12.7 there).
+// With column groups, which the transposed tiles do not take, up to 64 rows: the weights' 16-row fragments meet eight 8-row
+// activation fragments, and the activations of a CTA (64 rows x K) are re-read from L2 by every CTA.  One row tile more would read
+// the weights twice.
 bool arcb_gemm_rows_applies(const void* a, const void* w, const GemmEpilogue& ep, int K, int act_f16) {
-  if (!ep.step || ep.M > 64 || act_f16 == 2 || K % 64 || ep.N % 128) return false;   // other K: the CUDA-core kernels, as beyond 64 rows
+  if (!ep.step || ep.M > (ep.grp.n_group ? 64 : 32) || act_f16 == 2 || K % 64 || ep.N % 128) return false;   // other K: the CUDA-core kernels, as beyond 64 rows
   const GroupArgs& g = ep.grp;
   if (g.tile_src || g.tile_group || g.n_tiles || g.panels || (g.n_group && g.n_group % 32) || g.lda % 8 || g.a_group % 8) return false;
   // 16-byte accesses; what is not aligned meets the tensor maps' refusal
@@ -325,8 +326,7 @@ int arcb_launch_gemm_rows(const void* a, const void* w, const GemmEpilogue& ep, 
       }
       e = ep.M <= 8    ? launch_heads<1>(a, w, ep, K, act_f16, stream)
           : ep.M <= 16 ? launch_heads<2>(a, w, ep, K, act_f16, stream)
-          : ep.M <= 32 ? launch_heads<4>(a, w, ep, K, act_f16, stream)
-                       : launch_heads<8>(a, w, ep, K, act_f16, stream);
+                       : launch_heads<4>(a, w, ep, K, act_f16, stream);
       break;
   }
   arcb_count_launch(1);
