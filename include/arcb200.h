@@ -39,7 +39,7 @@ extern "C" {
 
 #define ARCB_GEMM_AUTO 0 /* tcgen05 GEMM wherever the shape allows (K % 64 == 0)   */
 #define ARCB_GEMM_SIMT 1 /* CUDA-core GEMM everywhere (debug cross-check)      */
-#define ARCB_GEMM_TC 2   /* tcgen05 GEMM everywhere                            */
+#define ARCB_GEMM_TC 2   /* as AUTO; the arcb_op_* calls refuse K % 64 != 0    */
 #define ARCB_GEMM_TC_1CTA 3 /* arcb_op_gemm only: the 1-CTA tcgen05 kernels        */
 #define ARCB_GEMM_TC_2CTA 4 /* arcb_op_gemm only: the 2-CTA (cta_group::2) kernel  */
 

@@ -6,8 +6,9 @@
 // is read exactly once, and the softmax is kept online per 8-lane group (warp shuffles for the
 // dot product, one rescale per 16 rows), merged across the 4 groups at the end.
 //
-// With n_splits > 1 every split writes (m, l, acc[64]) to scratch and a second kernel merges
-// the splits; with n_splits == 1 the normalised output is written directly.
+// One split writes the normalised output directly.  Two to eight splits of a cache with 128 rows for each are the CTAs of a
+// cluster, whose first one merges them in shared memory; more splits, or shorter caches, write (m, l, acc[64]) to scratch and a
+// second kernel merges them.
 #include "attn_stream.cuh"
 #include "gemm.cuh"
 #include "launch.cuh"

@@ -36,7 +36,6 @@ __device__ __forceinline__ float cta_sum(float v, float* sm) {
 
 __device__ __forceinline__ float sum_sq(float4 v) { return (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); }
 
-
 // `lane` of `lanes` threads on the row
 __device__ __forceinline__ void embed_row(const LmEmbedArgs& a, int row, int tok, int lane, int lanes = 32) {
   tok = min(max(tok, 0), a.vocab - 1);

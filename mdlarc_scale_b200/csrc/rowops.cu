@@ -1,4 +1,4 @@
-// Row-wise kernels (one warp per row, HBM-bound, float4 accesses):
+// Row-wise kernels (float4 accesses; one warp per row, bound by HBM, or in steps of few rows one CTA per row, bound by latency):
 //   embed_norm    : token + example embedding -> residual stream, fused first RMSNorm
 //   rmsnorm       : RMSNorm of the residual stream -> 16-bit GEMM operand
 //   decode_begin  : grid-state position update + embedding + first RMSNorm of a decode step
