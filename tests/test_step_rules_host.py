@@ -74,6 +74,19 @@ def test_lines_move_with_the_sm_count(rules):
     assert shape(rules, 40, 3072, 1024, 148)[1] == 6 and shape(rules, 40, 3072, 1024, 74)[1] in (1, 2, 3)
 
 
+# (column tiles, K blocks) -> CTAs of a cluster: the products that test_gpu_divided_steps.py means by its clusters
+DIVIDED = {(1, 1): [(6, 4), (11, 4)],
+           (5, 8): [(18, 12), (12, 12), (12, 20), (21, 20), (8, 20), (15, 20), (10, 16), (6, 20), (10, 20)],
+           (2, 4): [(30, 20), (53, 20), (28, 20), (41, 20), (36, 20), (47, 20), (30, 16), (48, 20)]}
+
+
+@pytest.mark.parametrize("least,most", sorted(DIVIDED))
+def test_clusters_of_step_products(rules, least, most):
+    for tiles, blocks in DIVIDED[least, most]:
+        for M in (33, 48, 80, 129, 130, 256):
+            assert least <= shape(rules, M, 128 * tiles, 64 * blocks, 148, 132)[1] <= most, (tiles, blocks, M)
+
+
 @pytest.mark.parametrize("sms", [1, 66, 148, 160])
 def test_scratch_holds_every_choice(rules, sms):
     """Splits that no cluster merges find scratch, whatever the cache, and have a CTA iteration of rows each."""
