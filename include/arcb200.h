@@ -414,7 +414,8 @@ int arcb_op_rmsnorm(const float* d_x, const float* d_w, void* d_out16, int32_t r
 /* y[M,N] (fp32) = A[M,K] * W[N,K]^T, A and W both in the 16-bit format `act_format`
  * (the tensor-core MMA needs one format for both operands): nn.Linear without bias as used
  * at src/inference.py:402,410 / src/transformer.py:260-263.
- * gemm_path selects the tcgen05 or the CUDA-core kernel. */
+ * gemm_path selects the tcgen05 or the CUDA-core kernel.  ARCB_ACT_F32: 32-bit operands (AUTO: bf16 pieces on tcgen05
+ * where K % 64 == 0, as 32-bit layered models use; SIMT: multiply-adds). */
 int arcb_op_gemm(const void* d_a16, const void* d_w16, float* d_y, int32_t M, int32_t N,
                  int32_t K, int32_t act_format, int32_t gemm_path, void* stream);
 

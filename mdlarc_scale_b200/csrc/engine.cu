@@ -12,6 +12,7 @@
 #include "attn_prefill.cuh"
 #include "attn_stream.cuh"
 #include "gemm.cuh"
+#include "gemm_split.cuh"
 #include "launch.cuh"
 #include "engine.cuh"
 #include "rowops.cuh"
@@ -624,14 +625,23 @@ extern "C" int arcb_op_gemm(const void* a16, const void* w, float* y, int32_t M,
   if (!a16 || !w || !y || M <= 0) return arcb_fail(ARCB_E_ARG, "bad gemm arguments");
   CKL(ensure_gemm_init(), "gemm init");
   if (N % 128 || K % 32) return arcb_fail(ARCB_E_ARG, "gemm needs N % 128 == 0 and K % 32 == 0");
+  GemmEpilogue ep{};
+  ep.mode = EPI_STORE_F32; ep.M = M; ep.N = N; ep.y = y;
+  if (act_format == ARCB_ACT_F32) {
+    if (gemm_path != ARCB_GEMM_AUTO && gemm_path != ARCB_GEMM_SIMT) return arcb_fail(ARCB_E_ARG, "32-bit gemm: gemm_path AUTO or SIMT");
+    ep.act_f16 = 2;
+    if (gemm_path == ARCB_GEMM_AUTO && arcb_gemm_split_applies(a16, w, ep, K))
+      CKL(arcb_launch_gemm_split(a16, w, ep, K, (cudaStream_t)stream), "gemm");
+    else
+      CKL(arcb_launch_gemm(a16, w, ep, K, 2, false, (cudaStream_t)stream, 0), "gemm");
+    return ARCB_OK;
+  }
   const int variant = gemm_path == ARCB_GEMM_TC_1CTA ? 1 : (gemm_path == ARCB_GEMM_TC_2CTA ? 2 : 0);
   bool tc = gemm_path == ARCB_GEMM_TC || variant != 0 || (gemm_path == ARCB_GEMM_AUTO);
   if (tc && !arcb_gemm_tc_supported(M, N, K)) {
     if (gemm_path != ARCB_GEMM_AUTO) return arcb_fail(ARCB_E_ARG, "tcgen05 gemm needs K % 64 == 0");
     tc = false;
   }
-  GemmEpilogue ep{};
-  ep.mode = EPI_STORE_F32; ep.M = M; ep.N = N; ep.y = y;
   CKL(arcb_launch_gemm(a16, w, ep, K, act_format == ARCB_ACT_F16, tc, (cudaStream_t)stream, variant), "gemm");
   return ARCB_OK;
 }

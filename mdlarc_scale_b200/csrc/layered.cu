@@ -14,6 +14,7 @@
 #include "attn_prefill_gqa.cuh"
 #include "engine.cuh"
 #include "gemm.cuh"
+#include "gemm_split.cuh"
 #include "launch.cuh"
 #include "layerops.cuh"
 #include "mlstm.cuh"
@@ -738,6 +739,7 @@ bool lm_armed(const arcb_session* s) { return s->ls->armed; }
 namespace {
 
 int lm_gemm(const LayeredModel& m, const void* a, const void* w, GemmEpilogue& ep, int K, cudaStream_t stream, int variant = 0) {
+  if (m.fmt == 2 && m.d.gemm_path != ARCB_GEMM_SIMT && arcb_gemm_split_applies(a, w, ep, K)) return arcb_launch_gemm_split(a, w, ep, K, stream);
   return arcb_launch_gemm(a, w, ep, K, m.fmt, lm_tc(m), stream, variant);
 }
 
