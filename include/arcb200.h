@@ -520,6 +520,44 @@ typedef struct arcb_prompt_build_args {
 
 int arcb_build_prompts(const arcb_prompt_build_args* args, void* stream);
 
+/* Padded batch to the arrays arcb_prefill_args takes (pack_prompts.cu).  Real tokens become rows that store K/V at their
+ * index among the real tokens of their sequence and see the real tokens at or ahead of them (not causal: all of the sequence).
+ * A first generated token is read at padded index max(len - 1, 0); where that is a padded position, a query-only row is made
+ * for it (src/inference.py:420-423).  The batch arrays are those of the whole batch, [n_batch][seq_len]. */
+typedef struct arcb_pack_args {
+  const void* d_ids;               /* [batch][seq_len] */
+  const void* d_pos;               /* [batch][seq_len][3] */
+  const uint8_t* d_mask;           /* [batch][seq_len], non-zero: a real token; NULL: all are */
+  int32_t id_bytes, pos_bytes;     /* 4 or 8 */
+  int32_t n_seqs, seq_len;         /* sequences of this call */
+  int32_t causal;
+  int32_t all_positions;           /* padded positions become query-only rows */
+  int32_t with_first;
+  int32_t reserved;
+  const int32_t* d_rows;           /* [n_seqs] batch row = cache row */
+  const int32_t* d_len;            /* [n_seqs] real tokens */
+  const int32_t* d_row_start;      /* [n_seqs] first packed row */
+  const int32_t* d_kv_start;       /* [n_seqs] first K/V scratch row */
+  const int32_t* d_extra;          /* [n_seqs] row of the query-only first-token row where one is needed */
+  int32_t* d_token_ids;            /* [n_tokens], d_pos_xyz three per token */
+  int32_t* d_pos_xyz;
+  int32_t* d_seq;
+  int32_t* d_kv_slot;
+  int32_t* d_kv_count;
+  int32_t* d_kv_row;
+  int32_t* d_first_row;            /* [n_seqs], with_first */
+  int32_t* d_first_seq;
+  int32_t* d_prompt_len;
+  int32_t* d_grid_x;
+  int32_t* d_grid_y;
+  int32_t* d_grid_in_output;
+} arcb_pack_args;
+
+int arcb_pack_prompts(const arcb_pack_args* args, void* stream);
+
+/* d_out [n_rows][3]: real tokens of a row, whether its index max(real tokens - 1, 0) is one, one more than its last real index. */
+int arcb_mask_stats(const uint8_t* d_mask, int32_t n_rows, int32_t seq_len, int32_t* d_out, void* stream);
+
 /* One fixed-width record per generated sequence: the candidate grid mapped back to the task's own
  * orientation and colours. status: 0 = no grid (nothing between the last IO_SEP and END),
  * 1 = rectangular grid, 2 = malformed (jagged or only separators). input_copy = 1 when the grid as

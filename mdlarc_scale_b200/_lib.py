@@ -46,7 +46,7 @@ EXPORTS = [
     "arcb_session_poll", "arcb_engine_saturation_count", "arcb_session_attention_probe", "arcb_launch_count", "arcb_op_rmsnorm", "arcb_op_gemm",
     "arcb_op_gemm_residual", "arcb_gemm_splitk_scratch_bytes", "arcb_op_gemm_residual_splitk",
     "arcb_attn_scratch_bytes", "arcb_op_decode_attention", "arcb_op_decode_attention_static",
-    "arcb_op_head", "arcb_build_prompts", "arcb_canonicalize_candidates",
+    "arcb_op_head", "arcb_build_prompts", "arcb_canonicalize_candidates", "arcb_pack_prompts", "arcb_mask_stats",
 ]
 STATIC_ATTN_MAX_RECORDS = 16384
 
@@ -129,6 +129,19 @@ class PromptBuildArgs(C.Structure):
     ]
 
 
+class PackArgs(C.Structure):
+    _fields_ = [
+        ("d_ids", C.c_void_p), ("d_pos", C.c_void_p), ("d_mask", C.c_void_p),
+        ("id_bytes", C.c_int32), ("pos_bytes", C.c_int32), ("n_seqs", C.c_int32), ("seq_len", C.c_int32),
+        ("causal", C.c_int32), ("all_positions", C.c_int32), ("with_first", C.c_int32), ("reserved", C.c_int32),
+        ("d_rows", C.c_void_p), ("d_len", C.c_void_p), ("d_row_start", C.c_void_p), ("d_kv_start", C.c_void_p),
+        ("d_extra", C.c_void_p), ("d_token_ids", C.c_void_p), ("d_pos_xyz", C.c_void_p), ("d_seq", C.c_void_p),
+        ("d_kv_slot", C.c_void_p), ("d_kv_count", C.c_void_p), ("d_kv_row", C.c_void_p), ("d_first_row", C.c_void_p),
+        ("d_first_seq", C.c_void_p), ("d_prompt_len", C.c_void_p), ("d_grid_x", C.c_void_p), ("d_grid_y", C.c_void_p),
+        ("d_grid_in_output", C.c_void_p),
+    ]
+
+
 class CandidateArgs(C.Structure):
     _fields_ = [
         ("n_rows", C.c_int32), ("max_new", C.c_int32),
@@ -182,6 +195,8 @@ def load() -> C.CDLL:
     lib.arcb_session_attention_probe.argtypes = [vp, C.POINTER(C.c_float)]
     lib.arcb_engine_saturation_count.argtypes = [vp, C.POINTER(i64), i32, vp]
     lib.arcb_build_prompts.argtypes = [C.POINTER(PromptBuildArgs), vp]
+    lib.arcb_pack_prompts.argtypes = [C.POINTER(PackArgs), vp]
+    lib.arcb_mask_stats.argtypes = [vp, i32, i32, vp, vp]
     lib.arcb_canonicalize_candidates.argtypes = [C.POINTER(CandidateArgs), vp]
     lib.arcb_launch_count.restype = i64
     lib.arcb_launch_count.argtypes = [C.c_int]

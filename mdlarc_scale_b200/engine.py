@@ -511,6 +511,102 @@ def plan_prefill(ids: np.ndarray, pos: np.ndarray, mask: np.ndarray, rows: np.nd
         n_first=n_first, kv_row_identity=identity, **plan_first)
 
 
+class PaddedBatch:
+    """A padded batch (tokens [B, S], positions [B, S, 3], mask [B, S] or None, host arrays or tensors) on the engine's
+    device, and the prefill calls of it: what ``plan_prefill`` makes on the host is made there by one kernel.
+
+    ``lens`` (real tokens), ``last_valid`` (whether index max(len - 1, 0) is one) and ``end`` (one more than the last real
+    index) of every row are host arrays."""
+
+    def __init__(self, ids, pos, mask, device):
+        self.device = torch.device(device)
+        self.n, self.seq_len = (int(v) for v in ids.shape)
+        pos = pos[:self.n, :self.seq_len, :3]
+        if tuple(pos.shape) != (self.n, self.seq_len, 3):
+            raise ValueError("positions must have shape [batch, seq_len, 3]")
+        if mask is not None and tuple(mask.shape) != (self.n, self.seq_len):
+            raise ValueError("mask must have shape [batch, seq_len]")
+        self.h2d_bytes = 0
+        self.ids, self.pos = (t if t.dtype in (torch.int32, torch.int64) else t.to(torch.int64) for t in map(self._upload, (ids, pos)))
+        self.mask = None
+        if mask is None:
+            self.lens = np.full(self.n, self.seq_len, np.int64)
+            self.last_valid, self.end = np.ones(self.n, bool), self.lens
+            return
+        if isinstance(mask, torch.Tensor):
+            mask = mask.detach().to(torch.bool)
+        if isinstance(mask, torch.Tensor) and mask.device.type == "cuda":
+            self.mask = mask.to(self.device).contiguous()
+            stats = torch.empty((self.n, 3), dtype=torch.int32, device=self.device)
+            with torch.cuda.device(self.device):
+                _lib.check(_lib.load().arcb_mask_stats(self.mask.data_ptr(), self.n, self.seq_len, stats.data_ptr(), _stream_ptr(self.device)))
+            stats = stats.cpu().numpy().astype(np.int64)
+            self.lens, self.last_valid, self.end = stats[:, 0], stats[:, 1].astype(bool), stats[:, 2]
+            return
+        host = np.ascontiguousarray(mask, dtype=bool)
+        self.mask = self._upload(host)
+        self.lens = host.sum(axis=1)
+        self.last_valid = host[np.arange(self.n), np.clip(self.lens - 1, 0, None)]
+        self.end = np.where(self.lens > 0, self.seq_len - host[:, ::-1].argmax(axis=1), 0)
+
+    def _upload(self, a) -> torch.Tensor:
+        """Whole numbers of 4 or 8 bytes (or a mask) on the device, contiguous."""
+        if not isinstance(a, torch.Tensor):
+            a = np.ascontiguousarray(a, dtype=a.dtype if a.dtype in (np.int32, np.int64, np.bool_) else np.int64)
+            a = torch.from_numpy(a if a.flags.writeable else a.copy())
+        t = a.detach()
+        if t.device != self.device:
+            self.h2d_bytes += t.numel() * t.element_size()
+        return t.to(self.device, non_blocking=True).contiguous()
+
+    def plan(self, rows: np.ndarray, is_causal: bool = True, all_positions: bool = False, with_first: bool = True) -> PrefillPlan:
+        """``plan_prefill`` of the batch rows ``rows`` (ascending), as device tensors."""
+        n, S, dev = len(rows), self.seq_len, self.device
+        lens, last_valid = self.lens[rows], self.last_valid[rows]
+        counts = np.full(n, S, np.int64) if all_positions else lens            # packed rows of each sequence
+        row_start, kv_start = np.cumsum(counts) - counts, np.cumsum(lens) - lens
+        packed, n_kv = int(counts.sum()), int(lens.sum())
+        needs = np.zeros(n, bool) if all_positions or not with_first else ~last_valid
+        extra = packed + np.cumsum(needs) - needs
+        total = packed + int(needs.sum())
+        # query blocks of at most 256 rows of a sequence, most expensive first: the attention kernel takes them in this order, so
+        # that its tail is made of cheap ones
+        blocks = (counts + 255) // 256
+        of = np.repeat(np.arange(n), blocks)
+        at = 256 * (np.arange(int(blocks.sum())) - np.repeat(np.cumsum(blocks) - blocks, blocks))
+        qb_rows = np.minimum(256, counts[of] - at)
+        keys = np.minimum(at + qb_rows, lens[of]) if is_causal else lens[of]
+        own = np.flatnonzero(needs)
+        qb0, qbn = np.concatenate([row_start[of] + at, extra[own]]), np.concatenate([qb_rows, np.ones(len(own), np.int64)])
+        qb_kv0 = np.concatenate([kv_start[of], kv_start[own]])
+        order = np.argsort(-np.concatenate([keys, np.minimum(lens[own], np.maximum(lens[own] - 1, 0) + 1)]), kind="stable")
+        host = torch.from_numpy(np.concatenate([rows, lens, row_start, kv_start, extra, qb0[order], qbn[order], qb_kv0[order]]).astype(np.int32))
+        small = host.to(dev, non_blocking=True)
+        self.h2d_bytes += host.numel() * 4
+        per, q = small[:5 * n].view(5, n), small[5 * n:].view(3, -1)
+        out = torch.empty(8 * total, dtype=torch.int32, device=dev)
+        tok, pxyz, seq, slot, cnt, kv_row = (out[a * total:b * total] for a, b in ((0, 1), (1, 4), (4, 5), (5, 6), (6, 7), (7, 8)))
+        first = torch.empty((6, n), dtype=torch.int32, device=dev) if with_first else None
+        args = _lib.PackArgs(
+            d_ids=_ptr(self.ids), d_pos=_ptr(self.pos), d_mask=_ptr(self.mask), id_bytes=self.ids.element_size(),
+            pos_bytes=self.pos.element_size(), n_seqs=n, seq_len=S, causal=int(is_causal), all_positions=int(all_positions),
+            with_first=int(with_first), d_rows=_ptr(per[0]), d_len=_ptr(per[1]), d_row_start=_ptr(per[2]), d_kv_start=_ptr(per[3]),
+            d_extra=_ptr(per[4]), d_token_ids=_ptr(tok), d_pos_xyz=_ptr(pxyz), d_seq=_ptr(seq), d_kv_slot=_ptr(slot),
+            d_kv_count=_ptr(cnt), d_kv_row=_ptr(kv_row))
+        if with_first:
+            for k, name in enumerate(("first_row", "first_seq", "prompt_len", "grid_x", "grid_y", "grid_in_output")):
+                setattr(args, "d_" + name, _ptr(first[k]))
+        with torch.cuda.device(dev):
+            _lib.check(_lib.load().arcb_pack_prompts(C.byref(args), _stream_ptr(dev)))
+        # K/V scratch rows are the packed rows where every real token comes ahead of every query-only row
+        identity = not all_positions or bool((lens[:-1] == S).all() and self.end[rows[-1]] == lens[-1])
+        f = [None] * 6 if first is None else list(first)
+        return PrefillPlan(
+            n_tokens=total, token_ids=tok, pos_xyz=pxyz.view(-1, 3), seq=seq, kv_slot=slot, kv_count=cnt, n_qblocks=q.shape[1],
+            qblock_row0=q[0], qblock_rows=q[1], qblock_kv0=q[2], kv_row=kv_row, n_kv_rows=n_kv, n_first=n if with_first else 0,
+            first_row=f[0], first_seq=f[1], prompt_len=f[2], grid_x=f[3], grid_y=f[4], grid_in_output=f[5], kv_row_identity=identity)
+
+
 def chunk_rows(lens: np.ndarray, max_tokens: int) -> list[np.ndarray]:
     """Greedy split of sequence indices into chunks whose packed token count fits ``max_tokens``."""
     chunks, cur, tot = [], [], 0

@@ -26,7 +26,7 @@ import torch
 from .data import (DIHEDRAL_TRANSFORMS, END_TOKEN_ID, IO_SEP_TOKEN_ID, apply_color_perm_grid, as_rect_array,
                    compute_positions_3d, decode_output_grid, dihedral_np, encode_example, encode_example_np,
                    generate_color_permutations)
-from .engine import Engine, Session, chunk_rows, engine_for, plan_prefill
+from .engine import Engine, PaddedBatch, Session, chunk_rows, engine_for, plan_prefill
 
 DEFAULT_PREFILL_TOKENS = 65536  # packed prompt tokens per prefill call (bounds the workspace)
 POLL_EVERY = 32                 # decode steps between two host checks of the finished counter
@@ -110,6 +110,9 @@ def generate_tokens(engine: Engine, ids: np.ndarray, pos: np.ndarray, mask: np.n
     dev = engine.device
     B, S = ids.shape
     lens = mask.sum(axis=1)
+    # the plans of the prefill calls are made on the device, unless most of what would have to cross is padding
+    plain = pos.shape == (B, S, 3) and mask.shape == (B, S)
+    batch = PaddedBatch(ids, pos, mask, dev) if plain and 0 < B * S <= 4 * int(lens.sum()) else None
     t_max = int(lens.max()) + int(max_new)
     cap = int(min(max_prefill_tokens, int(lens.sum()) + 2 * B))
     cap = max(cap, int(lens.max()) + 2, B)
@@ -131,15 +134,17 @@ def generate_tokens(engine: Engine, ids: np.ndarray, pos: np.ndarray, mask: np.n
     first_logits = torch.zeros((B, 14), dtype=torch.float32, device=dev) if want_logits else None
     n_prefill = 0
     for rows in chunk_rows(lens, session.max_prefill_tokens):
-        plan = plan_prefill(ids, pos, mask, rows)
-        h2d += plan.h2d_bytes()
+        if batch is not None:
+            plan = batch.plan(rows)
+        else:
+            plan = plan_prefill(ids, pos, mask, rows)
+            h2d += plan.h2d_bytes()
+            plan = plan.to(dev)
         n_prefill += plan.n_tokens
-        fl = None
-        if first_logits is not None:
-            fl = torch.zeros((len(rows), 14), dtype=torch.float32, device=dev)
-        session.prefill(plan.to(dev), ex_dev, first_logits=fl)
-        if fl is not None:
-            first_logits[torch.from_numpy(rows).to(dev)] = fl
+        fl = None if first_logits is None else first_logits[int(rows[0]):int(rows[-1]) + 1]     # consecutive rows
+        session.prefill(plan, ex_dev, first_logits=fl)
+    if batch is not None:
+        h2d += batch.h2d_bytes
     steps_total = max_new - 1
     done = 0
     while done < steps_total:

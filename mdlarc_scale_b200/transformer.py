@@ -5,7 +5,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from .engine import Engine, plan_prefill
+from .engine import Engine, PaddedBatch
 from .inference import DEFAULT_PREFILL_TOKENS, _resolve_engine
 
 
@@ -21,24 +21,19 @@ def forward_logits(model, input_ids: torch.Tensor, pos_xyz: torch.Tensor,
     """
     engine = _resolve_engine(model, input_ids.device)
     B, S = input_ids.shape
-    ids = input_ids.detach().cpu().numpy()
-    pos = pos_xyz.detach().cpu().numpy()
-    mask = (np.ones((B, S), dtype=bool) if attention_mask is None
-            else attention_mask.detach().to(torch.bool).cpu().numpy())
     dev = engine.device
     per_call = max(1, max_prefill_tokens // max(S, 1))
+    batch = PaddedBatch(input_ids, pos_xyz, attention_mask, dev)
     cap = min(B, per_call) * S
-    session = engine.new_session(B, max(int(mask.sum(axis=1).max()), 1), 1, cap, stop_on_end=False)
+    session = engine.new_session(B, max(int(batch.lens.max()), 1), 1, cap, stop_on_end=False)
     ex_dev = None
     if example_ids is not None and engine.use_example_embedding:
         ex_dev = example_ids.detach().to(device=dev, dtype=torch.int32).contiguous()
     out = torch.empty((B, S, 14), dtype=torch.float32, device=dev)
     for r0 in range(0, B, per_call):
         rows = np.arange(r0, min(B, r0 + per_call))
-        plan = plan_prefill(ids, pos, mask, rows, is_causal=is_causal, all_positions=True, with_first=False)
-        logits = torch.empty((plan.n_tokens, 14), dtype=torch.float32, device=dev)
-        session.prefill(plan.to(dev), ex_dev, logits_all=logits)
-        out[r0:r0 + len(rows)] = logits.view(len(rows), S, 14)
+        plan = batch.plan(rows, is_causal=is_causal, all_positions=True, with_first=False)
+        session.prefill(plan, ex_dev, logits_all=out[r0:r0 + len(rows)])
     session.poll()
     session.close()
     return out.to(input_ids.device) if input_ids.device.type == "cuda" else out.cpu()
