@@ -113,6 +113,12 @@ extern "C" int arcb_engine_create(const arcb_config* cfg, arcb_engine** out) {
                              (size_t)cfg->max_z * ARCB_ROPE_PZ);
   r |= dev_alloc(e, &e->rope, rope_n);
   r |= dev_alloc(e, &e->d_err, 64);
+  r |= dev_alloc(e, &e->step_layers, e->layers.size());
+  if (!r) {
+    std::vector<StepLayer> host;
+    for (const auto& L : e->layers) host.push_back({L.ln1_w, L.w_qkv, L.w_out, L.ln2_w, L.w_gu, L.b_gu, L.w_down, L.b_down});
+    r = (int)cudaMemcpy(e->step_layers, host.data(), host.size() * sizeof(StepLayer), cudaMemcpyHostToDevice);
+  }
   if (r) {
     arcb_engine_destroy(e);
     return arcb_fail(ARCB_E_STATE, "cudaMalloc of packed weights failed");
@@ -318,6 +324,10 @@ extern "C" int arcb_session_create(arcb_engine* e, const arcb_session_desc* dsc,
   // stream order.
   s->state_ints = ints;
   s->n_state_ints = w.n_int;
+  s->step_probe = reinterpret_cast<unsigned long long*>(ints + ((13 * (size_t)B + 9) & ~(size_t)1));
+  // a caller that chooses kernels or splits gets the separate launches
+  if (dsc->attn_splits <= 0 && e->cfg.gemm_path == ARCB_GEMM_AUTO && e->cfg.attn_path == ARCB_ATTN_AUTO)
+    s->step_cluster = arcb_step_cluster(B, e->cfg.d_model, e->cfg.d_ff, e->cfg.n_layers, dsc->t_max);
   cudaError_t r = cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking);
   if (r != cudaSuccess) { delete s; return arcb_fail_cuda(r, "cudaStreamCreate"); }
   if (cudaEventCreate(&s->probe_begin) != cudaSuccess || cudaEventCreate(&s->probe_end) != cudaSuccess) {
@@ -493,9 +503,8 @@ extern "C" int arcb_prefill(arcb_session* s, const arcb_prefill_args* a, void* s
   return ARCB_OK;
 }
 
-static int record_decode_step(arcb_session* s, cudaStream_t stream) {
-  if (s->ls) return lm_record_step(s, stream);
-  arcb_engine* e = s->eng;
+static EmbedArgs step_embed_args(const arcb_session* s) {
+  const arcb_engine* e = s->eng;
   const arcb_config& c = e->cfg;
   const int B = s->desc.n_seqs;
   EmbedArgs ea{};
@@ -503,16 +512,31 @@ static int record_decode_step(arcb_session* s, cudaStream_t stream) {
   ea.token_ids = nullptr; ea.seq = nullptr; ea.example_ids = s->use_examples ? s->example_ids : nullptr;
   ea.token_embed = e->token_embed; ea.example_embed = e->example_embed; ea.ln_w = e->layers[0].ln1_w;
   ea.x = s->x; ea.xn16 = s->xn16; ea.eps = c.norm_eps; ea.act_f16 = e->act_f16() ? 1 : 0;
-  CKL(arcb_launch_decode_begin(s->st, ea, stream), "decode_begin");
+  return ea;
+}
+
+static HeadArgs step_head_args(const arcb_session* s) {
+  const arcb_engine* e = s->eng;
+  const arcb_config& c = e->cfg;
+  const int B = s->desc.n_seqs;
+  HeadArgs ha{};
+  ha.mode = HEAD_DECODE; ha.step = 1; ha.rows = B; ha.d = c.d_model; ha.eps = c.norm_eps; ha.x = s->x;
+  ha.lnf_w = e->lnf_w; ha.lm_head = e->lm_head;
+  return ha;
+}
+
+static int record_decode_step(arcb_session* s, cudaStream_t stream) {
+  if (s->ls) return lm_record_step(s, stream);
+  arcb_engine* e = s->eng;
+  const arcb_config& c = e->cfg;
+  const int B = s->desc.n_seqs;
+  CKL(arcb_launch_decode_begin(s->st, step_embed_args(s), stream), "decode_begin");
   for (int l = 0; l < c.n_layers; ++l) {
     int r = run_layer(s, l, B, s->st.pos, s->st.slot, nullptr, s->st.kv_len,
                       s->desc.stop_on_end == 1 ? s->st.finished : nullptr, false, nullptr, stream);
     if (r) return r;
   }
-  HeadArgs ha{};
-  ha.mode = HEAD_DECODE; ha.step = 1; ha.rows = B; ha.d = c.d_model; ha.eps = c.norm_eps; ha.x = s->x;
-  ha.lnf_w = e->lnf_w; ha.lm_head = e->lm_head;
-  CKL(arcb_launch_head(ha, s->st, stream), "head(decode)");
+  CKL(arcb_launch_head(step_head_args(s), s->st, stream), "head(decode)");
   return ARCB_OK;
 }
 
@@ -522,6 +546,23 @@ extern "C" int arcb_decode(arcb_session* s, int32_t n_steps, void* stream_v) {
     return arcb_fail(ARCB_E_STATE, "arcb_prefill with first-token rows must run before arcb_decode");
   if (n_steps <= 0) return ARCB_OK;
   cudaStream_t stream = (cudaStream_t)stream_v;
+  if (s->step_cluster > 0) {
+    const arcb_engine* e = s->eng;
+    const arcb_config& c = e->cfg;
+    StepArgs a{};
+    a.layers = e->step_layers; a.n_layers = c.n_layers; a.rows = s->desc.n_seqs; a.d = c.d_model; a.dff = c.d_ff; a.n_heads = c.n_heads;
+    a.n_steps = n_steps;
+    a.embed = step_embed_args(s);
+    a.head = step_head_args(s);
+    a.rope = e->rope; a.max_x = c.max_x; a.max_y = c.max_y; a.max_z = c.max_z;
+    a.cache = reinterpret_cast<__nv_bfloat16*>(s->desc.d_kv_cache);
+    a.skip = s->desc.stop_on_end == 1 ? s->st.finished : nullptr;
+    a.probe = s->step_probe;
+    CKL(arcb_launch_step_cluster(s->st, a, s->step_cluster, stream), "decode steps");
+    s->step_stream = stream;
+    s->probe_recorded = true;
+    return ARCB_OK;
+  }
   for (int attempt = 0; !s->graph_exec && attempt < 2; ++attempt) {
     const long long before = g_launches.load();
     CK(cudaStreamBeginCapture(s->capture_stream, cudaStreamCaptureModeThreadLocal));
@@ -582,7 +623,14 @@ extern "C" int arcb_engine_saturation_count(arcb_engine* e, int64_t* count, int3
 
 extern "C" int arcb_session_attention_probe(arcb_session* s, float* ms) {
   if (!s || !ms) return arcb_fail(ARCB_E_ARG, "null argument");
-  if (!s->probe_recorded || !s->graph_exec) return arcb_fail(ARCB_E_STATE, "no decode step has run yet");
+  if (!s->probe_recorded || (!s->graph_exec && !s->step_cluster)) return arcb_fail(ARCB_E_STATE, "no decode step has run yet");
+  if (s->step_cluster) {
+    unsigned long long ns[2] = {0, 0};
+    CK(cudaStreamSynchronize(s->step_stream));
+    CK(cudaMemcpy(ns, s->step_probe, sizeof ns, cudaMemcpyDeviceToHost));
+    *ms = (float)(ns[1] - ns[0]) * 1e-6f;
+    return ARCB_OK;
+  }
   cudaError_t r = cudaEventSynchronize(s->probe_end);
   if (r == cudaSuccess) r = cudaEventElapsedTime(ms, s->probe_begin, s->probe_end);
   if (r != cudaSuccess) {

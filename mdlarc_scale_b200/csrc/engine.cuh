@@ -7,6 +7,7 @@
 #include "../../include/arcb200.h"
 #include "common.cuh"
 #include "rowops.cuh"
+#include "step_cluster.cuh"
 
 int arcb_fail(int code, const char* msg);
 int arcb_fail_cuda(cudaError_t e, const char* where);
@@ -49,6 +50,7 @@ struct arcb_engine {
   float* example_embed = nullptr;
   float* lnf_w = nullptr;
   float* lm_head = nullptr;
+  StepLayer* step_layers = nullptr;   // device copy of the layers' pointers
   float* rope = nullptr;  // cos_x | sin_x | cos_y | sin_y | cos_z | sin_z
   int* d_err = nullptr;
   std::vector<void*> allocs;
@@ -78,6 +80,9 @@ struct arcb_session {
   cudaGraphExec_t graph_exec = nullptr;
   cudaStream_t capture_stream = nullptr;
   long long graph_kernels = 0;
+  int step_cluster = 0;            // > 0: steps run inside one cluster of that many CTAs instead of the recorded graph
+  unsigned long long* step_probe = nullptr;
+  cudaStream_t step_stream = nullptr;   // of the last such steps
   bool armed = false;
   // event pair recorded (as graph nodes) around the layer-0 decode-attention launch of every replay
   cudaEvent_t probe_begin = nullptr, probe_end = nullptr;

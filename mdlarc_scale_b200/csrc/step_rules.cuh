@@ -98,3 +98,38 @@ GmShape gm_shape(int M, int N, int K, int sms, F&& clusters_at_once) {
   best.stages = share < room ? share : room;
   return best;
 }
+
+// Steps inside one cluster (step_cluster.cu): shared memory of a CTA, in bytes from its start.
+struct StepClusterSmem {
+  int xn, hs, q, rec, red, tokens, head, even, odd, total;
+};
+constexpr int STEP_CLUSTER_SMEM_MAX = 220 * 1024;
+
+inline StepClusterSmem step_cluster_smem(int rows, int d, int dff, int heads, int cl) {
+  const int items = rows * heads, records = items < cl ? cl : items;
+  const int qkv = (3 * d / 16 + cl - 1) / cl, gu = 2 * ((dff / 16 + cl - 1) / cl), wide = qkv > gu ? qkv : gu, narrow = (d / 16 + cl - 1) / cl;
+  const int long_k = d > dff ? d : dff;
+  StepClusterSmem s;
+  s.xn = 2 * 8 * d * 4;
+  s.hs = s.xn + 8 * (d * 2 + 64);
+  s.q = s.hs + 8 * (dff * 2 + 64);
+  s.rec = s.q + 8 * d * 2;
+  s.red = s.rec + records * 68 * 4;
+  s.tokens = s.red + wide * 8 * 160 * 4;
+  s.head = s.tokens + (14 + 8) * d * 4;
+  s.even = (s.head + 15 * d * 4 + 127) / 128 * 128;
+  s.odd = s.even + wide * 32 * d;                                    // 16 rows a tile
+  s.total = s.odd + narrow * 32 * long_k;
+  return s;
+}
+
+// B200, four layers of width 256, us a token of a call, a graph of launches / one cluster: one row over 200 rows 85 / 57, 1000 91 / 62,
+// 2000 92 / 67; two rows over 1000 94 / 70; four over 200 86 / 75, 500 94 / 79; eight over 100 85 / 95, 200 88 / 96.  Weights and cached
+// rows beyond 16 MB a step (14 MB at 2000) are for the whole machine.
+constexpr int STEP_CLUSTER_ROWS = 4;
+inline bool step_cluster_fits(int rows, int d, int dff, int n_layers, int t_max, int cl) {
+  if (rows < 1 || rows > STEP_CLUSTER_ROWS || d > 512 || d % 128 || dff % 64) return false;
+  if (step_cluster_smem(rows, d, dff, d / 64, cl).total > STEP_CLUSTER_SMEM_MAX) return false;
+  const long long bytes = (long long)n_layers * (2LL * (4LL * d * d + 3LL * d * dff) + 4LL * d * rows * t_max);
+  return bytes <= 16LL << 20;
+}

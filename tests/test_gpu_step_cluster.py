@@ -1,0 +1,114 @@
+"""Decode steps inside one cluster against the separate launches (which a session with a chosen split count takes)."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import have_b200
+from mdlarc_scale_b200 import _lib
+from mdlarc_scale_b200.engine import Engine
+from mdlarc_scale_b200.inference import generate_tokens
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_b200(), reason="needs a B200")]
+
+
+def engine(d, dff, layers, act="f16", seed=0):
+    g = torch.Generator().manual_seed(seed)
+
+    def r(*s, std=1.0, mean=0.0):
+        return (torch.randn(s, generator=g) * std + mean).to(torch.bfloat16).float()
+    w = {"token_embed.weight": r(14, d), "example_embed.weight": r(8, d, std=0.02), "ln_f.weight": r(d, std=0.05, mean=1.0),
+         "lm_head.weight": r(14, d, std=d ** -0.5)}
+    for n in range(layers):
+        p = f"blocks.{n}."
+        w.update({p + "ln1.weight": r(d, std=0.05, mean=1.0), p + "attn.qkv_proj.weight": r(3 * d, d, std=d ** -0.5),
+                  p + "attn.out_proj.weight": r(d, d, std=d ** -0.5), p + "ln2.weight": r(d, std=0.05, mean=1.0),
+                  p + "ffn.fc_gate.weight": r(dff, d, std=d ** -0.5), p + "ffn.fc_gate.bias": r(dff, std=0.05),
+                  p + "ffn.fc_up.weight": r(dff, d, std=d ** -0.5), p + "ffn.fc_up.bias": r(dff, std=0.05),
+                  p + "ffn.fc_down.weight": r(d, dff, std=0.5 * dff ** -0.5), p + "ffn.fc_down.bias": r(d, std=0.05)})
+    config = dict(d_model=d, n_heads=d // 64, n_layers=layers, d_ff=dff, vocab_size=14, max_seq_len=4096, num_examples=8, max_x=32,
+                  max_y=32, max_z=8, rope_base=10000.0, norm_eps=1e-5, use_example_embedding=True)
+    return Engine(w, config, "cuda:0", act_format=act)
+
+
+def batch(rows, lens, seed=0):
+    g = np.random.default_rng(seed)
+    lens = np.resize(np.array(lens), rows)
+    width = int(lens.max())
+    ids, mask = g.integers(0, 12, (rows, width)), np.arange(width)[None] < lens[:, None]
+    pos = np.stack([g.integers(0, m, (rows, width)) for m in (30, 30, 5)], -1)
+    return ids, pos, mask, g.integers(0, 8, rows)
+
+
+# one to four rows and one more; fewer and more (row, head) items than CTAs, items that do not divide them; K of fewer blocks than warps; more
+# tiles and blocks than are requested ahead; prompts at the edges of the slices of 16 keys
+@pytest.mark.parametrize("act", ["f16", "bf16"])
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("d,dff,layers", [(128, 64, 1), (128, 192, 3), (256, 704, 4), (256, 896, 2), (384, 256, 1), (256, 64, 2), (512, 1024, 1)])
+def test_steps_match_separate_launches(d, dff, layers, rows, act):
+    eng = engine(d, dff, layers, act, seed=rows)
+    ids, pos, mask, ex = batch(rows, [1, 15, 16, 17, 130, 257, 90, 33], seed=d)
+    new = 9
+    forced = np.random.default_rng(1).integers(0, 12, (rows, new)).astype(np.int32)
+    lib, counts, logits = _lib.load(), [], []
+    for splits in (0, 1):
+        lib.arcb_launch_count(1)
+        out = generate_tokens(eng, ids, pos, mask, ex, new, stop_on_end=False, forced=forced, want_logits=True, attn_splits=splits)
+        counts.append(lib.arcb_launch_count(1))
+        logits.append(out.step_logits)
+    # steps that fit were not launched one kernel after the other
+    fits = rows <= 4 and (d, dff) != (512, 1024)
+    assert counts[0] < counts[1] - 20 if fits else counts[0] >= counts[1] - 1
+    # both round at the same places; sums in another order turn a rounding (2^-11, bf16 2^-8) over here and there
+    scale = logits[1].square().mean().sqrt()
+    assert bool(torch.isfinite(logits[0]).all())
+    assert float((logits[0] - logits[1]).square().mean().sqrt() / scale) < (2 ** -9 if act == "f16" else 2 ** -6)
+    eng.close()
+
+
+def test_loop_ends_freezes_and_constrains_as_separate_launches_do():
+    eng = engine(256, 704, 2)
+    ids, pos, mask, ex = batch(4, [40, 9, 77, 130])
+    for kw in (dict(), dict(stop_on_end=False), dict(freeze_finished=False),
+               dict(constraints=dict(palette_mask=np.tile(np.arange(10) % 3 == 0, (4, 1)), target_shape=np.full((4, 2), 3), disallow_tokens=(10, 12))),
+               dict(temperature=1.3, top_k=5, sample_seed=11)):
+        a, b = (generate_tokens(eng, ids, pos, mask, ex, 70, want_logits=True, attn_splits=s, **kw) for s in (0, 1))
+        n = min(a.tokens.shape[1], b.tokens.shape[1])
+        for i in range(4):
+            same = (a.tokens[i, :n] == b.tokens[i, :n]).cpu()
+            first = n if bool(same.all()) else int((~same).float().argmax())
+            # up to the first token that a rounding decides, and that one has to be close
+            torch.testing.assert_close(a.step_logits[i, :first], b.step_logits[i, :first], rtol=0.02, atol=0.02)
+            if first < n and "temperature" not in kw and "constraints" not in kw:
+                top = b.step_logits[i, first].sort().values
+                assert float(top[-1] - top[-2]) < 0.04
+
+
+def test_steps_in_parts_are_steps_in_one_go():
+    eng = engine(256, 704, 3)
+    ids, pos, mask, ex = batch(2, [50, 31])
+    from mdlarc_scale_b200.engine import plan_prefill
+    got = []
+    for parts in ([12], [1, 1, 10], [5, 7]):
+        s = eng.new_session(2, 80, 13, 128, stop_on_end=False, want_step_logits=True)
+        s.prefill(plan_prefill(ids, pos, mask, np.arange(2)).to(torch.device("cuda:0")), torch.from_numpy(ex).int().cuda())
+        for n in parts:
+            s.decode(n)
+        s.poll()
+        got.append((s.out_tokens.clone(), s.step_logits.clone()))
+        assert 0.0 <= s.attention_probe_ms() < 1.0
+        s.close()
+    for t, lg in got[1:]:
+        assert torch.equal(t, got[0][0]) and torch.equal(lg, got[0][1])
+
+
+def test_full_cache_drops_keys_and_reports_it():
+    eng = engine(128, 192, 1)
+    ids, pos, mask, ex = batch(1, [30])
+    from mdlarc_scale_b200.engine import plan_prefill
+    for splits in (0, 1):
+        s = eng.new_session(1, 32, 200, 64, stop_on_end=False, attn_splits=splits)
+        s.prefill(plan_prefill(ids, pos, mask, np.arange(1)).to(torch.device("cuda:0")), torch.from_numpy(ex).int().cuda())
+        s.decode(s.t_max - 30 + 3)
+        with pytest.raises(_lib.ArcbError):
+            s.poll()
+        s.close()
