@@ -960,6 +960,8 @@ int lm_mixer(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
     }
     if (R.pa && m.d.mlstm_path == ARCB_MLSTM_AUTO && arcb_mlstm_chunk_supported(L.dimp, L.vdimp, m.fmt))
       CKL(arcb_launch_mlstm_chunk(a, stream), "mlstm chunks");
+    else if (R.pa && m.d.mlstm_path == ARCB_MLSTM_AUTO && arcb_mlstm_chunk32_supported(L.dimp, L.vdimp, m.fmt))
+      CKL(arcb_launch_mlstm_chunk32(a, stream), "mlstm chunks");
     else
       CKL(arcb_launch_mlstm_step(a, stream), "mlstm");
   } else if (R.pa && m.fmt != 2 && m.d.attn_path == ARCB_ATTN_AUTO && R.pa->n_qblocks > 0 &&

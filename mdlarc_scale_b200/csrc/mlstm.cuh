@@ -40,6 +40,8 @@ struct MlstmArgs {
 bool arcb_mlstm_chunk_supported(int dimp, int vdimp, int fmt);
 int arcb_mlstm_chunk_init();
 int arcb_launch_mlstm_chunk(const MlstmArgs& a, cudaStream_t stream);
+bool arcb_mlstm_chunk32_supported(int dimp, int vdimp, int fmt);
+int arcb_launch_mlstm_chunk32(const MlstmArgs& a, cudaStream_t stream);
 int arcb_launch_mlstm_step(const MlstmArgs& a, cudaStream_t stream);
 void arcb_count_launch(long long n);
 int arcb_mlstm_walk_init();
