@@ -85,8 +85,10 @@ moe_route_kernel(MoeArgs a) {
   }
 }
 
-// One CTA of eight warps per ROUTER_ROWS rows, which also multiplies the rows with the router (16-bit formats).
-constexpr int ROUTER_WARPS = 8, ROUTER_ROWS = 2;
+// One CTA of sixteen warps per ROUTER_ROWS rows, which also multiplies the rows with the router (16-bit formats).
+// Bound by a chain of latencies, not by bytes (31 rows, 32 experts, 1024 columns: 64 KB of router): two experts a warp
+// and all of its columns' loads at once, 14.1 -> 11.1 us a launch (eight warps of four experts, two loads ahead).
+constexpr int ROUTER_WARPS = 16, ROUTER_ROWS = 2, ROUTER_EXPERTS = 2;
 template <int PER_LANE>
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
 moe_router_kernel(MoeArgs a) {
@@ -99,27 +101,37 @@ moe_router_kernel(MoeArgs a) {
 #pragma unroll
   for (int r = 0; r < ROUTER_ROWS; ++r)
     x[r] = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.xn) + (size_t)min(row0 + r, a.rows - 1) * a.pitch);
-  for (int e0 = warp * 4; e0 < a.experts; e0 += ROUTER_WARPS * 4) {
-    float d[ROUTER_ROWS][4] = {};
+  for (int e0 = warp * ROUTER_EXPERTS; e0 < a.experts; e0 += ROUTER_WARPS * ROUTER_EXPERTS) {
+    float d[ROUTER_ROWS][ROUTER_EXPERTS] = {};
     const uint4* w = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.w_router) + (size_t)e0 * a.pitch);
-#pragma unroll 2
-    for (int i = lane; i < n; i += 32) {                 // rows behind the last expert are zero
-      uint4 wv[4];
+    // up to five loads of 256 columns on their way: a warp's time is its rounds of loads
+    constexpr int AT_ONCE = 5;
+    for (int i0 = lane; i0 < n; i0 += 32 * AT_ONCE) {
+      uint4 wv[AT_ONCE][ROUTER_EXPERTS], xv[AT_ONCE][ROUTER_ROWS];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) wv[e] = __ldg(w + (size_t)e * n + i);
+      for (int b = 0; b < AT_ONCE; ++b) {
+        const int i = i0 + 32 * b;
 #pragma unroll
-      for (int r = 0; r < ROUTER_ROWS; ++r) {
-        const uint4 xv = x[r][i];
-        const uint32_t xr[4] = {xv.x, xv.y, xv.z, xv.w};
+        for (int e = 0; e < ROUTER_EXPERTS; ++e) wv[b][e] = i < n ? __ldg(w + (size_t)e * n + i) : make_uint4(0u, 0u, 0u, 0u);   // rows behind the last expert are zero
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 p = unpack2_act(xr[j], a.fmt);
+        for (int r = 0; r < ROUTER_ROWS; ++r) xv[b][r] = i < n ? x[r][i] : make_uint4(0u, 0u, 0u, 0u);
+      }
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t wr[4] = {wv[e].x, wv[e].y, wv[e].z, wv[e].w};
-            const float2 q = unpack2_act(wr[j], a.fmt);
-            d[r][e] = fmaf(p.x, q.x, d[r][e]);
-            d[r][e] = fmaf(p.y, q.y, d[r][e]);
+      for (int b = 0; b < AT_ONCE; ++b) {
+        if (i0 + 32 * b >= n) break;
+#pragma unroll
+        for (int r = 0; r < ROUTER_ROWS; ++r) {
+          const uint32_t xr[4] = {xv[b][r].x, xv[b][r].y, xv[b][r].z, xv[b][r].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 p = unpack2_act(xr[j], a.fmt);
+#pragma unroll
+            for (int e = 0; e < ROUTER_EXPERTS; ++e) {
+              const uint32_t wr[4] = {wv[b][e].x, wv[b][e].y, wv[b][e].z, wv[b][e].w};
+              const float2 q = unpack2_act(wr[j], a.fmt);
+              d[r][e] = fmaf(p.x, q.x, d[r][e]);
+              d[r][e] = fmaf(p.y, q.y, d[r][e]);
+            }
           }
         }
       }
@@ -127,7 +139,7 @@ moe_router_kernel(MoeArgs a) {
 #pragma unroll
     for (int r = 0; r < ROUTER_ROWS; ++r)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < ROUTER_EXPERTS; ++e) {
         d[r][e] = warp_sum(d[r][e]);
         if (lane == 0 && e0 + e < a.experts) s_z[r][e0 + e] = d[r][e];
       }
@@ -153,20 +165,35 @@ moe_router_kernel(MoeArgs a) {
 
 // One CTA per row.  Every CTA takes the running sum over the experts' padded counts for itself; the first one also
 // lists the tiles and clears the padding slots' weights.
+// Everything a row needs is requested ahead of the sums, which cost two barriers: 9.0 -> 7.9 us at 31 rows.
 constexpr int SCATTER_THREADS = 128;
 __global__ void __launch_bounds__(SCATTER_THREADS)
 moe_scatter_kernel(MoeArgs a) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ int s_first[MOE_MAX_EXPERTS + 1];
+  __shared__ int s_first[MOE_MAX_EXPERTS + 1], s_n[MOE_MAX_EXPERTS];
   __shared__ int s_slot[MOE_MAX_TOP];
   __shared__ int s_warp[2 * SCATTER_THREADS / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // this row's choices, on their way while the counts are added up
+  const int row = blockIdx.x;
+  const size_t at = (size_t)row * a.top + tid;
+  const int my_expert = tid < a.top ? a.expert[at] : 0, my_rank = tid < a.top ? a.rank[at] : 0;
+  const float my_weight = tid < a.top ? a.weight[at] : 0.f;
+  const size_t bytes = (size_t)a.pitch * act_bytes(a.fmt);
+  const int pieces = (int)(bytes / 16);
+  const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(a.xn) + row * bytes);
+  uint4 ahead[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (tid + i * SCATTER_THREADS < pieces) ahead[i] = src[tid + i * SCATTER_THREADS];
   int incl[2], padded[2];                                // experts tid and tid + 128
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int e = tid + i * SCATTER_THREADS;
-    padded[i] = e < a.experts ? (a.count[e] + a.gran - 1) / a.gran * a.gran : 0;
+    const int count = e < a.experts ? a.count[e] : 0;
+    s_n[e] = count;
+    padded[i] = (count + a.gran - 1) / a.gran * a.gran;
     int v = padded[i];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -186,29 +213,28 @@ moe_scatter_kernel(MoeArgs a) {
     if (e == MOE_MAX_EXPERTS - 1) s_first[MOE_MAX_EXPERTS] = before + incl[i];
   }
   __syncthreads();
-  const int row = blockIdx.x;
   if (row == 0) {
     for (int e = warp; e < a.experts; e += SCATTER_THREADS / 32) {
-      const int first = s_first[e], n = a.count[e], end = (n + a.gran - 1) / a.gran * a.gran;
+      const int first = s_first[e], n = s_n[e], end = (n + a.gran - 1) / a.gran * a.gran;
       for (int t = lane * 128; t < end; t += 32 * 128) a.tile_expert[(first + t) >> 7] = e;
       for (int i = n + lane; i < end; i += 32) a.slot_weight[first + i] = 0.f;
     }
     if (tid == 0) *a.n_tiles = s_first[MOE_MAX_EXPERTS] >> 7;
   }
   if (tid < a.top) {
-    const size_t at = (size_t)row * a.top + tid;
-    const int slot = s_first[a.expert[at]] + a.rank[at];
+    const int slot = s_first[my_expert] + my_rank;
     s_slot[tid] = slot;
     a.slot[at] = slot;
-    a.slot_weight[slot] = a.weight[at];
+    a.slot_weight[slot] = my_weight;
   }
   __syncthreads();
-  const size_t bytes = (size_t)a.pitch * act_bytes(a.fmt);
-  const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(a.xn) + row * bytes);
-  for (int i = tid; i < (int)(bytes / 16); i += SCATTER_THREADS) {
-    const uint4 v = src[i];
+  auto spread = [&](int i, uint4 v) {
     for (int k = 0; k < a.top; ++k) reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(a.xs) + s_slot[k] * bytes)[i] = v;
-  }
+  };
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (tid + i * SCATTER_THREADS < pieces) spread(tid + i * SCATTER_THREADS, ahead[i]);
+  for (int i = tid + 2 * SCATTER_THREADS; i < pieces; i += SCATTER_THREADS) spread(i, src[i]);
 }
 
 }  // namespace
