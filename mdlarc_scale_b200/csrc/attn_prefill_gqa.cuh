@@ -29,6 +29,7 @@ struct AttnPrefillGqaArgs {
   int rotp, rot_panels, rot_panel;
   float scale;
   int act_f16;
+  int* next;                   // item counter: 0, and 0 again when the launch is done; one launch at a time
   int* err;
 };
 

@@ -821,7 +821,7 @@ int lm_latent(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
       a.qblock_row0 = pa.d_qblock_row0 + q0; a.qblock_rows = pa.d_qblock_rows + q0; a.kv0 = pa.d_qblock_kv0 + q0; a.n_qblocks = nq;
       a.sink = d.sink ? L.sink : nullptr; a.n_rows = R.n; a.n_heads = a.n_kv = L.hp; a.dimp = L.dimp; a.vdimp = L.vdimp; a.t_max = T;
       a.n_seqs = B; a.window = d.window; a.kv_rows = nt * 128; a.kv_pitch = L.n_expand; a.v_col = L.hp * L.dimp; a.k_rot = ls->k[l];
-      a.rotp = L.rotp; a.rot_panels = L.panels(); a.rot_panel = L.kvp / 64; a.scale = d.scale; a.act_f16 = m.fmt; a.err = s->eng->d_err;
+      a.rotp = L.rotp; a.rot_panels = L.panels(); a.rot_panel = L.kvp / 64; a.scale = d.scale; a.act_f16 = m.fmt; a.next = ls->st.n_finished + 1; a.err = s->eng->d_err;
       CKL(arcb_launch_attn_prefill_gqa(a, stream), "prefill attention");
     }
   } else {
@@ -972,7 +972,7 @@ int lm_mixer(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
     a.out = ls->mix; a.seq = R.seq; a.kv_count = R.kv_len; a.qblock_row0 = R.pa->d_qblock_row0; a.qblock_rows = R.pa->d_qblock_rows;
     a.sink = d.sink ? L.sink : nullptr; a.n_qblocks = R.pa->n_qblocks; a.n_rows = R.n; a.n_heads = d.heads; a.n_kv = d.kv_heads;
     a.dimp = L.dimp; a.vdimp = L.vdimp; a.t_max = T; a.n_seqs = B; a.scale = d.scale; a.act_f16 = m.fmt; a.err = s->eng->d_err;
-    a.window = d.window;
+    a.window = d.window; a.next = ls->st.n_finished + 1;
     CKL(arcb_launch_attn_prefill_gqa(a, stream), "prefill attention");
   } else {
     AttnGqaArgs a{};
@@ -1112,6 +1112,7 @@ int lm_prefill(arcb_session* s, const arcb_prefill_args* a, cudaStream_t stream)
   if (a->n_qblocks > 0 && (!a->d_qblock_row0 || !a->d_qblock_rows)) return arcb_fail(ARCB_E_ARG, "null query blocks");
   int r = lm_clear(s, stream);
   if (r) return r;
+  CK(cudaMemsetAsync(ls->st.n_finished + 1, 0, 4, stream));   // the prefill attention's item counter, should a launch have failed
   CKL(arcb_launch_lm_embed(lm_embed_args(s, a->n_tokens, a->d_token_ids), stream), "embed");
   if (a->n_groups > 0 && (!a->h_group_qblock || !a->h_group_tile || !a->d_tile_src || !a->d_qblock_kv0 || a->n_qblocks <= 0))
     return arcb_fail(ARCB_E_ARG, "null group arrays");
