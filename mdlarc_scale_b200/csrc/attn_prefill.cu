@@ -118,16 +118,17 @@ __device__ __forceinline__ void flash_tma_producer(const CUtensorMap* tmap_q, co
   }
 }
 
-// ---- MMA issuer of Q tile x (one thread): S(0), S(1), PV(0), S(2), PV(1), ... each behind a blocking
+// ---- MMA issuer of Q tile x (one warp, an elected lane of it issues): S(0), S(1), PV(0), S(2), PV(1), ... each behind a blocking
 // wait on the one barrier it needs ----
 __device__ __forceinline__ void flash_mma_issuer(int x, const Bars& B, uint32_t q_smem, uint32_t kv_smem,
                                                  uint32_t tmem_base, int n_a, int n_b, uint32_t idesc_qk,
                                                  uint32_t idesc_pv, int* err) {
   const int n_x = x ? n_b : n_a;
   const int n_tiles = max(n_a, n_b);
+  const uint32_t el = elect_one();
   bool ok = true;
   auto wait_or_flag = [&](uint32_t bar, uint32_t parity, int code) {
-    if (ok && !mbar_wait_bounded(bar, parity)) {
+    if (ok && !__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity))) {
       arcb_set_error(err, code);
       ok = false;
     }
@@ -138,8 +139,8 @@ __device__ __forceinline__ void flash_mma_issuer(int x, const Bars& B, uint32_t 
     const uint64_t dk = umma_desc_k_sw128(kv_smem + (j % KV_STAGES) * 2 * KV_TILE_BYTES);
 #pragma unroll
     for (int ks = 0; ks < HD / 16; ++ks)
-      umma_f16(tmem_base + x * 128, dq + 2 * ks, dk + 2 * ks, idesc_qk, ks ? 1u : 0u);
-    umma_commit(B.s[x]);
+      umma_f16_if(el, tmem_base + x * 128, dq + 2 * ks, dk + 2 * ks, idesc_qk, ks ? 1u : 0u);
+    umma_commit_if(el, B.s[x]);
   };
   auto mma_o = [&](int j) {  // O_x (+)= P_x V(j); then this tile is done with K/V stage j
     const uint64_t dv = umma_desc_mn_sw128(kv_smem + (j % KV_STAGES) * 2 * KV_TILE_BYTES + KV_TILE_BYTES);
@@ -148,11 +149,11 @@ __device__ __forceinline__ void flash_mma_issuer(int x, const Bars& B, uint32_t 
     for (int ks = 0; ks < BKV / 16; ++ks) {
       // A = P_x from tensor memory: 16 keys = 8 columns of packed 16-bit pairs;
       // 16 keys = 16 rows of 128 bytes = 2048 bytes further into the V tile
-      umma_f16_ts(d_o, tmem_base + TMEM_P + x * 64 + ks * 8, dv + (uint64_t)(ks * (2048 >> 4)), idesc_pv,
+      umma_f16_ts_if(el, d_o, tmem_base + TMEM_P + x * 64 + ks * 8, dv + (uint64_t)(ks * (2048 >> 4)), idesc_pv,
                   (j | ks) ? 1u : 0u);
     }
-    umma_commit(B.o[x]);
-    umma_commit(B.kv_empty + 8 * (j % KV_STAGES));
+    umma_commit_if(el, B.o[x]);
+    umma_commit_if(el, B.kv_empty + 8 * (j % KV_STAGES));
   };
   for (int j = 0; ok && j < n_x; ++j) {
     wait_or_flag(B.kv_full + 8 * (j % KV_STAGES), (j / KV_STAGES) & 1, ARCB_DEV_WAIT_TIMEOUT_TMA);   // K(j) has landed
@@ -178,7 +179,7 @@ __device__ __forceinline__ void flash_mma_issuer(int x, const Bars& B, uint32_t 
   // they have landed, in order, so that each arrival counts for the right use of the stage
   for (int j = n_x; ok && j < n_tiles; ++j) {
     wait_or_flag(B.kv_full + 8 * (j % KV_STAGES), (j / KV_STAGES) & 1, ARCB_DEV_WAIT_TIMEOUT_TMA);
-    if (ok) mbar_arrive(B.kv_empty + 8 * (j % KV_STAGES));
+    if (ok && el) mbar_arrive(B.kv_empty + 8 * (j % KV_STAGES));
   }
 }
 
@@ -221,7 +222,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   // the barriers above end at byte 136 of this region; the TMEM-address slot sits well clear of them
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // known to be the same in a warp
   const int blk = blockIdx.x, h = blockIdx.y;
   const int row0 = a.qblock_row0[blk];
   const int rows = a.qblock_rows[blk];  // 1..256
@@ -263,17 +264,17 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const int cnt_a = max(max(s_max_cnt[0], s_max_cnt[1]), max(s_max_cnt[2], s_max_cnt[3]));
   const int cnt_b = max(max(s_max_cnt[4], s_max_cnt[5]), max(s_max_cnt[6], s_max_cnt[7]));
-  const int n_a = (cnt_a + BKV - 1) / BKV;
-  const int n_b = (cnt_b + BKV - 1) / BKV;
+  const int n_a = __shfl_sync(0xffffffffu, (cnt_a + BKV - 1) / BKV, 0);
+  const int n_b = __shfl_sync(0xffffffffu, (cnt_b + BKV - 1) / BKV, 0);
   const int n_tiles = max(n_a, n_b);
 
   if (warp == 0) {
     if (lane == 0 && n_tiles > 0) flash_tma_producer(&tmap_q, &tmap_k, &tmap_v, B, q_smem, kv_smem, h, row0, rows, kv0, n_tiles, a.err);
   } else if (warp == 1 || warp == 2) {
-    if (lane == 0 && n_tiles > 0)
+    if (n_tiles > 0)
       flash_mma_issuer(warp - 1, B, q_smem, kv_smem, tmem_base, n_a, n_b, idesc_qk, idesc_pv, a.err);
   } else {
     // ---- softmax / output threads: one query row each ----
@@ -632,13 +633,15 @@ __device__ __forceinline__ void flash_items_producer(const CUtensorMap* tmap_q, 
   }
 }
 
-// One thread: the products of Q tile x, as flash_mma_issuer, over all items.
+// One warp, an elected lane of it issues (operands then stay in uniform registers; one thread alone took
+// longer to issue a tile's products than they run): the products of Q tile x, as flash_mma_issuer, over all items.
 __device__ __forceinline__ void flash_items_issuer(int x, const Bars& B, const ItemBars& I, uint32_t q_smem, uint32_t kv_smem,
                                                    uint32_t tmem_base, const FlashItem* s_item, uint32_t idesc_qk,
                                                    uint32_t idesc_pv, int* err) {
+  const uint32_t el = elect_one();
   bool ok = true;
   auto wait_or_flag = [&](uint32_t bar, uint32_t parity, int code) {
-    if (ok && !mbar_wait_bounded(bar, parity)) {
+    if (ok && !__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity))) {
       arcb_set_error(err, code);
       ok = false;
     }
@@ -647,24 +650,27 @@ __device__ __forceinline__ void flash_items_issuer(int x, const Bars& B, const I
   for (int k = 0;; ++k) {
     const int par = k & 1;
     wait_or_flag(I.full + 8 * par, (k >> 1) & 1, ARCB_DEV_WAIT_TIMEOUT_TMA);
-    if (!ok || s_item[par].rows < 0) return;
-    const int n_a = s_item[par].n_a, n_b = s_item[par].n_b, n_x = x ? n_b : n_a, n_tiles = max(n_a, n_b);
+    if (!ok) return;
+    auto field = [&](int v) { return __shfl_sync(0xffffffffu, v, 0); };
+    const int rows = field(s_item[par].rows), n_a = field(s_item[par].n_a), n_b = field(s_item[par].n_b);
+    if (rows < 0) return;
+    const int n_x = x ? n_b : n_a, n_tiles = max(n_a, n_b);
     const uint64_t dq = umma_desc_k_sw128(q_smem + (par * 2 + x) * Q_BYTES);
     auto mma_s = [&](int j) {  // S_x = Q_x K(j)^T
       const uint64_t dk = umma_desc_k_sw128(kv_smem + ((tile + j) % KV_STAGES) * 2 * KV_TILE_BYTES);
 #pragma unroll
-      for (int ks = 0; ks < HD / 16; ++ks) umma_f16(tmem_base + x * 128, dq + 2 * ks, dk + 2 * ks, idesc_qk, ks ? 1u : 0u);
-      umma_commit(B.s[x]);
-      if (j == n_x - 1) umma_commit(I.empty + 8 * par);
+      for (int ks = 0; ks < HD / 16; ++ks) umma_f16_if(el, tmem_base + x * 128, dq + 2 * ks, dk + 2 * ks, idesc_qk, ks ? 1u : 0u);
+      umma_commit_if(el, B.s[x]);
+      if (j == n_x - 1) umma_commit_if(el, I.empty + 8 * par);
     };
     auto mma_o = [&](int j) {  // O_x (+)= P_x V(j); then this tile is done with K/V stage j
       const int s = (tile + j) % KV_STAGES;
       const uint64_t dv = umma_desc_mn_sw128(kv_smem + s * 2 * KV_TILE_BYTES + KV_TILE_BYTES);
 #pragma unroll
       for (int ks = 0; ks < BKV / 16; ++ks)
-        umma_f16_ts(tmem_base + 256 + x * 64, tmem_base + TMEM_P + x * 64 + ks * 8, dv + (uint64_t)(ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
-      umma_commit(B.o[x]);
-      umma_commit(B.kv_empty + 8 * s);
+        umma_f16_ts_if(el, tmem_base + 256 + x * 64, tmem_base + TMEM_P + x * 64 + ks * 8, dv + (uint64_t)(ks * (2048 >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
+      umma_commit_if(el, B.o[x]);
+      umma_commit_if(el, B.kv_empty + 8 * s);
     };
     for (int j = 0; j < n_x; ++j) {
       wait_or_flag(B.kv_full + 8 * ((tile + j) % KV_STAGES), ((tile + j) / KV_STAGES) & 1, ARCB_DEV_WAIT_TIMEOUT_TMA);
@@ -685,13 +691,13 @@ __device__ __forceinline__ void flash_items_issuer(int x, const Bars& B, const I
       tc_fence_after();
       mma_o(n_x - 1);
     } else {
-      mbar_arrive(I.empty + 8 * par);
+      if (el) mbar_arrive(I.empty + 8 * par);
     }
     // stages that only the other Q tile uses go back as soon as they have landed, in order
     for (int j = n_x; j < n_tiles; ++j) {
       wait_or_flag(B.kv_full + 8 * ((tile + j) % KV_STAGES), ((tile + j) / KV_STAGES) & 1, ARCB_DEV_WAIT_TIMEOUT_TMA);
       if (!ok) return;
-      mbar_arrive(B.kv_empty + 8 * ((tile + j) % KV_STAGES));
+      if (el) mbar_arrive(B.kv_empty + 8 * ((tile + j) % KV_STAGES));
     }
     done += n_x;
     tile += n_tiles;
@@ -733,7 +739,7 @@ attn_prefill_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   const uint32_t xbar0 = B.s[0] + 64;      // 8 barriers: one per (Q tile, lane quarter) pair of warps
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // known to be the same in a warp
 
   const int wg = (warp >> 2) - 1;          // softmax warpgroup 0..3 (helpers: -1)
   const int grp = wg >> 1;                 // Q tile
@@ -770,14 +776,14 @@ attn_prefill_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp < 4) {
     reg_dealloc_32();
     if (warp == 0) {
       flash_items_producer(&tmap_q, &tmap_k, &tmap_v, B, I, q_smem, kv_smem, a, first, s_item, s_cnt);
     } else if (warp <= 2) {
-      if (lane == 0) flash_items_issuer(warp - 1, B, I, q_smem, kv_smem, tmem_base, s_item, idesc_qk, idesc_pv, a.err);
+      flash_items_issuer(warp - 1, B, I, q_smem, kv_smem, tmem_base, s_item, idesc_qk, idesc_pv, a.err);
     }
   } else {
     reg_alloc_112();
