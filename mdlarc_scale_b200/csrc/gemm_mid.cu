@@ -41,7 +41,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   const uint32_t bar_acc = bars + 16 * sh.stages;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + (bar_acc + 8 - base));
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // known to be the same in a warp
   const int rank = blockIdx.x % sh.splits, n0 = blockIdx.x / sh.splits * 128;
   const int kb0 = rank * num_k / sh.splits, kb1 = (rank + 1) * num_k / sh.splits;
   const uint32_t tmem_cols = sh.rows <= 128 ? 128 : 256;
@@ -69,7 +69,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   pdl_wait();
 
   if (warp == 0 && lane == 0) {
@@ -83,10 +83,12 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       fetch(kb0 + i, s);
       if (++s == sh.stages) { s = 0; turn ^= 1; }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
+    // the whole warp, an elected lane issues: operands stay in uniform registers
+    const uint32_t el = elect_one();
     bool ok = true;
     for (int i = 0, s = 0, turn = 0; i < kb1 - kb0; ++i) {
-      if (!mbar_wait_bounded(bars + 8 * s, turn)) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(bars + 8 * s, turn))) {
         arcb_set_error(ep.err, ARCB_DEV_WAIT_TIMEOUT_TMA);
         *abort_flag = 1;
         ok = false;
@@ -95,11 +97,11 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       tc_fence_after();
       const uint64_t dw = umma_desc_k_sw128(base + s * stage_bytes), da = umma_desc_k_sw128(base + s * stage_bytes + GM_W_BYTES);
 #pragma unroll
-      for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem, dw + 2 * k4, da + 2 * k4, idesc, (i | k4) ? 1u : 0u);
-      umma_commit(bars + 8 * (sh.stages + s));
+      for (int k4 = 0; k4 < 4; ++k4) umma_f16_if(el, tmem, dw + 2 * k4, da + 2 * k4, idesc, (i | k4) ? 1u : 0u);
+      umma_commit_if(el, bars + 8 * (sh.stages + s));
       if (++s == sh.stages) { s = 0; turn ^= 1; }
     }
-    if (ok) umma_commit(bar_acc);
+    if (ok) umma_commit_if(el, bar_acc);
   }
   __syncwarp();
 
