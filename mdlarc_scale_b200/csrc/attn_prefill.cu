@@ -544,7 +544,8 @@ constexpr int SPLIT_SMEM_BYTES = SMEM_BYTES + 2 * Q_BYTES;   // Q tiles of two i
 // (all heads' most expensive blocks first) does not keep keys in L2, what keeps them there is not even.
 // B200, us a launch, an item a CTA / this: 262 prompts of 250 tokens, 20 heads 543 / 370, 150 prompts of about 360
 // tokens 431 / 311, 20 of 2 k tokens 700 / 635, 4 of 10 k tokens 1740 / 1720; 37 prompts of 64 to 500 tokens, 12 heads 92.5 / 73.6;
-// 60 items in all (fewer than SMs) 26 / 27.
+// 60 items in all (fewer than SMs) 26 / 27.  Products issued by a warp instead of a thread: 37 prompts 74 -> 64, a part of 1024 prompts of
+// about 250 tokens 367 -> 300, 4 of 10 k tokens 1670 -> 1610 (another box than the figures before).
 struct FlashItem { int row0, rows, n_a, n_b, head; };    // rows < 0: the list has ended
 
 // Barriers of the items: Q full / empty by item parity.  Empty: two issuers and the 16 softmax warps, which also read the
