@@ -1,0 +1,45 @@
+"""Recurrence of 32-bit models with 64-wide heads by chunks of 64 tokens, against the oracle in 64 bits and the recurrence
+token by token."""
+import pytest
+import torch
+
+from gpu_util import have_b200
+from mdlarc_scale_b200 import registry
+from mdlarc_scale_b200.layered import Segment
+from oracle import vodavik as vo
+from vodavik_util import config, mlstm, oracle_logits, rel_error, tokens
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_b200(), reason="needs a B200")]
+# A chunk's result is a sum of at most 64 + 64 products of 64 terms, each rounded to 2^-24 of the largest: below 2^-24 * 2 * 64,
+# 8e-6 of the layer's output; two layers and the projections around them leave 3e-5, what every 32-bit result of these
+# models is held to.
+TOL = 3e-5
+
+
+def portions(eng, toks, sizes):
+    s = eng.new_session(3, len(toks), 1, 4096, stop_on_end=False)
+    other, slot, at, rows = s.acquire(), s.acquire(), 0, []
+    for n in sizes:
+        # beside another sequence of the same lengths, so that a call holds more than one segment
+        seg = [Segment(k, toks[at:at + n], list(range(n))) for k in (slot, other)]
+        rows.append(s.step(seg)[0])
+        at += n
+    s.poll()
+    s.close()
+    return torch.cat(rows)
+
+
+@pytest.mark.parametrize("sizes", [[1], [2], [63], [64], [65], [128], [130], [64, 64], [1, 64, 1], [65, 63, 2], [200, 131]], ids=str)
+@pytest.mark.parametrize("heads,dim,vdim", [(3, 64, 64), (2, 40, 56)])
+@pytest.mark.parametrize("bias", [-9.0, 0.0, 9.0])
+def test_chunks(sizes, heads, dim, vdim, bias):
+    """Portions that end on, ahead of and behind a chunk, from an empty and from a carried state; forget gates that drop
+    everything at once, the usual ones, and ones that keep everything."""
+    cfg = config(160, 200, [mlstm(heads, dim, vdim), mlstm(heads, dim, vdim)])
+    w = vo.random_weights(cfg, 7)
+    for name in [n for n in w if n.endswith(".mix.f.b")]:
+        w[name] = w[name] + bias
+    toks = tokens(cfg, sum(sizes), 3)
+    got = portions(registry.build_engine(cfg, w, "cuda:0", "f32"), toks, sizes)
+    assert rel_error(got, oracle_logits(cfg, w, toks)) < TOL
+    assert rel_error(got, portions(registry.build_engine(cfg, w, "cuda:0", "f32", mlstm_path="step"), toks, sizes)) < 2 * TOL
