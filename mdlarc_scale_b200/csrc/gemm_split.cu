@@ -6,8 +6,9 @@
 // do not round to nearest, so sums stay short there: the leading products of 128 columns have an accumulator of their own, the five
 // smaller ones another, and both are added in registers to the running 32-bit sum.  A row's order of addition depends on K alone.
 // Errors against 64 bits, this / multiply-adds in 32 bits (gemm_simt_wide_kernel): K 1280 1.4e-7 / 6.4e-7 of the result's norm, K 5120
-// 2.0e-7 / 1.3e-6, factors spread over e^+-3 1.9e-7 / 6.4e-7; largest of an element 6e-8 / 4e-7 of its sum of magnitudes.  Values without
-// such pieces (infinities, NaN, beyond the largest bf16) send a tile to multiply-adds; below 2^-110 the pieces lose bits as subnormals.
+// 2.0e-7 / 1.3e-6, factors spread over e^+-3 1.9e-7 / 6.4e-7; largest of an element 6e-8 / 4e-7 of its sum of magnitudes.  The sums of a
+// row of A or W with values that have no such pieces (infinities, NaN, beyond the largest bf16) are multiply-adds instead, those of the
+// rows beside it stay as they are; below 2^-110 the pieces lose bits as subnormals.
 //
 // What bounds it: 24 instructions of 128 x 128 x 16 for 64 columns (12 where the weights are bf16 values, as those of a checkpoint
 // in 16 bits are: their other pieces are zeros), and next to them the splitting of 16 k values by 16 warps, 6 to 8 operations each, on
@@ -53,6 +54,80 @@ __device__ __forceinline__ void tmem_wait_ld_dep16(uint32_t (&r)[16]) {
                  "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                :
                : "memory");
+}
+
+// Sums of a tile that meet a value without pieces, by multiply-adds in order of K as gemm_simt_wide_kernel takes them: those of such a row
+// of A or of W.  All others stay as they are, so that what a neighbour holds changes no bit of a row.  `base_ptr`: the tile's
+// sums, then (the operands are done with) blocks of 32 columns of both operands.
+__device__ __noinline__ void redo_without_pieces(uint8_t* base_ptr, const float* A, const float* W, int K, size_t lda, long long a_row0,
+                                                 long long a_rows, size_t w_row0) {
+  constexpr int PA = 33, PW = 36;
+  float* part = reinterpret_cast<float*>(base_ptr);
+  float* sa = part + 128 * GS_PITCH;
+  float* sw = sa + 128 * PA;
+  volatile int* flag = reinterpret_cast<volatile int*>(sw + 128 * PW);      // rows of A, then of W
+  static_assert((128 * (GS_PITCH + PA + PW) + 256) * 4 <= 2 * GS_STAGE && 128 * PA % 4 == 0, "shared memory");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid < 256) flag[tid] = 0;
+  __syncthreads();
+  // 512 threads: four values of rows tid / 8 and tid / 8 + 64 of both operands
+  const int q = (tid & 7) * 4;
+  auto quad = [&](bool of_w, int row, int k) {
+    if (of_w) return __ldg(reinterpret_cast<const float4*>(W + (w_row0 + row) * K + k));
+    return a_row0 + row < a_rows ? __ldcg(reinterpret_cast<const float4*>(A + (size_t)(a_row0 + row) * lda + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  if (warp < GS_WARPS)
+    for (int i = 0; i < 4; ++i) {
+      const int row = (tid >> 3) + 64 * (i & 1);
+      uint64_t odd = 0ull;
+      for (int k = q; k < K; k += 32) {
+        const float4 v = quad(i >> 1, row, k);
+        uint32_t p[3];
+        split2(v.x, v.y, p[0], p[1], p[2], odd);
+        split2(v.z, v.w, p[0], p[1], p[2], odd);
+      }
+      float ox, oy;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(ox), "=f"(oy) : "l"(odd));
+      if (!(ox == 0.f && oy == 0.f)) flag[128 * (i >> 1) + row] = 1;
+    }
+  __syncthreads();
+  const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * GS_COLS;
+  uint32_t cols = 0;
+  bool row = false;
+  if (warp < GS_WARPS) {
+    cols = __ballot_sync(0xffffffffu, flag[128 + c0 + lane] != 0);
+    row = flag[r] != 0;
+  }
+  const bool any = cols || __any_sync(0xffffffffu, row);
+  float acc[GS_COLS];
+#pragma unroll
+  for (int i = 0; i < GS_COLS; ++i) acc[i] = 0.f;
+  for (int k0 = 0; k0 < K; k0 += 32) {
+    if (warp < GS_WARPS)
+      for (int i = 0; i < 2; ++i) {
+        const int rr = (tid >> 3) + 64 * i;
+        const float4 a = quad(false, rr, k0 + q);
+        float* to = sa + rr * PA + q;
+        to[0] = a.x; to[1] = a.y; to[2] = a.z; to[3] = a.w;
+        *reinterpret_cast<float4*>(sw + rr * PW + q) = quad(true, rr, k0 + q);
+      }
+    __syncthreads();
+    if (any)
+      for (int k = 0; k < 32; k += 4) {
+        const float a[4] = {sa[r * PA + k], sa[r * PA + k + 1], sa[r * PA + k + 2], sa[r * PA + k + 3]};
+#pragma unroll
+        for (int i = 0; i < GS_COLS; ++i) {
+          const float4 w = *reinterpret_cast<const float4*>(sw + (c0 + i) * PW + k);
+          acc[i] = fmaf(a[3], w.w, fmaf(a[2], w.z, fmaf(a[1], w.y, fmaf(a[0], w.x, acc[i]))));
+        }
+      }
+    __syncthreads();
+  }
+  if (any)
+#pragma unroll
+    for (int i = 0; i < GS_COLS; ++i)
+      if (row || (cols >> i & 1)) part[r * GS_PITCH + c0 + i] = acc[i];
+  __syncthreads();
 }
 
 template <int MODE>
@@ -227,21 +302,7 @@ gemm_split_kernel(const float* A, const float* W, GemmEpilogue ep, int K, uint32
 #pragma unroll
     for (int i = 0; i < GS_COLS; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
   }
-  if (__syncthreads_or(odd)) {
-    // values without pieces: the tile's sums by multiply-adds, as they come
-    if (warp < GS_WARPS) {
-      const int r = (warp & 3) * 32 + lane;
-      const bool in = a_row0 + r < a_rows;
-      const float* a = A + (size_t)(in ? a_row0 + r : a_row0) * lda;
-      for (int c = (warp >> 2) * GS_COLS; c < ((warp >> 2) + 1) * GS_COLS; ++c) {
-        const float* w = W + (w_row0 + c) * K;
-        float sum = 0.f;
-        for (int k = 0; in && k < K; ++k) sum = fmaf(a[k], __ldg(w + k), sum);
-        part[r * GS_PITCH + c] = sum;
-      }
-    }
-    __syncthreads();
-  }
+  if (__syncthreads_or(odd)) redo_without_pieces(base_ptr, A, W, K, lda, a_row0, a_rows, w_row0);
   if (warp < GS_WARPS) {
     constexpr bool PAIRED = MODE == EPI_GLU;
     constexpr int STEP = (PAIRED ? 2 : 1) * GS_WARPS, U = 4;

@@ -57,3 +57,27 @@ def test_values_without_pieces(value, where):
     assert torch.equal(got[hit].nan_to_num(), plain[hit].nan_to_num())
     ref = a.double() @ w.double().T
     assert ((got - ref).abs()[~hit] <= (a.double().abs() @ w.double().abs().T)[~hit] * 2.0 ** -19).all()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
+@pytest.mark.parametrize("M,N,K", [(128, 128, 64), (200, 256, 192), (70, 128, 1280)])
+def test_rows_beside_such_values_keep_their_bits(M, N, K, value):
+    a, w = operands(M, N, K, "plain")
+    clean = product(a, w)
+    for row, col in ((0, None), (M - 1, None), (M // 2, N - 1), (None, 0), (None, 77)):
+        b, v = a.clone(), w.clone()
+        if row is not None:
+            b[row, K - 1] = value
+        if col is not None:
+            v[col, 0] = value
+        keep = torch.ones_like(clean, dtype=torch.bool)
+        if row is not None:
+            keep[row] = False
+        if col is not None:
+            keep[:, col] = False
+        got, plain = product(b, v), product(b, v, _lib.GEMM_SIMT)
+        assert torch.equal(got[keep], clean[keep])
+        assert torch.equal(got[~keep].nan_to_num(), plain[~keep].nan_to_num())
+        assert torch.equal(got.isnan(), plain.isnan()) and torch.equal(got.isinf(), plain.isinf())
+    b = torch.full_like(a, value)                # all of them
+    assert torch.equal(product(b, w).nan_to_num(), product(b, w, _lib.GEMM_SIMT).nan_to_num())
