@@ -33,7 +33,8 @@ struct GluArgs {
 
 // Products whose rows or columns belong to groups.  All fields zero: one plain product.
 //   rows    : tile_src[t] is the A row of output rows [128 t, 128 t + 128) (null: 128 t); tile_group[t] picks the
-//             rows [group * group_rows, ...) of W; n_tiles (device) is the number of tiles that hold anything
+//             rows [group * group_rows, ...) of W; n_tiles (device) is the number of tiles that hold anything; tile_rows[t], 32-bit
+//             products only: rows of A ahead of the padding, which is read as zeros (null: no padding)
 //   panels  : A is cut into panels of 64 columns, [sequence][panels][panel_rows][64]; tile_src then counts rows as
 //             sequence * panel_rows + row
 //   columns : columns [c n_group, (c + 1) n_group) read A columns [c a_group, c a_group + K)
@@ -41,6 +42,7 @@ struct GroupArgs {
   const int* tile_src;
   const int* tile_group;
   const int* n_tiles;
+  const int* tile_rows;
   int group_rows;
   long long w_rows;      // rows of W in all groups
   int n_group, a_group;

@@ -59,8 +59,8 @@ __device__ __forceinline__ void tmem_wait_ld_dep16(uint32_t (&r)[16]) {
 // Sums of a tile that meet a value without pieces, by multiply-adds in order of K as gemm_simt_wide_kernel takes them: those of such a row
 // of A or of W.  All others stay as they are, so that what a neighbour holds changes no bit of a row.  `base_ptr`: the tile's
 // sums, then (the operands are done with) blocks of 32 columns of both operands.
-__device__ __noinline__ void redo_without_pieces(uint8_t* base_ptr, const float* A, const float* W, int K, size_t lda, long long a_row0,
-                                                 long long a_rows, size_t w_row0) {
+__device__ __noinline__ void redo_without_pieces(uint8_t* base_ptr, const float* A, const float* W, int K, size_t lda, int a_row0, int rows_in,
+                                                 size_t w_row0) {
   constexpr int PA = 33, PW = 36;
   float* part = reinterpret_cast<float*>(base_ptr);
   float* sa = part + 128 * GS_PITCH;
@@ -74,7 +74,7 @@ __device__ __noinline__ void redo_without_pieces(uint8_t* base_ptr, const float*
   const int q = (tid & 7) * 4;
   auto quad = [&](bool of_w, int row, int k) {
     if (of_w) return __ldg(reinterpret_cast<const float4*>(W + (w_row0 + row) * K + k));
-    return a_row0 + row < a_rows ? __ldcg(reinterpret_cast<const float4*>(A + (size_t)(a_row0 + row) * lda + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return row < rows_in ? __ldcg(reinterpret_cast<const float4*>(A + (size_t)(a_row0 + row) * lda + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   if (warp < GS_WARPS)
     for (int i = 0; i < 4; ++i) {
@@ -167,7 +167,9 @@ gemm_split_kernel(const float* A, const float* W, GemmEpilogue ep, int K, uint32
   const uint32_t tmem = *tmem_slot;              // accumulators of chunk c at 256 (c & 1): leading products, smaller ones at + 128
 
   const int a_row0 = g.tile_src ? g.tile_src[blockIdx.y] : m0;
-  const long long a_rows = g.a_rows ? g.a_rows : ep.M;
+  int rows_in = (int)min(128ll, (g.a_rows ? g.a_rows : ep.M) - a_row0);      // rows of A in this tile, the others are zeros
+  // padding of a group is memory that nothing wrote: no part of it may choose how sums are taken
+  if (g.tile_rows) rows_in = min(rows_in, g.tile_rows[blockIdx.y]);
   const size_t lda = g.lda ? g.lda : K;
   const size_t w_row0 = (size_t)n0 + (g.tile_group ? (size_t)g.tile_group[blockIdx.y] * g.group_rows : 0);
   float* part = reinterpret_cast<float*>(base_ptr);
@@ -218,9 +220,9 @@ gemm_split_kernel(const float* A, const float* W, GemmEpilogue ep, int K, uint32
     auto fetch_a = [&](int b) {
 #pragma unroll
       for (int j = 0; j < GS_ITEMS; ++j) {
-        const long long row = a_row0 + r0 + 128 / GS_ITEMS * j;
-        const float4* src = reinterpret_cast<const float4*>(A + (size_t)row * lda + b * 64 + q * 8);
-        const bool in = row < a_rows;
+        const int row = r0 + 128 / GS_ITEMS * j;
+        const float4* src = reinterpret_cast<const float4*>(A + (size_t)(a_row0 + row) * lda + b * 64 + q * 8);
+        const bool in = row < rows_in;
         ra[j][0] = in ? __ldcg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
         ra[j][1] = in ? __ldcg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
@@ -302,7 +304,7 @@ gemm_split_kernel(const float* A, const float* W, GemmEpilogue ep, int K, uint32
 #pragma unroll
     for (int i = 0; i < GS_COLS; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
   }
-  if (__syncthreads_or(odd)) redo_without_pieces(base_ptr, A, W, K, lda, a_row0, a_rows, w_row0);
+  if (__syncthreads_or(odd)) redo_without_pieces(base_ptr, A, W, K, lda, a_row0, rows_in, w_row0);
   if (warp < GS_WARPS) {
     constexpr bool PAIRED = MODE == EPI_GLU;
     constexpr int STEP = (PAIRED ? 2 : 1) * GS_WARPS, U = 4;

@@ -234,7 +234,7 @@ LmWs lm_ws(const LayeredModel& m, int B, int P, int splits, int requested) {
   moe_sizes(m, (int)R, &w.max_slots, &w.max_rt, &ffp, &zp);
   w.moe_z = take(R * (size_t)zp * 4);
   w.moe_rows = take((size_t)w.max_rt * 4 * 4);               // expert, place, weight, slot
-  w.moe_slots = take(((size_t)w.max_slots + w.max_slots / 128 + 2) * 4);   // weights, experts of the tiles
+  w.moe_slots = take(((size_t)w.max_slots + 2 * (w.max_slots / 128) + 2) * 4);   // weights, experts and rows of the tiles
   w.moe_xs = take((size_t)w.max_slots * m.wp * m.es * (m.has_moe ? 1 : 0));
   w.moe_hid = take((size_t)w.max_slots * ffp * m.es);
   w.moe_out = take((size_t)w.max_slots * m.wp * m.es * (m.has_moe ? 1 : 0));
@@ -673,6 +673,7 @@ int lm_session_create(arcb_session* s) {
   mo.slot = mo.rank + 2 * (size_t)w.max_rt;
   mo.slot_weight = reinterpret_cast<float*>(base + w.moe_slots);
   mo.tile_expert = reinterpret_cast<int*>(mo.slot_weight + w.max_slots);
+  mo.tile_rows = mo.tile_expert + w.max_slots / 128;
   mo.xs = base + w.moe_xs;
   ls->gemm_scratch = reinterpret_cast<float*>(base + w.gscratch);
   ls->head_rows = w.head_rows;
@@ -904,11 +905,11 @@ int lm_mlp(arcb_session* s, int l, const Rows& R, cudaStream_t stream) {
   const int slots = arcb_moe_max_slots(R.n, d.experts, d.top, mo.gran), variant = mo.gran == 256 ? 2 : 1;
   GemmEpilogue ee = eu;
   ee.M = slots; ee.N = 2 * L.ffp; ee.out16 = ls->moe_hid; ee.glu.limit = d.glu_limit; ee.glu.row = mo.slot_weight;
-  ee.grp.tile_group = mo.tile_expert; ee.grp.n_tiles = mo.n_tiles; ee.grp.group_rows = 2 * L.ffp; ee.grp.w_rows = (long long)d.experts * 2 * L.ffp;
+  ee.grp.tile_group = mo.tile_expert; ee.grp.n_tiles = mo.n_tiles; ee.grp.tile_rows = mo.tile_rows; ee.grp.group_rows = 2 * L.ffp; ee.grp.w_rows = (long long)d.experts * 2 * L.ffp;
   CKL(lm_gemm(m, mo.xs, L.w_egu, ee, m.wp, stream, variant), "expert gate/up gemm");
   GemmEpilogue ed{};
   ed.mode = EPI_ACT; ed.M = slots; ed.N = m.wp; ed.out16 = ls->moe_out; ed.act_f16 = m.fmt; ed.err = s->eng->d_err;
-  ed.grp.tile_group = mo.tile_expert; ed.grp.n_tiles = mo.n_tiles; ed.grp.group_rows = m.wp; ed.grp.w_rows = (long long)d.experts * m.wp;
+  ed.grp.tile_group = mo.tile_expert; ed.grp.n_tiles = mo.n_tiles; ed.grp.tile_rows = mo.tile_rows; ed.grp.group_rows = m.wp; ed.grp.w_rows = (long long)d.experts * m.wp;
   CKL(lm_gemm(m, ls->moe_hid, L.w_edown, ed, L.ffp, stream, variant), "expert down gemm");
   if (L.sffp && step && ls->side && !arcb_pdl_enabled()) CK(cudaStreamWaitEvent(stream, ls->join, 0));
   return ARCB_OK;

@@ -216,7 +216,10 @@ moe_scatter_kernel(MoeArgs a) {
   if (row == 0) {
     for (int e = warp; e < a.experts; e += SCATTER_THREADS / 32) {
       const int first = s_first[e], n = s_n[e], end = (n + a.gran - 1) / a.gran * a.gran;
-      for (int t = lane * 128; t < end; t += 32 * 128) a.tile_expert[(first + t) >> 7] = e;
+      for (int t = lane * 128; t < end; t += 32 * 128) {
+        a.tile_expert[(first + t) >> 7] = e;
+        a.tile_rows[(first + t) >> 7] = min(max(n - t, 0), 128);
+      }
       for (int i = n + lane; i < end; i += 32) a.slot_weight[first + i] = 0.f;
     }
     if (tid == 0) *a.n_tiles = s_first[MOE_MAX_EXPERTS] >> 7;

@@ -19,6 +19,7 @@ struct MoeArgs {
   int* slot;               // [rows * top]
   float* slot_weight;      // [max_slots], 0 in padding slots
   int* tile_expert;        // [max_slots / 128] expert of every 128-slot tile
+  int* tile_rows;          // [max_slots / 128] slots of every tile that hold a row; the others are padding, which nothing writes
   int* n_tiles;            // 128-slot tiles in use
   const void* xn;          // [rows][pitch] activation format
   void* xs;                // [max_slots][pitch]: the rows of xn in slot order
