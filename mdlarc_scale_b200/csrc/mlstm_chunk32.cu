@@ -20,10 +20,10 @@ constexpr int TILE = 64 * CP;
 // q^T, k^T, weighted k, v, scores^T, state
 constexpr int C32_SMEM = 6 * TILE * 4;
 
-// acc[i][j] += sum_k a[k][4 ty + i] * b[k][4 tx + j], k = 0 .. 63
-__device__ __forceinline__ void tile_product(uint64_t (&acc)[4][2], const float* a, const float* b, int ty, int tx) {
+// acc[i][j] += sum_k a[k][4 ty + i] * b[k][4 tx + j], k = 0 .. n - 1
+__device__ __forceinline__ void tile_product(uint64_t (&acc)[4][2], const float* a, const float* b, int ty, int tx, int n = 64) {
 #pragma unroll 8
-  for (int k = 0; k < 64; ++k) {
+  for (int k = 0; k < n; ++k) {
     const float4 x = *reinterpret_cast<const float4*>(a + k * CP + 4 * ty);
     const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b + k * CP + 4 * tx);
     const float xs[4] = {x.x, x.y, x.z, x.w};
@@ -128,7 +128,9 @@ mlstm_chunk32_kernel(MlstmArgs a) {
         const double u = __shfl_up_sync(0xffffffffu, sum, o);
         if (lane >= o) sum += u;
       }
-      const double F1 = sum, F0 = sum - lf1;
+      double ahead = __shfl_up_sync(0xffffffffu, sum, 1);
+      if (lane == 0) ahead = 0.;
+      const double F1 = sum, F0 = ahead + lf0;   // not sum - lf1: nothing of a token reaches the one ahead of it
       const double none = -1e300;
       const double c0 = 2 * lane < nt ? (double)gate_log(gi[0], a.gate_cap, false) - F0 : none, c1 = 2 * lane + 1 < nt ? (double)gate_log(gi[1], a.gate_cap, false) - F1 : none;
       double top = fmax(c0, c1);
@@ -203,7 +205,22 @@ mlstm_chunk32_kernel(MlstmArgs a) {
       const float4 f = quad_of(acc[i]);
       set_quad(acc[i], make_float4(r * f.x, r * f.y, r * f.z, r * f.w));
     }
-    tile_product(acc, pt, vs, ty, tx);
+    // tokens ahead of the thread's four rows, then the rows' own, each up to itself: a later token's value may be anything, and zero
+    // times that is not always zero
+    tile_product(acc, pt, vs, ty, tx, 4 * ty);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 x = *reinterpret_cast<const float4*>(pt + (4 * ty + j) * CP + 4 * ty);
+      const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(vs + (4 * ty + j) * CP + 4 * tx);
+      const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int i = j; i < 4; ++i) {
+        uint64_t xx;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(xs[i]));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][0]) : "l"(xx), "l"(y.x));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][1]) : "l"(xx), "l"(y.y));
+      }
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int t = 4 * ty + i;

@@ -43,3 +43,19 @@ def test_chunks(sizes, heads, dim, vdim, bias):
     got = portions(registry.build_engine(cfg, w, "cuda:0", "f32"), toks, sizes)
     assert rel_error(got, oracle_logits(cfg, w, toks)) < TOL
     assert rel_error(got, portions(registry.build_engine(cfg, w, "cuda:0", "f32", mlstm_path="step"), toks, sizes)) < 2 * TOL
+
+
+@pytest.mark.parametrize("n", [40, 64, 65, 150])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_later_tokens_leave_earlier_ones_alone(n, value):
+    """One token of a prompt whose embedding is no number: the rows ahead of it keep every bit."""
+    cfg = config(160, 200, [mlstm(3, 64, 64), mlstm(2, 40, 56)])
+    w = vo.random_weights(cfg, 7)
+    w["embed"][199] = value
+    eng = registry.build_engine(cfg, w, "cuda:0", "f32")
+    toks = [t % 199 for t in tokens(cfg, n, 3)]
+    clean = portions(eng, toks, [n])
+    for at in {0, 1, 3, 30, n - 1, min(n - 1, 63), min(n - 1, 64), min(n - 1, 66)}:
+        got = portions(eng, toks[:at] + [199] + toks[at + 1:], [n])
+        assert torch.equal(got[:at], clean[:at]) and bool(torch.isfinite(got[:at]).all()), at
+        assert bool(got[at].isnan().all())
