@@ -5,6 +5,8 @@
 // neighbouring value columns.  A decode step reads and writes the state once, 16 bytes a lane and contiguous across the
 // warp, with all of a thread's loads in flight together; nothing else of the step is large, so the launch is bound by
 // that traffic.  The head's RMS norm, gain and output gate are applied before the row leaves.
+#include <atomic>
+
 #include "launch.cuh"
 #include "mlstm.cuh"
 
@@ -129,7 +131,7 @@ mlstm_step_kernel(MlstmArgs a) {
 // Segments of any length.  A walk is a chain of tokens, so what a token costs is latency: gates, decays and the head norm
 // are taken for TC tokens at a time, beside the state's updates instead of between them, and the chunk's operands are
 // fetched one chunk ahead.  Three barriers a chunk.  B200, 20 heads of 64 x 64, two segments of up to 999
-// tokens in fp32: 1427 us token by token, 356 here.
+// tokens in fp32: 1427 us token by token, 356 here.  REST: only the rows that mlstm_chunked_rows leaves.
 template <int DMAX, int VP>
 struct WalkCfg {
   using C = MlstmCfg<DMAX, VP>;
@@ -139,7 +141,7 @@ struct WalkCfg {
   static constexpr int SMEM = (2 * TC * ROW + TC * C::RG * VP + TC * DMAX) * 4;
 };
 
-template <int DMAX, int VP>
+template <int DMAX, int VP, bool REST = false>
 __global__ void __launch_bounds__(MlstmCfg<DMAX, VP>::NT, 1)
 mlstm_walk_kernel(MlstmArgs a) {
   using C = MlstmCfg<DMAX, VP>;
@@ -155,7 +157,8 @@ mlstm_walk_kernel(MlstmArgs a) {
   __shared__ float s_gl[2][TC], s_keep[TC], s_add[TC], s_floor[TC];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int h = blockIdx.x, sg = blockIdx.y;
-  const int row0 = a.seg_row0[sg], rows = a.seg_rows[sg], seq = a.seg_seq[sg], pos0 = a.seg_pos0[sg];
+  const int done = REST ? mlstm_chunked_rows(a.seg_rows[sg]) : 0;
+  const int row0 = a.seg_row0[sg] + done, rows = a.seg_rows[sg] - done, seq = a.seg_seq[sg], pos0 = a.seg_pos0[sg] + done;
   if (seq < 0 || seq >= a.n_seqs) {
     if (tid == 0) arcb_set_error(a.err, ARCB_DEV_BAD_INDEX);
     return;
@@ -304,6 +307,14 @@ int arcb_mlstm_walk_init() {
       (e = init_walk<256, 64>()) != cudaSuccess || (e = init_walk<256, 128>()) != cudaSuccess || (e = init_walk<256, 256>()) != cudaSuccess)
     return (int)e;
   return 0;
+}
+
+int arcb_launch_mlstm_rest64(const MlstmArgs& a, cudaStream_t stream) {
+  static std::atomic<unsigned long long> opted{0};
+  cudaError_t e = arcb_opt_in_smem(mlstm_walk_kernel<64, 64, true>, WalkCfg<64, 64>::SMEM, opted);
+  if (e == cudaSuccess) e = arcb_launch(mlstm_walk_kernel<64, 64, true>, dim3(a.H, a.n_segs), dim3(MlstmCfg<64, 64>::NT), WalkCfg<64, 64>::SMEM, stream, a);
+  arcb_count_launch(1);
+  return (int)e;
 }
 
 int arcb_launch_mlstm_step(const MlstmArgs& a, cudaStream_t stream) {

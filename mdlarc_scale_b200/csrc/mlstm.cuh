@@ -40,7 +40,14 @@ struct MlstmArgs {
 bool arcb_mlstm_chunk_supported(int dimp, int vdimp, int fmt);
 int arcb_mlstm_chunk_init();
 int arcb_launch_mlstm_chunk(const MlstmArgs& a, cudaStream_t stream);
+// Rows of a segment that the chunkwise kernel in 32 bits takes, from its first; the walk takes the others.
+// ALONE, TAIL: see mlstm_chunk32.cu.
+constexpr int C32_CHUNK = 64, C32_ALONE = 36, C32_TAIL = 24;
+__host__ __device__ inline int mlstm_chunked_rows(int rows) {
+  return rows <= C32_ALONE ? 0 : rows % C32_CHUNK <= C32_TAIL ? rows - rows % C32_CHUNK : rows;
+}
 bool arcb_mlstm_chunk32_supported(int dimp, int vdimp, int fmt);
+int arcb_launch_mlstm_rest64(const MlstmArgs& a, cudaStream_t stream);
 int arcb_launch_mlstm_chunk32(const MlstmArgs& a, cudaStream_t stream);
 int arcb_launch_mlstm_step(const MlstmArgs& a, cudaStream_t stream);
 void arcb_count_launch(long long n);

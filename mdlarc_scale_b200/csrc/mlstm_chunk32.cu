@@ -6,15 +6,23 @@
 // (n alike with k alone).  Running sums and exponents are taken in 64 bits: F may be large where only its differences count.
 // Token by token the chain of a token's loads, updates and barriers costs 0.4 us; here a chunk is four 64 x 64 x 64 products of two-wide
 // multiply-adds, a 4 x 4 tile a thread, operands in shared memory in the layout each product reads by quads, the next chunk's in
-// registers.  A segment's chunks start at its first row, so its results depend on nothing else in the call.
+// registers.  What bounds it: a chunk is 14 us of products behind one another on one CTA an SM, 11 us of an SM's time on two.
+//
+// A chunk costs nearly the same whatever it holds, so few tokens are left to the walk (mlstm.cu): segments of up to C32_ALONE, and up to
+// C32_TAIL behind the last whole chunk (mlstm_chunked_rows).  The rule looks at a segment's length alone and its chunks start at its
+// first row, so its results depend on nothing else in the call.  B200, 20 heads, us of both launches / of the walk alone / of chunks
+// alone; one segment: 36 rows 17.5 / 17.6 / 18.5, 40 16.1 / 18.7 / 17.5, 65 21.6 / 29.7 / 32.0, 80 26.3 / 34.5 / 32.0, 900 205 / 360 / 224;
+// 64 segments: 8 rows 31 / 27 / 150, 30 85 / 82 / 163, 40 112 / 105 / 167, 48 121 / 124 / 173, 65 160 / 169 / 306, 80 189 / 199 / 309,
+// 100 236 / 248 / 326, 200 409 / 475 / 594 (chunks alone: one CTA an SM, and all products of a chunk whatever it holds).
 #include <atomic>
 
+#include "gemm.cuh"
 #include "launch.cuh"
 #include "mlstm.cuh"
 
 namespace {
 
-constexpr int CL = 64, CD = 64, CP = 68;         // tokens of a chunk, columns of a head, pitch of a tile
+constexpr int CL = C32_CHUNK, CD = 64, CP = 68;         // tokens of a chunk, columns of a head, pitch of a tile
 constexpr int CT_THREADS = 256;
 constexpr int TILE = 64 * CP;
 // q^T, k^T, weighted k, v, scores^T, state
@@ -52,7 +60,10 @@ __device__ __forceinline__ float sum16(float v) {
   return v;
 }
 
-__global__ void __launch_bounds__(CT_THREADS, 1)
+// CTAS an SM: one keeps the next chunk's loads and a product's operands in registers (212), where CTAs are more than SMs two are quicker
+// with 128: 64 segments of 64 rows 147 us, one CTA an SM 179.  The arithmetic is the same.
+template <int CTAS>
+__global__ void __launch_bounds__(CT_THREADS, CTAS)
 mlstm_chunk32_kernel(MlstmArgs a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -67,7 +78,7 @@ mlstm_chunk32_kernel(MlstmArgs a) {
   __shared__ float s_row[CL], s_floor[CL], s_w[CL], s_n[CD], s_nq[4][CL], s_np[4][CD], s_end[2];
   const int tid = threadIdx.x, lane = tid & 31, tx = tid & 15, ty = tid >> 4, tok = tid & 63, part = tid >> 6;
   const int h = blockIdx.x, sg = blockIdx.y;
-  const int row0 = a.seg_row0[sg], rows = a.seg_rows[sg], seq = a.seg_seq[sg];
+  const int row0 = a.seg_row0[sg], rows = mlstm_chunked_rows(a.seg_rows[sg]), seq = a.seg_seq[sg];
   const bool fresh = a.seg_pos0[sg] == 0;
   if (seq < 0 || seq >= a.n_seqs) {
     if (tid == 0) arcb_set_error(a.err, ARCB_DEV_BAD_INDEX);
@@ -175,72 +186,78 @@ mlstm_chunk32_kernel(MlstmArgs a) {
       for (int d = 0; d < 16; ++d) nq = fmaf(s_n[part * 16 + d], qt[(part * 16 + d) * CP + tok], nq);
       s_nq[part][tok] = nq;
     }
+    const bool live = (ty & ~1) * 4 < nt;        // the warp has rows
     // scores, weighted
     uint64_t acc[4][2] = {};
-    tile_product(acc, qt, kt, ty, tx);
-    float p[4][4], psum[4];
+    float psum[4];
+    if (live) {
+      tile_product(acc, qt, kt, ty, tx);
+      float p[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float4 f = quad_of(acc[i]);
-      const float x[4] = {f.x, f.y, f.z, f.w};
-      const double M = s_M[4 * ty + i];
-      psum[i] = 0.f;
+      for (int i = 0; i < 4; ++i) {
+        const float4 f = quad_of(acc[i]);
+        const float x[4] = {f.x, f.y, f.z, f.w};
+        const double M = s_M[4 * ty + i];
+        psum[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          p[i][j] = 4 * tx + j <= 4 * ty + i ? x[j] * expf((float)(s_c[4 * tx + j] - M)) : 0.f;
+          psum[i] += p[i][j];
+        }
+        psum[i] = sum16(psum[i]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(pt + (4 * tx + j) * CP + 4 * ty) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
+    }
+    __syncthreads();
+    if (live) {
+      // numerators: the carried state's part, then the chunk's
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
+      tile_product(acc, qt, S, ty, tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float r = s_row[4 * ty + i];
+        const float4 f = quad_of(acc[i]);
+        set_quad(acc[i], make_float4(r * f.x, r * f.y, r * f.z, r * f.w));
+      }
+      // tokens ahead of the thread's four rows, then the rows' own, each up to itself: a later token's value may be anything, and zero
+      // times that is not always zero
+      tile_product(acc, pt, vs, ty, tx, 4 * ty);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        p[i][j] = 4 * tx + j <= 4 * ty + i ? x[j] * expf((float)(s_c[4 * tx + j] - M)) : 0.f;
-        psum[i] += p[i][j];
+        const float4 x = *reinterpret_cast<const float4*>(pt + (4 * ty + j) * CP + 4 * ty);
+        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(vs + (4 * ty + j) * CP + 4 * tx);
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int i = j; i < 4; ++i) {
+          uint64_t xx;
+          asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(xs[i]));
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][0]) : "l"(xx), "l"(y.x));
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][1]) : "l"(xx), "l"(y.y));
+        }
       }
-      psum[i] = sum16(psum[i]);
-    }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(pt + (4 * tx + j) * CP + 4 * ty) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
-    __syncthreads();
-    // numerators: the carried state's part, then the chunk's
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
-    tile_product(acc, qt, S, ty, tx);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float r = s_row[4 * ty + i];
-      const float4 f = quad_of(acc[i]);
-      set_quad(acc[i], make_float4(r * f.x, r * f.y, r * f.z, r * f.w));
-    }
-    // tokens ahead of the thread's four rows, then the rows' own, each up to itself: a later token's value may be anything, and zero
-    // times that is not always zero
-    tile_product(acc, pt, vs, ty, tx, 4 * ty);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 x = *reinterpret_cast<const float4*>(pt + (4 * ty + j) * CP + 4 * ty);
-      const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(vs + (4 * ty + j) * CP + 4 * tx);
-      const float xs[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-      for (int i = j; i < 4; ++i) {
-        uint64_t xx;
-        asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(xs[i]));
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][0]) : "l"(xx), "l"(y.x));
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][1]) : "l"(xx), "l"(y.y));
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = 4 * ty + i;
-      const float dot = fmaf(s_row[t], (s_nq[0][t] + s_nq[1][t]) + (s_nq[2][t] + s_nq[3][t]), psum[i]);
-      const float den = fmaxf(fabsf(dot), s_floor[t]) + 1e-6f;
-      float4 o = quad_of(acc[i]);
-      o.x /= den; o.y /= den; o.z /= den; o.w /= den;
-      const float ss = sum16((o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w));      // padding columns are exactly zero
-      const float norm = 1.f / sqrtf(ss * inv_v + a.eps);
-      if (t < nt) {
-        const size_t row = row0 + t0 + t;
-        const float4 g = ld_act4(a.proj, row * a.pitch + a.off_g + (size_t)h * CD + 4 * tx, a.fmt);
-        const float4 w = __ldg(reinterpret_cast<const float4*>(a.norm_w + (size_t)h * CD + 4 * tx));
-        st_act4(a.out, (row * a.H + h) * CD + 4 * tx, make_float4(o.x * norm * (w.x * g.x), o.y * norm * (w.y * g.y), o.z * norm * (w.z * g.z), o.w * norm * (w.w * g.w)), a.fmt);
+      for (int i = 0; i < 4; ++i) {
+        const int t = 4 * ty + i;
+        const float dot = fmaf(s_row[t], (s_nq[0][t] + s_nq[1][t]) + (s_nq[2][t] + s_nq[3][t]), psum[i]);
+        const float den = fmaxf(fabsf(dot), s_floor[t]) + 1e-6f;
+        float4 o = quad_of(acc[i]);
+        o.x /= den; o.y /= den; o.z /= den; o.w /= den;
+        const float ss = sum16((o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w));      // padding columns are exactly zero
+        const float norm = 1.f / sqrtf(ss * inv_v + a.eps);
+        if (t < nt) {
+          const size_t row = row0 + t0 + t;
+          const float4 g = ld_act4(a.proj, row * a.pitch + a.off_g + (size_t)h * CD + 4 * tx, a.fmt);
+          const float4 w = __ldg(reinterpret_cast<const float4*>(a.norm_w + (size_t)h * CD + 4 * tx));
+          st_act4(a.out, (row * a.H + h) * CD + 4 * tx, make_float4(o.x * norm * (w.x * g.x), o.y * norm * (w.y * g.y), o.z * norm * (w.z * g.z), o.w * norm * (w.w * g.w)), a.fmt);
+        }
       }
     }
     // state: rows d = 4 ty + i
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
-    tile_product(acc, kw, vs, ty, tx);
+    tile_product(acc, kw, vs, ty, tx, (nt + 7) & ~7);      // the others are zeros
     {
       float n = 0.f;
 #pragma unroll
@@ -273,9 +290,14 @@ bool arcb_mlstm_chunk32_supported(int dimp, int vdimp, int fmt) { return dimp ==
 int arcb_launch_mlstm_chunk32(const MlstmArgs& a, cudaStream_t stream) {
   if (a.n_segs <= 0) return 0;
   if (a.n_segs > 65535) return -1;
-  static std::atomic<unsigned long long> opted{0};
-  cudaError_t e = arcb_opt_in_smem(mlstm_chunk32_kernel, C32_SMEM, opted);
-  if (e == cudaSuccess) e = arcb_launch(mlstm_chunk32_kernel, dim3(a.H, a.n_segs), dim3(CT_THREADS), C32_SMEM, stream, a);
-  arcb_count_launch(1);
-  return (int)e;
+  if (a.n_rows > C32_ALONE) {                    // else no segment is long enough
+    static std::atomic<unsigned long long> opted[2];
+    const bool two = (long long)a.H * a.n_segs > arcb_num_sms();
+    auto kernel = two ? mlstm_chunk32_kernel<2> : mlstm_chunk32_kernel<1>;
+    cudaError_t e = arcb_opt_in_smem(kernel, C32_SMEM, opted[two]);
+    if (e == cudaSuccess) e = arcb_launch(kernel, dim3(a.H, a.n_segs), dim3(CT_THREADS), C32_SMEM, stream, a);
+    arcb_count_launch(1);
+    if (e != cudaSuccess) return (int)e;
+  }
+  return arcb_launch_mlstm_rest64(a, stream);
 }

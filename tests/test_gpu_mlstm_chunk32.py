@@ -59,3 +59,21 @@ def test_later_tokens_leave_earlier_ones_alone(n, value):
         got = portions(eng, toks[:at] + [199] + toks[at + 1:], [n])
         assert torch.equal(got[:at], clean[:at]) and bool(torch.isfinite(got[:at]).all()), at
         assert bool(got[at].isnan().all())
+
+
+@pytest.mark.parametrize("n,chunked", [(1, 0), (36, 0), (37, 37), (63, 63), (64, 64), (65, 64), (88, 64), (89, 89), (128, 128), (152, 128), (153, 153)])
+def test_few_tokens_are_walked(n, chunked):
+    """Rows up to the first chunk's length, and few behind the last whole one, by the walk; the others by chunks."""
+    cfg = config(160, 200, [mlstm(3, 64, 64)])
+    w = vo.random_weights(cfg, 7)
+    toks = tokens(cfg, n, 3)
+    eng, step = (registry.build_engine(cfg, w, "cuda:0", "f32", mlstm_path=path) for path in ("auto", "step"))
+    got, walked = portions(eng, toks, [n]), portions(step, toks, [n])
+    assert rel_error(got, oracle_logits(cfg, w, toks)) < TOL
+    if chunked == 0:
+        assert torch.equal(got, walked)
+    else:                      # sums in another order: not one row in eight has the walk's bits all over
+        assert int((got[:chunked] == walked[:chunked]).all(dim=1).sum()) <= chunked // 8
+    # what is walked behind chunks is what a portion of its own gets (one token alone is a decode step)
+    if 0 < chunked < n - 1:
+        assert torch.equal(got, portions(eng, toks, [chunked, n - chunked]))
