@@ -123,13 +123,23 @@ inline StepClusterSmem step_cluster_smem(int rows, int d, int dff, int heads, in
   return s;
 }
 
-// B200, four layers of width 256, us a token of a call, a graph of launches / one cluster: one row over 200 rows 85 / 57, 1000 91 / 62,
-// 2000 92 / 67; two rows over 1000 94 / 70; four over 200 86 / 75, 500 94 / 79; eight over 100 85 / 95, 200 88 / 96.  Weights and cached
-// rows beyond 16 MB a step (14 MB at 2000) are for the whole machine.
+// Whether the cluster is the quicker of the two, from what both were measured to take (B200, 199 sizes of 128 to 384 columns, 1 to 4
+// rows, 1 to 12 layers, 100 to 30 k cached rows; deviations 1.2 and 2.1 us).  us a step of a launch of one step: the cluster 11 and a layer
+// 7.3, 1.1 a MB of its weights, 0.6 a row and 0.26 a row and MB, 4.4 a thousand keys that one CTA reads and 1.8 where CTAs take a second
+// (row, head) item; launches of a graph 16 and a layer 13.3, 0.6 a thousand cached rows, 0.7 a million of all rows' columns.  A launch of many
+// steps spares the cluster 5.6 us a step, and a first launch the recording of a graph, hence the 2 us.  Graph / one step a launch / 16:
+// 256 columns, 4 layers: one row over 300 rows 70 / 51 / 46, over 2400 76 / 60 / 55, four over 600 76 / 74 / 68; one layer: one row over 10 k 37 / 31 /
+// 25, four over 1200 31 / 29 / 24, over 2400 31 / 35 / 30; 384 columns, 4 layers: two rows over 300 72 / 66 / 60; not taken: four over 300 72 / 82 / 76, one
+// layer, four over 2400 31 / 48 / 42.  Weights and cached rows beyond 16 MB a step are for the whole machine.
 constexpr int STEP_CLUSTER_ROWS = 4;
 inline bool step_cluster_fits(int rows, int d, int dff, int n_layers, int t_max, int cl) {
   if (rows < 1 || rows > STEP_CLUSTER_ROWS || d > 512 || d % 128 || dff % 64) return false;
   if (step_cluster_smem(rows, d, dff, d / 64, cl).total > STEP_CLUSTER_SMEM_MAX) return false;
-  const long long bytes = (long long)n_layers * (2LL * (4LL * d * d + 3LL * d * dff) + 4LL * d * rows * t_max);
-  return bytes <= 16LL << 20;
+  const long long weights = 2LL * (4LL * d * d + 3LL * d * dff), cached = 4LL * d * rows * t_max;      // bytes of a layer
+  if (n_layers * (weights + cached) > 16LL << 20) return false;
+  const int items = rows * (d / 64), splits = items < cl ? cl / items : 1, turns = (items * splits + cl - 1) / cl;
+  const double mb = weights * 1e-6, kt = t_max * 1e-3;
+  const double cluster = 11. + n_layers * (7.3 + 1.1 * mb + rows * (0.6 + 0.26 * mb) + 4.4 * turns * kt / splits + 1.8 * (turns - 1));
+  const double graph = 16. + n_layers * (13.3 + 0.6 * kt + 0.7 * rows * d * kt * 1e-3);
+  return cluster <= graph + 2.;
 }

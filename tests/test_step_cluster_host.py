@@ -56,3 +56,11 @@ def test_what_fits_lies_apart_in_shared_memory(rules):
                     assert odd - even >= max(qkv, gu) * 32 * d and total - odd >= narrow * 32 * max(d, dff) and total <= 220 * 1024
                     assert all(v % 16 == 0 for v in out) and even % 128 == 0 and odd % 128 == 0
     assert seen > 100
+
+
+@pytest.mark.parametrize("args,want", [
+    ((1, 128, 512, 1, 30000), 1), ((1, 256, 704, 1, 12000), 1), ((4, 256, 704, 1, 1200), 1), ((4, 256, 704, 4, 580), 1), ((2, 384, 448, 4, 300), 1),
+    ((4, 384, 256, 1, 300), 1), ((4, 384, 256, 1, 1200), 0), ((3, 384, 64, 1, 2400), 0), ((4, 384, 448, 4, 300), 0), ((1, 384, 448, 1, 9000), 0)])
+def test_caches_and_rows_that_launches_read_sooner(rules, args, want):
+    """Both sides were measured; what the cluster is slower at goes to the launches."""
+    assert rules.fits(*args, 16) == want
