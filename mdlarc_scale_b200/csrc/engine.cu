@@ -559,8 +559,12 @@ extern "C" int arcb_decode(arcb_session* s, int32_t n_steps, void* stream_v) {
     a.skip = s->desc.stop_on_end == 1 ? s->st.finished : nullptr;
     a.probe = s->step_probe;
     CKL(arcb_launch_step_cluster(s->st, a, s->step_cluster, stream), "decode steps");
-    s->step_stream = stream;
-    s->probe_recorded = true;
+    // the end of these steps, for the probe; under a capture it becomes a node of the caller's graph, which a programmatic edge cannot leave
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(stream, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    s->probe_recorded = s->probe_end && !(captured && arcb_pdl_enabled());
+    if (s->probe_recorded) CK(cudaEventRecordWithFlags(s->probe_end, stream, captured ? cudaEventRecordExternal : cudaEventRecordDefault));
     return ARCB_OK;
   }
   for (int attempt = 0; !s->graph_exec && attempt < 2; ++attempt) {
@@ -625,9 +629,11 @@ extern "C" int arcb_session_attention_probe(arcb_session* s, float* ms) {
   if (!s || !ms) return arcb_fail(ARCB_E_ARG, "null argument");
   if (!s->probe_recorded || (!s->graph_exec && !s->step_cluster)) return arcb_fail(ARCB_E_STATE, "no decode step has run yet");
   if (s->step_cluster) {
+    // an event and a stream of the session's own: the caller's may be gone, or busy with later work
     unsigned long long ns[2] = {0, 0};
-    CK(cudaStreamSynchronize(s->step_stream));
-    CK(cudaMemcpy(ns, s->step_probe, sizeof ns, cudaMemcpyDeviceToHost));
+    CK(cudaEventSynchronize(s->probe_end));
+    CK(cudaMemcpyAsync(ns, s->step_probe, sizeof ns, cudaMemcpyDeviceToHost, s->capture_stream));
+    CK(cudaStreamSynchronize(s->capture_stream));
     *ms = (float)(ns[1] - ns[0]) * 1e-6f;
     return ARCB_OK;
   }

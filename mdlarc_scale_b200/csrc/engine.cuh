@@ -82,7 +82,6 @@ struct arcb_session {
   long long graph_kernels = 0;
   int step_cluster = 0;            // > 0: steps run inside one cluster of that many CTAs instead of the recorded graph
   unsigned long long* step_probe = nullptr;
-  cudaStream_t step_stream = nullptr;   // of the last such steps
   bool armed = false;
   // event pair recorded (as graph nodes) around the layer-0 decode-attention launch of every replay
   cudaEvent_t probe_begin = nullptr, probe_end = nullptr;

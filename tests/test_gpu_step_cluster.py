@@ -112,3 +112,33 @@ def test_full_cache_drops_keys_and_reports_it():
         with pytest.raises(_lib.ArcbError):
             s.poll()
         s.close()
+
+
+def test_probe_waits_for_its_own_steps():
+    """Of steps on a stream that has later work queued, and on one that is gone."""
+    eng = engine(128, 192, 1)
+    ids, pos, mask, ex = batch(1, [30])
+    from mdlarc_scale_b200.engine import plan_prefill
+    s = eng.new_session(1, 60, 20, 64, stop_on_end=False)
+    s.prefill(plan_prefill(ids, pos, mask, np.arange(1)).to(torch.device("cuda:0")), torch.from_numpy(ex).int().cuda())
+    s.decode(4)
+    after = torch.cuda.Event()
+    torch.cuda._sleep(600_000_000)               # 0.3 s
+    after.record()
+    assert 0.0 < s.attention_probe_ms() < 1.0 and not after.query()
+    torch.cuda.synchronize()
+    handle = np.zeros(1, np.int64)
+    assert torch.cuda.cudart().cudaStreamCreate(handle.ctypes.data) == torch.cuda.cudart().cudaError.success
+    with torch.cuda.stream(torch.cuda.ExternalStream(int(handle[0]))):
+        s.decode(4)
+    assert torch.cuda.cudart().cudaStreamDestroy(int(handle[0])) == torch.cuda.cudart().cudaError.success
+    assert 0.0 < s.attention_probe_ms() < 1.0
+    s.poll()
+    # captured by the caller: the probe is of the replay
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        s.decode(2)
+    g.replay()
+    assert 0.0 < s.attention_probe_ms() < 1.0
+    s.poll()
+    s.close()
