@@ -222,10 +222,11 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
   auto norm = [&](const float* x, const float* gain) {
     if (warp >= M) return;
     const float* row = x + warp * d;
-    float4 v[4], g[4];
+    constexpr int Q = STEP_CLUSTER_WIDTH / 128;
+    float4 v[Q], g[Q];
     float ss = 0.f;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < Q; ++k) {
       const int c = (lane + 32 * k) * 4;
       v[k] = c < d ? *reinterpret_cast<const float4*>(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
       g[k] = c < d ? __ldg(reinterpret_cast<const float4*>(gain + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -233,7 +234,7 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
     }
     const float inv = rsqrtf(warp_sum(ss) / (float)d + a.embed.eps);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < Q; ++k) {
       const int c = (lane + 32 * k) * 4;
       if (c < d)
         *reinterpret_cast<uint2*>(xn + warp * xn_pitch + c * 2) =

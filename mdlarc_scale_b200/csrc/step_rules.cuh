@@ -131,9 +131,10 @@ inline StepClusterSmem step_cluster_smem(int rows, int d, int dff, int heads, in
 // 256 columns, 4 layers: one row over 300 rows 70 / 51 / 46, over 2400 76 / 60 / 55, four over 600 76 / 74 / 68; one layer: one row over 10 k 37 / 31 /
 // 25, four over 1200 31 / 29 / 24, over 2400 31 / 35 / 30; 384 columns, 4 layers: two rows over 300 72 / 66 / 60; not taken: four over 300 72 / 82 / 76, one
 // layer, four over 2400 31 / 48 / 42.  Weights and cached rows beyond 16 MB a step are for the whole machine.
-constexpr int STEP_CLUSTER_ROWS = 4;
+// Shared memory holds a layer of 384 columns up to d_ff 448, of 256 up to 1024 and of 128 up to 1536 (16 CTAs); none of 512.
+constexpr int STEP_CLUSTER_ROWS = 4, STEP_CLUSTER_WIDTH = 384;
 inline bool step_cluster_fits(int rows, int d, int dff, int n_layers, int t_max, int cl) {
-  if (rows < 1 || rows > STEP_CLUSTER_ROWS || d > 512 || d % 128 || dff % 64) return false;
+  if (rows < 1 || rows > STEP_CLUSTER_ROWS || d > STEP_CLUSTER_WIDTH || d % 128 || dff % 64) return false;
   if (step_cluster_smem(rows, d, dff, d / 64, cl).total > STEP_CLUSTER_SMEM_MAX) return false;
   const long long weights = 2LL * (4LL * d * d + 3LL * d * dff), cached = 4LL * d * rows * t_max;      // bytes of a layer
   if (n_layers * (weights + cached) > 16LL << 20) return false;

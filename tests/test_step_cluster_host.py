@@ -64,3 +64,8 @@ def test_what_fits_lies_apart_in_shared_memory(rules):
 def test_caches_and_rows_that_launches_read_sooner(rules, args, want):
     """Both sides were measured; what the cluster is slower at goes to the launches."""
     assert rules.fits(*args, 16) == want
+
+
+def test_widths_that_shared_memory_holds(rules):
+    widest = {d: max((dff for dff in range(64, 4097, 64) if rules.fits(1, d, dff, 1, 64, 16)), default=0) for d in range(128, 1025, 128)}
+    assert widest == {128: 1536, 256: 1024, 384: 448, **{d: 0 for d in range(512, 1025, 128)}}
