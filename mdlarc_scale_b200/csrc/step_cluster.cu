@@ -1,8 +1,8 @@
 // Decode steps of the smallest models (up to 4 rows of 384 columns): any number of steps in one launch of one cluster.
 //
 // A step of such a model is 28 launches of 1.5 to 3.7 us for four layers, each a chain of loads, one reduction and a store, while
-// all weights together stream from L2 in a few microseconds.  Here 16 SMs (8 where the model fits them and no cluster of 16 runs) take
-// the whole loop: columns of every product are divided among the CTAs, rows of 16 weights at a time on mma.m16n8k16 (the sequences
+// all weights together stream from L2 in a few microseconds.  Here 16 SMs take the whole loop (on a device that runs no cluster of 16 the
+// launches stay): columns of every product are divided among the CTAs, rows of 16 weights at a time on mma.m16n8k16 (the sequences
 // are its columns); what the next phase reads (queries, attention records, residual stream, hidden units) is written into every
 // CTA's shared memory, and a cluster barrier (five a layer) takes the place of a launch.  A phase's weights are copied into shared
 // memory while the phase before it runs.  Norms, embedding and the merge of attention records are repeated in every CTA.
@@ -533,23 +533,23 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
   landed(bar_even, turn_even);                   // the request behind the last layer
 }
 
-constexpr int SC_DEVICES = 64;
+constexpr int SC_DEVICES = 64, SC_CLUSTER = 16;
 
-// Clusters of `cl` CTAs that run on this device, at their most shared memory.
+// Whether a cluster runs on this device, at its most shared memory.
 template <bool F16>
-bool cluster_runs(int cl) {
+bool cluster_runs() {
   static std::mutex mu;
-  static int known[SC_DEVICES][2];
+  static int known[SC_DEVICES];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= SC_DEVICES) return false;
   std::lock_guard<std::mutex> lock(mu);
-  return asked_once(known[dev][cl == 16], [&](int& n) {
+  return asked_once(known[dev], [&](int& n) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = cl;
+    attr.val.clusterDim.x = SC_CLUSTER;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cl);
+    cfg.gridDim = dim3(SC_CLUSTER);
     cfg.blockDim = dim3(SC_THREADS);
     cfg.dynamicSmemBytes = STEP_CLUSTER_SMEM_MAX;
     cfg.attrs = &attr;
@@ -565,9 +565,7 @@ bool cluster_runs(int cl) {
 }  // namespace
 
 int arcb_step_cluster(int rows, int d, int dff, int n_layers, int t_max) {
-  for (int cl = 16; cl >= 8; cl /= 2)
-    if (step_cluster_fits(rows, d, dff, n_layers, t_max, cl) && cluster_runs<true>(cl) && cluster_runs<false>(cl)) return cl;
-  return 0;
+  return step_cluster_fits(rows, d, dff, n_layers, t_max, SC_CLUSTER) && cluster_runs<true>() && cluster_runs<false>() ? SC_CLUSTER : 0;
 }
 
 int arcb_launch_step_cluster(const DecodeState& st, const StepArgs& a, int cluster, cudaStream_t stream) {
