@@ -524,6 +524,7 @@ class PaddedBatch:
         pos = pos[:self.n, :self.seq_len, :3]
         if tuple(pos.shape) != (self.n, self.seq_len, 3):
             raise ValueError("positions must have shape [batch, seq_len, 3]")
+        mask = None if mask is None else mask[:self.n]
         if mask is not None and tuple(mask.shape) != (self.n, self.seq_len):
             raise ValueError("mask must have shape [batch, seq_len]")
         self.h2d_bytes = 0

@@ -58,3 +58,14 @@ def test_shapes_that_do_not_fit_are_refused():
     for bad_pos, bad_mask in ((pos[:, :4], None), (pos[:1], None), (pos[..., :2], None), (pos, np.ones((2, 6), bool)), (pos, np.ones((1, 5), bool))):
         with pytest.raises(ValueError):
             PaddedBatch(ids, bad_pos, bad_mask, "cuda:0")
+
+
+def test_rows_behind_the_batch_are_left_out():
+    """Positions and masks of more sequences than there are tokens for, as the host's plan takes them."""
+    g = np.random.default_rng(3)
+    ids, pos, mask = g.integers(0, 14, (3, 20)), g.integers(0, 5, (5, 20, 3)), masks("right", 5, 20, g)
+    want = plan_prefill(ids, pos, mask, np.arange(3), all_positions=True, with_first=False)
+    for move in (lambda a: a, lambda a: torch.from_numpy(a).cuda()):
+        got = PaddedBatch(move(ids), move(pos), move(mask), "cuda:0").plan(np.arange(3), all_positions=True, with_first=False)
+        for name in ("token_ids", "pos_xyz", "seq", "kv_slot", "kv_count", "kv_row"):
+            assert torch.equal(getattr(want, name), getattr(got, name).cpu()), name
