@@ -5,19 +5,21 @@ import torch
 
 from gpu_util import have_b200
 from mdlarc_scale_b200 import _lib
-from mdlarc_scale_b200.engine import Engine
+from mdlarc_scale_b200.engine import Engine, initial_grid_state
 from mdlarc_scale_b200.inference import generate_tokens
 
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_b200(), reason="needs a B200")]
 
 
-def engine(d, dff, layers, act="f16", seed=0):
+def engine(d, dff, layers, act="f16", seed=0, chain=False):
     g = torch.Generator().manual_seed(seed)
 
     def r(*s, std=1.0, mean=0.0):
         return (torch.randn(s, generator=g) * std + mean).to(torch.bfloat16).float()
     w = {"token_embed.weight": r(14, d), "example_embed.weight": r(8, d, std=0.02), "ln_f.weight": r(d, std=0.05, mean=1.0),
          "lm_head.weight": r(14, d, std=d ** -0.5)}
+    if chain:
+        w["lm_head.weight"] = (w["token_embed.weight"].roll(1, 0) * d ** -0.5).bfloat16().float()
     for n in range(layers):
         p = f"blocks.{n}."
         w.update({p + "ln1.weight": r(d, std=0.05, mean=1.0), p + "attn.qkv_proj.weight": r(3 * d, d, std=d ** -0.5),
@@ -65,22 +67,83 @@ def test_steps_match_separate_launches(d, dff, layers, rows, act):
     eng.close()
 
 
-def test_loop_ends_freezes_and_constrains_as_separate_launches_do():
-    eng = engine(256, 704, 2)
+def grid_after(state, tok):
+    """Grid state after a fed token (src/inference.py:127-168)."""
+    x, y = state
+    if tok in (10, 12):
+        return 0, 0
+    if tok == 11:
+        return 0, min(y + 1, 29)
+    return (min(x + 1, 30), y) if tok < 10 else (x, y)
+
+
+def uniform(seed, stream, index):
+    m = 2 ** 64 - 1
+    z = (seed + 0x9E3779B97F4A7C15 * (stream + 1) + 0xD1B54A32D192ED03 * (index + 1)) & m
+    z = (z ^ z >> 30) * 0xBF58476D1CE4E5B9 & m
+    z = (z ^ z >> 27) * 0x94D049BB133111EB & m
+    return ((z ^ z >> 31) >> 40) / 2 ** 24
+
+
+def choices(logits, state, row, index, constraints=None, temperature=0.0, top_k=None, sample_seed=0):
+    """Tokens that these logits allow (several where a rounding decides a sample)."""
+    adj = logits.numpy().astype(np.float32).copy()
+    c = constraints or {}
+    adj[list(c.get("disallow_tokens", ()))] = -np.inf
+    if "palette_mask" in c:
+        adj[:10][~c["palette_mask"][row]] -= np.float32(2.0)
+    if "target_shape" in c and min(c["target_shape"][row]) >= 0:
+        (h, w), (x, y) = c["target_shape"][row], state
+        adj[slice(0, 10) if x >= w else slice(11, 12)] -= np.float32(2.0)
+        if y >= h:
+            adj[:10] -= np.float32(2.0)
+            adj[11] -= np.float32(2.0)
+    if temperature <= 0:
+        return {int(adj.argmax())}
+    kept = sorted(range(14), key=lambda v: (-adj[v], v))[:top_k or 14]
+    p = np.array([np.exp((float(adj[v]) - float(adj.max())) / temperature) if v in kept else 0.0 for v in range(14)])
+    at, ends = uniform(sample_seed, row, index), np.cumsum(p) / p.sum()
+    return {int(np.argmax(ends > min(max(u, 0.0), 1 - 1e-9))) for u in (at - 1e-5, at, at + 1e-5)}
+
+
+# The row of the output matrix that belongs to a token's successor points along that token's embedding: rows count up to END and
+# on from 0, so they end (and at different steps).
+@pytest.mark.parametrize("kw", [
+    dict(), dict(stop_on_end=False), dict(freeze_finished=False),
+    dict(constraints=dict(palette_mask=np.tile(np.arange(10) % 3 == 0, (4, 1)), target_shape=np.full((4, 2), 3), disallow_tokens=(10, 12))),
+    dict(constraints=dict(target_shape=np.array([[2, 5], [1, 1], [-1, -1], [4, 2]]))),
+    dict(temperature=1.3, top_k=5, sample_seed=11), dict(temperature=3.0, sample_seed=2 ** 63 + 5)], ids=lambda kw: "-".join(kw) or "plain")
+def test_loop_ends_freezes_and_constrains(kw):
+    """Every token is the one that its logits, the row's grid and the request's options give; the logits are those of separate launches
+    fed the same tokens."""
+    eng = engine(256, 704, 2, chain=True)
     ids, pos, mask, ex = batch(4, [40, 9, 77, 130])
-    for kw in (dict(), dict(stop_on_end=False), dict(freeze_finished=False),
-               dict(constraints=dict(palette_mask=np.tile(np.arange(10) % 3 == 0, (4, 1)), target_shape=np.full((4, 2), 3), disallow_tokens=(10, 12))),
-               dict(temperature=1.3, top_k=5, sample_seed=11)):
-        a, b = (generate_tokens(eng, ids, pos, mask, ex, 70, want_logits=True, attn_splits=s, **kw) for s in (0, 1))
-        n = min(a.tokens.shape[1], b.tokens.shape[1])
-        for i in range(4):
-            same = (a.tokens[i, :n] == b.tokens[i, :n]).cpu()
-            first = n if bool(same.all()) else int((~same).float().argmax())
-            # up to the first token that a rounding decides, and that one has to be close
-            torch.testing.assert_close(a.step_logits[i, :first], b.step_logits[i, :first], rtol=0.02, atol=0.02)
-            if first < n and "temperature" not in kw and "constraints" not in kw:
-                top = b.step_logits[i, first].sort().values
-                assert float(top[-1] - top[-2]) < 0.04
+    new = 40
+    a = generate_tokens(eng, ids, pos, mask, ex, new, want_logits=True, **kw)
+    toks, logits = a.tokens.cpu().numpy(), a.step_logits.cpu()
+    last = mask.sum(1) - 1
+    gx, gy, _ = initial_grid_state(ids[np.arange(4), last], pos[np.arange(4), last], np.ones(4, bool))
+    frozen_rows = kw.get("stop_on_end", True) and kw.get("freeze_finished", True)
+    options = {k: v for k, v in kw.items() if k not in ("stop_on_end", "freeze_finished")}
+    alive = np.zeros(toks.shape, bool)
+    for r in range(4):
+        state, ended = (int(gx[r]), int(gy[r])), False
+        for i, tok in enumerate(toks[r].tolist()):
+            alive[r, i] = not (frozen_rows and ended)
+            assert tok in (choices(logits[r, i], state, r, i, **options) if alive[r, i] else {13}), (r, i)
+            ended |= tok == 13
+            state = grid_after(state, tok)
+    if not kw:
+        assert (toks == 13).any(1).all() and not alive.all()       # rows have ended, and stayed
+    if kw == dict(freeze_finished=False):
+        assert (toks == 13).any(1).all() and ((toks[:, :-1] == 13) & (toks[:, 1:] != 13)).any()
+    forced = np.full((4, new), 13, np.int32)
+    forced[:, :toks.shape[1]] = toks
+    b = generate_tokens(eng, ids, pos, mask, ex, new, stop_on_end=False, forced=forced, want_logits=True, attn_splits=1)
+    n = toks.shape[1]
+    scale = float(b.step_logits[:, :n].square().mean().sqrt())
+    assert float((logits[:, :n] - b.step_logits.cpu()[:, :n])[torch.from_numpy(alive)].abs().max()) < 0.02 * scale
+    eng.close()
 
 
 def test_steps_in_parts_are_steps_in_one_go():
