@@ -145,6 +145,7 @@ def generate_tokens(engine: Engine, ids: np.ndarray, pos: np.ndarray, mask: np.n
         session.prefill(plan, ex_dev, first_logits=fl)
     if batch is not None:
         h2d += batch.h2d_bytes
+    batch = plan = None             # their device memory (up to 33 bytes a padded position, 32 a token) is not kept through the steps
     steps_total = max_new - 1
     done = 0
     while done < steps_total:

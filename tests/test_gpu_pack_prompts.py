@@ -1,10 +1,14 @@
 """Prefill calls planned on the device against the host's plan of the same padded batch."""
+import weakref
+
 import numpy as np
 import pytest
 import torch
 
 from gpu_util import have_b200
-from mdlarc_scale_b200.engine import PaddedBatch, plan_prefill
+from mdlarc_scale_b200 import inference
+from mdlarc_scale_b200.engine import PaddedBatch, Session, plan_prefill
+from test_gpu_step_cluster import batch, engine
 
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_b200(), reason="needs a B200")]
 
@@ -69,3 +73,28 @@ def test_rows_behind_the_batch_are_left_out():
         got = PaddedBatch(move(ids), move(pos), move(mask), "cuda:0").plan(np.arange(3), all_positions=True, with_first=False)
         for name in ("token_ids", "pos_xyz", "seq", "kv_slot", "kv_count", "kv_row"):
             assert torch.equal(getattr(want, name), getattr(got, name).cpu()), name
+
+
+def test_the_batch_is_gone_when_steps_begin(monkeypatch):
+    """Generation holds the padded arrays on the device for the prompt alone."""
+    eng = engine(128, 192, 1)
+    ids, pos, mask, ex = batch(64, [300, 280])
+    made, left = [], []
+
+    class Noted(PaddedBatch):
+        def __init__(self, *args):
+            super().__init__(*args)
+            made.append(weakref.ref(self.ids))
+            made.append(weakref.ref(self.pos))
+
+        def plan(self, *args, **kw):
+            p = super().plan(*args, **kw)
+            made.append(weakref.ref(p.pos_xyz))
+            return p
+
+    decode = Session.decode
+    monkeypatch.setattr(inference, "PaddedBatch", Noted)
+    monkeypatch.setattr(Session, "decode", lambda self, n: (left.extend(w() is not None for w in made), decode(self, n))[1])
+    inference.generate_tokens(eng, ids, pos, mask, ex, 4)
+    assert len(made) == 3 and left and not any(left)
+    eng.close()
