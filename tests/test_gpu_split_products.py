@@ -81,3 +81,13 @@ def test_rows_beside_such_values_keep_their_bits(M, N, K, value):
         assert torch.equal(got.isnan(), plain.isnan()) and torch.equal(got.isinf(), plain.isinf())
     b = torch.full_like(a, value)                # all of them
     assert torch.equal(product(b, w).nan_to_num(), product(b, w, _lib.GEMM_SIMT).nan_to_num())
+
+
+@pytest.mark.parametrize("kind", ["plain", "wide", "16-bit weights", "mixed weights"])
+@pytest.mark.parametrize("K", [64, 128, 192, 320, 640, 1280, 2560])
+def test_no_further_off_than_multiply_adds(K, kind):
+    """Of 131072 sums: the norm of all errors, at every length."""
+    a, w = operands(256, 512, K, kind)
+    ref = a.double() @ w.double().T
+    got, plain = ((product(a, w, path).double() - ref).norm() for path in (_lib.GEMM_AUTO, _lib.GEMM_SIMT))
+    assert got <= plain
