@@ -35,7 +35,7 @@ extern "C" {
 
 #define ARCB_ACT_F16 0  /* 16-bit activations held as IEEE half (default)     */
 #define ARCB_ACT_BF16 1 /* 16-bit activations held as bfloat16                */
-#define ARCB_ACT_F32 2  /* 32-bit everywhere, CUDA-core products (layered engines only) */
+#define ARCB_ACT_F32 2  /* 32-bit operands, sums and state (layered engines only)  */
 
 #define ARCB_GEMM_AUTO 0 /* tcgen05 GEMM wherever the shape allows (K % 64 == 0)   */
 #define ARCB_GEMM_SIMT 1 /* CUDA-core GEMM everywhere (debug cross-check)      */

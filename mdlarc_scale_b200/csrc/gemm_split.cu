@@ -12,10 +12,11 @@
 //
 // What bounds it: 24 instructions of 128 x 128 x 16 for 64 columns (12 where the weights are bf16 values, as those of a checkpoint
 // in 16 bits are: their other pieces are zeros), and next to them the splitting of 16 k values by 16 warps, 6 to 8 operations each, on
-// their way from memory to the two operand stages, with one block of loads ahead: 1.0 to 1.2 us a block of 64 columns, issue slots 55 %
-// busy, the tensor pipe 24 %.  8 warps with twice the work each: the same.
-// B200, us a launch, multiply-adds / here with 16-bit weights (any weights): 1719 rows, 1280 x 1280 151 / 35 (41), 5120 x 1280 470 / 130
-// (144), 1280 x 5120 588 / 118 (132); 28 rows, 32000 x 1280 160 / 67 (72); 1 row, 1280 x 1280 82 / 33 (35), 1280 x 5120 316 / 114 (123).
+// their way from memory to the two operand stages, with one block of loads ahead: 1.0 to 1.2 us a block of 64 columns, issue slots 61 %
+// busy, the tensor pipe 26 % (any weights: 56 %, 48 %).  8 warps with twice the work each: the same.
+// B200, us a launch, multiply-adds / here with 16-bit weights (any weights): 1719 rows, 1280 x 1280 151 / 35 (39), 5120 x 1280 470 / 131
+// (144), 1280 x 5120 588 / 119 (134); 28 rows, 32000 x 1280 160 / 68 (72); 1 row, 1280 x 1280 82 / 33 (35), 1280 x 5120 316 / 119 (125).
+// Registers are at their limit (96): a few more held through the loop for redo_without_pieces cost 3 to 13 % of a launch.
 #include <atomic>
 
 #include "common.cuh"

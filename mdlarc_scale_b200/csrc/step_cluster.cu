@@ -8,8 +8,8 @@
 // memory while the phase before it runs.  Norms, embedding and the merge of attention records are repeated in every CTA.
 // Rounding points are those of the separate kernels; sums over K and over keys are divided differently.
 // What bounds it is latency: of 18 k cycles a layer (width 256, one row) 5.5 k are barriers with the stores they wait for, 3.5 k
-// products, 3.3 k their epilogues, 3 k attention, 1.5 k norms.  B200, one row of 168 to 215 cached rows, us a step: launches of
-// a graph 70, here 45 (weights through registers 48, by 16-byte asynchronous copies 52).
+// products, 3.3 k their epilogues, 3 k attention, 1.5 k norms.  B200, one row of 168 to 300 cached rows, us a step: launches of
+// a graph 70, here 46 in a launch of many steps, 51 in one of a single step (weights through registers 48, by 16-byte asynchronous copies 52).
 #include <mutex>
 
 #include "common.cuh"
