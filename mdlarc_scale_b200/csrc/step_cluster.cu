@@ -174,6 +174,7 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
   __shared__ __align__(8) unsigned long long s_bar[2];
   const uint32_t bar_even = smem_u32(s_bar), bar_odd = bar_even + 8;
   uint32_t turn_even = 0, turn_odd = 0;
+  bool ok = true;                                                    // no wait has run out
   const int rank = (int)cluster_ctarank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int M = a.rows, d = a.d, H = a.n_heads, T = st.t_max;
   const int xn_pitch = d * 2 + 64, hs_pitch = a.dff * 2 + 64;       // neighbouring rows on the other half of the banks
@@ -241,14 +242,12 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
             make_uint2(pack2_act((v[k].x * inv) * g[k].x, (v[k].y * inv) * g[k].y, fmt), pack2_act((v[k].z * inv) * g[k].z, (v[k].w * inv) * g[k].w, fmt));
     }
   };
-  // this part's weights have landed; nobody else's have to be waited for
-  bool ok = true;
+  // this part's weights have landed; nobody else's have to be waited for.  A launch gives up once, and asks for nothing more then.
   auto landed = [&](uint32_t bar, uint32_t& turn) {
-    if (ok && !mbar_wait_bounded(bar, turn)) {   // a launch gives up once
-      arcb_set_error(st.err, ARCB_DEV_WAIT_TIMEOUT_TMA);
-      ok = false;
-    }
-    turn ^= 1;
+    if (!ok) return;
+    ok = mbar_wait_bounded(bar, turn);
+    if (ok) turn ^= 1;
+    else arcb_set_error(st.err, ARCB_DEV_WAIT_TIMEOUT_TMA);
   };
   // Sums of this CTA's tiles to all CTAs: a thread a destination and quad of a row.
   const int cl_bits = 31 - __clz(cl);
@@ -295,7 +294,7 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
       const StepLayer L = a.layers[l];
       __nv_bfloat16* kc = a.cache + (size_t)l * 2 * M * H * T * ARCB_HEAD_DIM;
       __nv_bfloat16* vc = kc + (size_t)M * H * T * ARCB_HEAD_DIM;
-      request(Part{L.w_out, d, tiles_d, false}, rank, cl, odd, bar_odd);
+      if (ok) request(Part{L.w_out, d, tiles_d, false}, rank, cl, odd, bar_odd);
       norm(xa, L.ln1);
       __syncthreads();
       landed(bar_even, turn_even);
@@ -463,7 +462,7 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
       }
       __syncthreads();
       const Part gu{L.w_gu, d, 2 * units_gu, true};
-      request(gu, rank, cl, even, bar_even);
+      if (ok) request(gu, rank, cl, even, bar_even);
       landed(bar_odd, turn_odd);
       multiply<F16>(d, tiles_d, sm + lay.odd, xn, xn_pitch, red);
       __syncthreads();
@@ -471,7 +470,7 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
       __syncwarp();
       cluster_sync_all();
 
-      request(Part{L.w_down, a.dff, tiles_d, false}, rank, cl, odd, bar_odd);
+      if (ok) request(Part{L.w_down, a.dff, tiles_d, false}, rank, cl, odd, bar_odd);
       norm(xb, L.ln2);
       __syncthreads();
       landed(bar_even, turn_even);
@@ -491,7 +490,7 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
       __syncwarp();
       cluster_sync_all();
 
-      request(Part{a.layers[l + 1 < a.n_layers ? l + 1 : 0].w_qkv, d, tiles_qkv, false}, rank, cl, even, bar_even);
+      if (ok) request(Part{a.layers[l + 1 < a.n_layers ? l + 1 : 0].w_qkv, d, tiles_qkv, false}, rank, cl, even, bar_even);
       landed(bar_odd, turn_odd);
       multiply<F16>(a.dff, tiles_d, sm + lay.odd, hs, hs_pitch, red);
       __syncthreads();
@@ -531,6 +530,10 @@ step_cluster_kernel(DecodeState st, StepArgs a, int cl, StepClusterSmem lay) {
     cluster_sync_all();                          // also: nobody leaves while its memory is written
   }
   landed(bar_even, turn_even);                   // the request behind the last layer
+  if (!ok) {                                     // what is still on its way gets another limit each: it writes into this CTA's memory
+    mbar_wait_bounded(bar_even, turn_even);
+    mbar_wait_bounded(bar_odd, turn_odd);
+  }
 }
 
 constexpr int SC_DEVICES = 64, SC_CLUSTER = 16;
